@@ -49,8 +49,10 @@ def reference_root() -> Optional[str]:
 
 def build_ref(reference_root: Optional[str]) -> Optional[str]:
     """Builds oracle/_ref/ref_partition_harness from the reference tree at
-    reference_root; returns None when no tree is given or it does not exist."""
-    if not reference_root or not os.path.isdir(reference_root):
+    reference_root; returns None when no tree is given or it holds no
+    partitioner sources."""
+    if not reference_root or not os.path.isfile(
+            os.path.join(reference_root, "L2", "sparse", "src", "sw", "c++", "gen_signature.cpp")):
         return None
     subprocess.run([os.path.join(HERE, "build_ref.sh"), reference_root], check=True, capture_output=True)
     return REF_HARNESS
