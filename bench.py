@@ -617,7 +617,8 @@ def run_gb300(args):
     # past the stop in the last pass launch and return at once)
     inf_l = h.info()
     per_pass = inf_l.kernelsPerIter * inf_l.loopUnroll
-    launches = sum(1 + per_pass * -(-k // inf_l.loopUnroll) for k in iters)
+    # loopUnroll 0: the whole loop is one launch
+    launches = sum(1 + (per_pass * -(-k // inf_l.loopUnroll) if inf_l.loopUnroll else 1) for k in iters)
 
     # Dominant kernel: the SpMV, timed alone on the same stream and matrix.
     spmv_ms = None

@@ -28,24 +28,6 @@ namespace xjpcg {
 
 constexpr int kVecThreads = 256;
 
-__device__ __forceinline__ void write_record(CgState* s, uint32_t k, double rr, double rz, double alpha,
-                                             double beta) {
-    if (s->records == nullptr || s->recCap < 2) return;
-    const uint32_t slot = (k + 1u < s->recCap) ? k + 1u : 1u + (k % (s->recCap - 1u));
-    IterRecord rec;
-    rec.id = 0;
-    rec.iter = k;
-    rec.vecSize = s->vecSize;
-    rec.maxIter = s->maxIterP1;
-    rec.tols = s->tols;
-    rec.res = rr;
-    rec.rz = rz;
-    rec.alpha = alpha;
-    rec.beta = beta;
-    rec.clock = globaltimer_ns();
-    s->records[slot] = rec;
-}
-
 __global__ void __launch_bounds__(kVecThreads) cg_init_kernel(int n, int n4, const double* __restrict__ b,
                                                               const double* __restrict__ diag, double* __restrict__ x,
                                                               double* __restrict__ r, double* __restrict__ p,

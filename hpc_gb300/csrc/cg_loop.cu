@@ -1,0 +1,790 @@
+// cg_loop.cu -- the whole fp64 JPCG loop in one kernel, for systems whose
+// vectors fit on the chip.
+//
+// What bounds a small system is the chain of dependent steps in an iteration,
+// not bytes or operations: on GB300 a dependent FP64 add takes 64 cycles, a
+// division 550, a load from L2 300 and more, a release fence 540, a counter
+// barrier over 152 SMs 1,600 and a cluster barrier 370 (all measured).  As two
+// kernels per iteration in a graph, with a grid barrier inside the second, an
+// iteration took 14 to 15 us however small the system.  Here one launch runs
+// all iterations: r, x, z = J r, p and J never leave shared memory, nor does
+// the part of the matrix that fits beside them; only p is also written to
+// global memory, for the other CTAs' gathers.
+//
+// Two forms:
+//   cg_cluster_kernel  one cluster of up to 16 CTAs; p is gathered, and the
+//                      sums are exchanged, through distributed shared memory.
+//                      Three cluster barriers per iteration.
+//   cg_loop_kernel     one CTA per SM, cooperative; sums go through posts and
+//                      counters in global memory.
+//
+// Measured, us per iteration (two kernels per iteration / loop / cluster):
+//   7-point   16^3   14.7 /  8.8 / 6.9      27-point   8^3  15.1 / 13.1 / 6.5
+//             32^3   14.7 /  9.5 /  -                 16^3  16.9 / 10.9 / 8.4
+//             48^3   18.1 / 12.3 /  -                 32^3  18.0 / 11.7 /  -
+//             64^3   25.5 / 17.5 /  -                 48^3  24.2 / 17.9 /  -
+//             80^3   31.3 / 26.7 /  -                 60^3  33.0 / 34.6 /  -
+//
+// Every row is summed in its stored order, as in the sliced SpMV kernels; the
+// dot products are summed per thread, per warp, per CTA and over the CTAs, in
+// an order that depends on n alone, so a solve is bitwise reproducible.
+#include <algorithm>
+
+#include "xjpcg_device.cuh"
+#include "xjpcg_internal.hpp"
+
+namespace xjpcg {
+
+namespace {
+constexpr int kLoopThreads = 448;   // at most; 144 registers (512 threads spilled and took 3 to 6 % longer)
+constexpr int kVecThreads = 256;    // threads that update r and z: enough to fill the FP64 pipe, and every warp costs two sums
+constexpr int kCols = 8;            // stored columns per step of a row: their loads go out together
+constexpr int kPosts = 5;           // posts a lane reads at once: 152 CTAs in one step
+constexpr uint64_t kLoopBudgetNs = 2000000000ull;  // 2 s
+constexpr size_t kLoopSmem = 226 * 1024;
+
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+// Waits until the counter has reached target.  False after the wait's budget.
+// One thread per CTA polls one address: 152 CTAs meet in 1,600 cycles, where
+// every CTA polling every CTA's flag took 8,900 (the few lines that all read).
+__device__ __forceinline__ bool wait_count(const uint32_t* counter, uint32_t target) {
+    uint64_t t0 = 0;
+    for (uint32_t spin = 0;; ++spin) {
+        uint32_t v;
+        asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(counter) : "memory");
+        if ((int32_t)(v - target) >= 0) return true;
+        if ((spin & 255u) == 255u) {
+            const uint64_t now = globaltimer_ns();
+            if (t0 == 0) t0 = now;
+            if (now - t0 > kLoopBudgetNs) return false;
+        }
+    }
+}
+
+__device__ __forceinline__ void arrive(uint32_t* counter) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+}
+
+// Sum over the lanes below `count` (a power of two or 32), in lane 0 at least.
+// A dependent FP64 add takes 64 cycles here, so no level is taken in vain.
+__device__ __forceinline__ double lanes_sum(double v, int count) {
+    for (int o = 16; o > 0; o >>= 1)
+        if (o < count) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// A CTA's total to every CTA and back, by one warp: the sum of all CTAs'
+// totals, in every lane.  A post is two words of half the value and the
+// iteration's tag, so it needs no fence before the counter: the counter says
+// when to look, the tags say whether the post has landed.
+__device__ __forceinline__ double grid_total(double s, ulonglong2* posts, uint32_t* counter, uint32_t target,
+                                             uint32_t tag, int lane, bool& ok) {
+    if (lane == 0) {
+        const uint64_t bits = (uint64_t)__double_as_longlong(s);
+        const uint64_t lo = (bits & 0xffffffffull) | ((uint64_t)tag << 32), hi = (bits >> 32) | ((uint64_t)tag << 32);
+        asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(posts + blockIdx.x), "l"(lo), "l"(hi)
+                     : "memory");
+        arrive(counter);
+        ok = wait_count(counter, target);
+    }
+    __syncwarp();
+    double sum = 0.0;
+    uint64_t t0 = 0;
+    const int P = gridDim.x;
+    for (int b = lane; b < P; b += 32 * kPosts) {
+        ulonglong2 w[kPosts];
+        for (uint32_t spin = 0;; ++spin) {
+            bool all = true;
+#pragma unroll
+            for (int u = 0; u < kPosts; ++u)
+                if (b + 32 * u < P)
+                    asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];"
+                                 : "=l"(w[u].x), "=l"(w[u].y)
+                                 : "l"(posts + b + 32 * u)
+                                 : "memory");
+#pragma unroll
+            for (int u = 0; u < kPosts; ++u)
+                if (b + 32 * u < P) all = all && (uint32_t)(w[u].x >> 32) == tag && (uint32_t)(w[u].y >> 32) == tag;
+            if (all) break;
+            if ((spin & 255u) == 255u) {
+                const uint64_t now = globaltimer_ns();
+                if (t0 == 0) t0 = now;
+                if (now - t0 > kLoopBudgetNs) {
+                    ok = false;
+                    break;
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kPosts; ++u)
+            if (b + 32 * u < P)
+                sum += __longlong_as_double((long long)((w[u].x & 0xffffffffull) | (w[u].y << 32)));
+    }
+    __syncwarp();
+    return warp_sum(sum);
+}
+}  // namespace
+
+// CTA q owns a contiguous run of slices (so neighbouring rows' gathers meet in
+// its L1).  Per iteration:
+//   Ap = A p into sz, p.Ap        -> grid sum, alpha
+//   r -= alpha Ap, z = J r        -> grid sums of r.r and r.z, beta, stop test;
+//                                    the idle warps do x += alpha p meanwhile
+//   p = z + beta p, also to global -> barrier (release / acquire)
+// Only the last needs fences: the posts of the sums carry their own tags.
+// LAY: 0 int32 columns, 1 int16 offsets, 2 slice-shared offsets.
+template <int LAY>
+__global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
+    extern __shared__ __align__(16) unsigned char loopSmem[];
+    __shared__ double sAlpha, sBeta, sRz, sRr;
+    __shared__ int sGo[3], sOn;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    const int q = blockIdx.x, P = gridDim.x;
+    const int s0 = (int)((int64_t)a.nslices * q / P), s1 = (int)((int64_t)a.nslices * (q + 1) / P);
+    const int ns = s1 - s0, pairs = ns * 16, row0 = s0 * 32;
+    double* const sr = reinterpret_cast<double*>(loopSmem);
+    double* const sx = sr + a.rows;
+    double* const sz = sx + a.rows;
+    double* const sp = sz + a.rows;
+    double* const sj = sp + a.rows;
+    double* const part = sj + a.rows;  // 2 per warp
+    int4* const meta = reinterpret_cast<int4*>(part + 64);
+    int* const place = reinterpret_cast<int*>(meta + a.rows / 32);
+    unsigned char* const mat = reinterpret_cast<unsigned char*>(place + (a.rows / 32 + 3) / 4 * 4);
+
+    for (int i = tid; i < pairs; i += nt) {
+        const int e = row0 / 2 + i;
+        const bool in = e < a.n2;
+        const double2 zero = make_double2(0.0, 0.0);
+        reinterpret_cast<double2*>(sr)[i] = in ? reinterpret_cast<const double2*>(a.r)[e] : zero;
+        reinterpret_cast<double2*>(sp)[i] = in ? reinterpret_cast<const double2*>(a.p)[e] : zero;
+        reinterpret_cast<double2*>(sj)[i] = in ? reinterpret_cast<const double2*>(a.J)[e] : zero;
+        reinterpret_cast<double2*>(sx)[i] = zero;
+    }
+    // slice records: {first value, columns, pattern or first column, shared offsets?}
+    for (int i = tid; i < ns; i += nt) {
+        const int off = a.sliceOff[s0 + i];
+        int4 md = make_int4(off, (a.sliceOff[s0 + i + 1] - off) >> 5, off, 0);
+        if (LAY == 2) {
+            md.w = a.patLen[s0 + i] > 0 ? 1 : 0;
+            md.z = md.w ? a.patOff[a.patIdx[s0 + i]] : a.genOff[s0 + i];
+        }
+        meta[i] = md;
+    }
+    if (tid == 0) sRz = a.state->rz;
+    __syncthreads();
+    // The first nOn slices, as many as fit, stay in shared memory (place: their
+    // bytes there, values then columns).
+    if (tid == 0) {
+        int at = 0, i = 0;
+        for (; i < ns; ++i) {
+            const int4 md = meta[i];
+            const int bytes = 256 * md.y + (md.w ? (4 * md.y + 15) / 16 * 16 : (LAY == 1 ? 64 : 128) * md.y);
+            if (at + bytes > a.matBytes) break;
+            place[i] = at;
+            at += bytes;
+        }
+        sOn = i;
+    }
+    __syncthreads();
+    const int nOn = sOn;
+    for (int ls = wid; ls < nOn; ls += nw) {
+        const int4 md = meta[ls];
+        double* const v = reinterpret_cast<double*>(mat + place[ls]);
+        int* const c = reinterpret_cast<int*>(v + 32 * md.y);
+        for (int j = 0; j < md.y; ++j) {
+            v[j * 32 + lane] = a.sval[md.x + j * 32 + lane];
+            if (LAY == 0)
+                c[j * 32 + lane] = a.col32[md.z + j * 32 + lane];
+            else if (LAY == 1)
+                reinterpret_cast<int16_t*>(c)[j * 32 + lane] = a.col16[md.z + j * 32 + lane];
+            else if (!md.w)
+                c[j * 32 + lane] = a.gcol[md.z + j * 32 + lane];
+        }
+        if (LAY == 2 && md.w)
+            for (int j = lane; j < md.y; j += 32) c[j] = a.pat[md.z + j];
+    }
+    auto column = [&](const int4& md, int row, int j) {
+        if (LAY == 0) return __ldcs(a.col32 + md.z + j * 32 + lane);
+        if (LAY == 1) return min(row, a.n - 1) + __ldcs(a.col16 + md.z + j * 32 + lane);
+        return md.w ? row + __ldg(a.pat + md.z + j) : __ldcs(a.gcol + md.z + j * 32 + lane);
+    };
+    __syncthreads();
+    const double tols = a.state->tols;
+    const uint32_t maxIterP1 = a.state->maxIterP1;
+    double2* const p2 = reinterpret_cast<double2*>(a.p) + row0 / 2;
+    const int have2 = max(0, min(pairs, a.n2 - row0 / 2));  // pairs of this CTA that exist
+
+    int nwUp = 1;
+    while (nwUp < nw) nwUp *= 2;
+
+    uint32_t k = 0;
+    bool ok = true;
+    for (;;) {
+        const uint32_t target = (k + 1u) * (uint32_t)P, tag = a.tag0 + k;
+        // ---- Ap = A p (kept in sz) and this thread's part of p.Ap ----
+        double dacc = 0.0;
+        int ls = wid;
+        for (; ls < nOn; ls += nw) {
+            const int4 md = meta[ls];
+            const int r = ls * 32 + lane, row = row0 + r, at = place[ls];
+            double acc = 0.0;
+            {
+                const double* const v = reinterpret_cast<const double*>(mat + at) + lane;
+                const int* const c = reinterpret_cast<const int*>(mat + at + 256 * md.y);
+                const int base = LAY == 1 ? min(row, a.n - 1) : row;
+                for (int j = 0; j < md.y; j += kCols) {
+                    double xv[kCols];
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u)
+                        if (j + u < md.y) {
+                            int col;
+                            if (LAY == 1)
+                                col = base + reinterpret_cast<const int16_t*>(c)[(j + u) * 32 + lane];
+                            else
+                                col = LAY == 2 && md.w ? base + c[j + u] : c[(j + u) * 32 + lane];
+                            xv[u] = a.p[col];
+                        }
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u)
+                        if (j + u < md.y) acc = fma(v[(j + u) * 32], xv[u], acc);
+                }
+            }
+            sz[r] = row < a.n ? acc : 0.0;
+            if (row < a.n) dacc = fma(sp[r], acc, dacc);
+        }
+        for (; ls < ns; ls += nw) {
+            const int4 md = meta[ls];
+            const int r = ls * 32 + lane, row = row0 + r;
+            double acc = 0.0;
+            {
+                const double* vp = a.sval + md.x + lane;
+                int j = 0;
+                for (; j + kCols <= md.y; j += kCols) {
+                    double v[kCols];
+                    int c[kCols];
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u) {
+                        v[u] = ld_val(vp + u * 32);
+                        c[u] = column(md, row, j + u);
+                    }
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u) acc = fma(v[u], a.p[c[u]], acc);
+                    vp += kCols * 32;
+                }
+                const int rem = md.y - j;
+                if (rem > 0) {
+                    double v[kCols - 1], xv[kCols - 1];
+                    int c[kCols - 1];
+#pragma unroll
+                    for (int u = 0; u < kCols - 1; ++u)
+                        if (u < rem) {
+                            v[u] = ld_val(vp + u * 32);
+                            c[u] = column(md, row, j + u);
+                        }
+#pragma unroll
+                    for (int u = 0; u < kCols - 1; ++u)
+                        if (u < rem) xv[u] = a.p[c[u]];
+#pragma unroll
+                    for (int u = 0; u < kCols - 1; ++u)
+                        if (u < rem) acc = fma(v[u], xv[u], acc);
+                }
+            }
+            sz[r] = row < a.n ? acc : 0.0;
+            if (row < a.n) dacc = fma(sp[r], acc, dacc);
+        }
+        dacc = warp_sum(dacc);
+        if (lane == 0) part[wid] = dacc;
+        __syncthreads();
+        if (wid == 0) {
+            double s = lanes_sum(lane < nw ? part[lane] : 0.0, nwUp);
+            s = grid_total(s, a.posts, a.counters, target, tag, lane, ok);
+            if (lane == 0) {
+                const double al = sRz / s;
+                sAlpha = al;
+                sGo[0] = isfinite(al) ? 1 : 0;
+                if (q == 0) a.state->pAp = s;
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        const double alpha = sAlpha;
+        // ---- r -= alpha Ap, z = J r ----
+        double rr = 0.0, rz = 0.0;
+        for (int i = tid; i < have2 && tid < kVecThreads; i += min(nt, kVecThreads)) {
+            double2 rv = reinterpret_cast<double2*>(sr)[i];
+            const double2 av = reinterpret_cast<double2*>(sz)[i], jv = reinterpret_cast<double2*>(sj)[i];
+            rv.x = fma(-alpha, av.x, rv.x);
+            rv.y = fma(-alpha, av.y, rv.y);
+            const double2 zv = make_double2(rv.x * jv.x, rv.y * jv.y);
+            rr = fma(rv.x, rv.x, rr);
+            rr = fma(rv.y, rv.y, rr);
+            rz = fma(rv.x, zv.x, rz);
+            rz = fma(rv.y, zv.y, rz);
+            reinterpret_cast<double2*>(sr)[i] = rv;
+            reinterpret_cast<double2*>(sz)[i] = zv;
+        }
+        if (tid < kVecThreads) {
+            rr = warp_sum(rr);
+            rz = warp_sum(rz);
+            if (lane == 0) {
+                part[wid] = rr;
+                part[32 + wid] = rz;
+            }
+        }
+        __syncthreads();
+        if (wid < 2) {
+            double s = lanes_sum(lane < min(nw, kVecThreads / 32) ? part[32 * wid + lane] : 0.0, min(nwUp, kVecThreads / 32));
+            s = grid_total(s, a.posts + (1 + wid) * P, a.counters + (1 + wid) * 32, target, tag, lane, ok);
+            if (lane == 0) {
+                if (wid == 0) {
+                    sRr = s;
+                    sGo[1] = isfinite(s) && !(s < tols) && k + 1u < maxIterP1 ? 1 : 0;
+                } else {
+                    const double beta = s / sRz;
+                    sBeta = beta;
+                    sRz = s;
+                    sGo[2] = isfinite(beta) ? 1 : 0;
+                }
+            }
+        } else {
+            // x += alpha p while the sums are on their way
+            for (int i = tid; i < have2; i += nt) {
+                double2 xv = reinterpret_cast<double2*>(sx)[i];
+                const double2 pv = reinterpret_cast<double2*>(sp)[i];
+                xv.x = fma(alpha, pv.x, xv.x);
+                xv.y = fma(alpha, pv.y, xv.y);
+                reinterpret_cast<double2*>(sx)[i] = xv;
+            }
+        }
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        const bool go = (sGo[0] & sGo[1] & sGo[2]) != 0;
+        const double beta = sBeta;
+        if (q == 0 && tid == nt - 1) {
+            CgState* st = a.state;
+            write_record(st, k, sRr, sRz, alpha, beta);
+            if (!go) {
+                st->alpha = alpha;
+                st->rr = sRr;
+                st->rz = sRz;
+                st->beta = beta;
+                st->k = k + 1u;
+                if (!isfinite(alpha) || !isfinite(beta) || !isfinite(sRr)) st->status |= kStatusBreakdown;
+                st->done = 1u;
+            }
+        }
+        // ---- p = z + beta p ----
+        for (int i = tid; i < have2; i += nt) {
+            double2 pv = reinterpret_cast<double2*>(sp)[i];
+            if (wid < 2) {
+                double2 xv = reinterpret_cast<double2*>(sx)[i];
+                xv.x = fma(alpha, pv.x, xv.x);
+                xv.y = fma(alpha, pv.y, xv.y);
+                reinterpret_cast<double2*>(sx)[i] = xv;
+            }
+            if (go) {
+                const double2 zv = reinterpret_cast<double2*>(sz)[i];
+                pv.x = fma(beta, pv.x, zv.x);
+                pv.y = fma(beta, pv.y, zv.y);
+                reinterpret_cast<double2*>(sp)[i] = pv;
+                p2[i] = pv;
+            }
+        }
+        if (!go) break;
+        __syncthreads();
+        if (tid == 0) {
+            fence_gpu();
+            arrive(a.counters + 96);
+            ok = wait_count(a.counters + 96, target);
+            fence_gpu();
+        }
+        if (__syncthreads_or(!ok)) {
+            ok = false;
+            break;
+        }
+        ++k;
+    }
+    if (!ok) {
+        if (tid == 0) {
+            atomicOr(&a.state->status, kStatusWaitTimeout);
+            a.state->done = 1u;
+        }
+        return;
+    }
+    for (int i = tid; i < have2; i += nt)
+        reinterpret_cast<double2*>(a.x)[row0 / 2 + i] = reinterpret_cast<double2*>(sx)[i];
+}
+
+namespace {
+constexpr int kClusterThreads = 512;
+constexpr int kClusterMax = 16;
+constexpr size_t kClusterSmem = 212 * 1024;  // beside 14 KB of static shared memory
+constexpr int kClusterSlots = kClusterMax * (kClusterThreads / 32);
+
+// Every thread of the cluster; distributed shared memory written before is
+// visible after.
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__device__ __forceinline__ uint32_t map_rank(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
+    return a;
+}
+
+__device__ __forceinline__ double ld_cluster(uint32_t a) {
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
+    return v;
+}
+
+// v, in every lane, into the same place of every CTA of the cluster.
+__device__ __forceinline__ void to_all(double* place, double v, int P, int lane) {
+    if (lane < P)
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(map_rank(place, (uint32_t)lane)), "d"(v) : "memory");
+}
+
+__device__ __forceinline__ double slots_sum(const double* slots, int count, int lane) {
+    double s = lane < count ? slots[lane] : 0.0;
+    for (int i = lane + 32; i < count; i += 32) s += slots[i];
+    return warp_sum(s);
+}
+}  // namespace
+
+// One cluster.  R rows per CTA, so a column's owner is column / R.  The matrix
+// part in shared memory holds, per entry, the value and the cluster address of
+// its p, so a gather is one load (about 250 cycles).  Every warp writes its part
+// of a sum to every CTA; after the cluster barrier each CTA adds all of them in
+// the same order.  A CTA always runs to the same decision as the others, and no
+// CTA is read or written by another after its last cluster barrier.
+template <int LAY>
+__global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs a) {
+    extern __shared__ __align__(16) unsigned char loopSmem[];
+    __shared__ double slots[3][kClusterSlots];
+    __shared__ double sAlpha, sBeta, sRz, sRr;
+    __shared__ int sGo[3];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    const int q = blockIdx.x, P = gridDim.x, R = a.rows;
+    const int s0 = q * (R / 32), ns = max(0, min(R / 32, a.nslices - s0)), row0 = s0 * 32;
+    double* const sr = reinterpret_cast<double*>(loopSmem);
+    double* const sx = sr + R;
+    double* const sz = sx + R;
+    double* const sp = sz + R;
+    double* const sj = sp + R;
+    int4* const meta = reinterpret_cast<int4*>(sj + R);
+    double* const mv = reinterpret_cast<double*>(meta + R / 32);
+    for (int i = tid; i < R; i += nt) {
+        const int e = row0 + i;
+        const bool in = e < 2 * a.n2;
+        sr[i] = in ? a.r[e] : 0.0;
+        sp[i] = in ? a.p[e] : 0.0;
+        sj[i] = in ? a.J[e] : 0.0;
+        sx[i] = 0.0;
+    }
+    for (int i = tid; i < ns; i += nt) {
+        const int off = a.sliceOff[s0 + i];
+        int4 md = make_int4(off, (a.sliceOff[s0 + i + 1] - off) >> 5, off, 0);
+        if (LAY == 2) {
+            md.w = a.patLen[s0 + i] > 0 ? 1 : 0;
+            md.z = md.w ? a.patOff[a.patIdx[s0 + i]] : a.genOff[s0 + i];
+        }
+        meta[i] = md;
+    }
+    if (tid == 0) sRz = a.state->rz;
+    __syncthreads();
+    const int mat0 = ns > 0 ? meta[0].x : 0;
+    const int matN = ns > 0 ? meta[ns - 1].x + 32 * meta[ns - 1].y - mat0 : 0;
+    const bool onChip = (int64_t)matN * 12 <= a.matBytes;
+    uint32_t* const mc = reinterpret_cast<uint32_t*>(mv + matN);
+    // where entry j of this lane's row finds its p, in the cluster's shared memory
+    auto place = [&](const int4& md, int row, int j) {
+        int c;
+        if (LAY == 0)
+            c = a.col32[md.z + j * 32 + lane];
+        else if (LAY == 1)
+            c = min(row, a.n - 1) + a.col16[md.z + j * 32 + lane];
+        else
+            c = md.w ? row + a.pat[md.z + j] : a.gcol[md.z + j * 32 + lane];
+        return map_rank(sp + c % R, (uint32_t)(c / R));
+    };
+    if (onChip)
+        for (int ls = wid; ls < ns; ls += nw) {
+            const int4 md = meta[ls];
+            for (int j = 0; j < md.y; ++j) {
+                mv[md.x - mat0 + j * 32 + lane] = a.sval[md.x + j * 32 + lane];
+                mc[md.x - mat0 + j * 32 + lane] = place(md, row0 + ls * 32 + lane, j);
+            }
+        }
+    const double tols = a.state->tols;
+    const uint32_t maxIterP1 = a.state->maxIterP1;
+    cluster_sync();
+
+    uint32_t k = 0;
+    bool go = true;
+    while (go) {
+        // ---- Ap = A p ----
+        double dacc = 0.0;
+        for (int ls = wid; ls < ns; ls += nw) {
+            const int4 md = meta[ls];
+            const int r = ls * 32 + lane;
+            double acc = 0.0;
+            if (onChip) {
+                const int at = md.x - mat0 + lane;
+                for (int j = 0; j < md.y; j += kCols) {
+                    double xv[kCols];
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u)
+                        if (j + u < md.y) xv[u] = ld_cluster(mc[at + (j + u) * 32]);
+#pragma unroll
+                    for (int u = 0; u < kCols; ++u)
+                        if (j + u < md.y) acc = fma(mv[at + (j + u) * 32], xv[u], acc);
+                }
+            } else {
+                for (int j = 0; j < md.y; ++j)
+                    acc = fma(a.sval[md.x + j * 32 + lane], ld_cluster(place(md, row0 + r, j)), acc);
+            }
+            if (row0 + r >= a.n) acc = 0.0;
+            sz[r] = acc;
+            dacc = fma(sp[r], acc, dacc);
+        }
+        to_all(&slots[0][q * nw + wid], warp_sum(dacc), P, lane);
+        cluster_sync();
+        if (wid == 0) {
+            const double s = slots_sum(slots[0], P * nw, lane);
+            if (lane == 0) {
+                const double al = sRz / s;
+                sAlpha = al;
+                sGo[0] = isfinite(al) ? 1 : 0;
+                if (q == 0) a.state->pAp = s;
+            }
+        }
+        __syncthreads();
+        const double alpha = sAlpha;
+        // ---- r -= alpha Ap, z = J r ----
+        double rr = 0.0, rz = 0.0;
+        for (int i = tid; i < ns * 32; i += nt) {
+            const double rv = fma(-alpha, sz[i], sr[i]);
+            const double zv = rv * sj[i];
+            rr = fma(rv, rv, rr);
+            rz = fma(rv, zv, rz);
+            sr[i] = rv;
+            sz[i] = zv;
+        }
+        rr = warp_sum(rr);
+        rz = warp_sum(rz);
+        to_all(&slots[1][q * nw + wid], rr, P, lane);
+        to_all(&slots[2][q * nw + wid], rz, P, lane);
+        cluster_sync();
+        if (wid < 2) {
+            const double s = slots_sum(slots[1 + wid], P * nw, lane);
+            if (lane == 0) {
+                if (wid == 0) {
+                    sRr = s;
+                    sGo[1] = isfinite(s) && !(s < tols) && k + 1u < maxIterP1 ? 1 : 0;
+                } else {
+                    const double beta = s / sRz;
+                    sBeta = beta;
+                    sRz = s;
+                    sGo[2] = isfinite(beta) ? 1 : 0;
+                }
+            }
+        }
+        __syncthreads();
+        go = (sGo[0] & sGo[1] & sGo[2]) != 0;
+        const double beta = sBeta;
+        if (q == 0 && tid == nt - 1) {
+            CgState* st = a.state;
+            write_record(st, k, sRr, sRz, alpha, beta);
+            if (!go) {
+                st->alpha = alpha;
+                st->rr = sRr;
+                st->rz = sRz;
+                st->beta = beta;
+                st->k = k + 1u;
+                if (!isfinite(alpha) || !isfinite(beta) || !isfinite(sRr)) st->status |= kStatusBreakdown;
+                st->done = 1u;
+            }
+        }
+        // ---- x += alpha p, p = z + beta p ----
+        for (int i = tid; i < ns * 32; i += nt) {
+            const double pv = sp[i];
+            sx[i] = fma(alpha, pv, sx[i]);
+            if (go) sp[i] = fma(beta, pv, sz[i]);
+        }
+        if (go) cluster_sync();
+        ++k;
+    }
+    for (int i = tid; i < ns * 32; i += nt)
+        if (row0 + i < 2 * a.n2) a.x[row0 + i] = sx[i];
+}
+
+namespace {
+struct LoopShape {
+    int P, rows, threads;
+    size_t fixed;  // shared memory besides the matrix
+};
+
+LoopShape loop_shape(int n, int numSms) {
+    LoopShape s;
+    const int nslices = (n + 31) / 32;
+    s.P = std::min(numSms, nslices);
+    const int ns = (nslices + s.P - 1) / s.P;
+    s.rows = 32 * ns;
+    s.threads = std::max(64, std::min(kLoopThreads, 32 * ns));
+    s.fixed = sizeof(double) * (5 * (size_t)s.rows + 64) + sizeof(int4) * (size_t)ns +
+              sizeof(int) * (size_t)((ns + 3) / 4 * 4);
+    return s;
+}
+
+template <int LAY>
+cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
+    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kLoopSmem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)s.P);
+    cfg.blockDim = dim3((unsigned)s.threads);
+    cfg.dynamicSmemBytes = a.smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY>, a);
+}
+}  // namespace
+
+namespace {
+// The cluster form: its CTAs' rows and shared memory.
+LoopShape cluster_shape(int n) {
+    LoopShape s;
+    const int nslices = (n + 31) / 32;
+    const int ns = (nslices + kClusterMax - 1) / kClusterMax;
+    s.P = (nslices + ns - 1) / ns;
+    s.rows = 32 * ns;
+    s.threads = std::max(64, std::min(kClusterThreads, 32 * ns));
+    s.fixed = sizeof(double) * 5 * (size_t)s.rows + sizeof(int4) * (size_t)ns;
+    return s;
+}
+
+template <int LAY>
+cudaError_t cluster_config(const LoopShape& s, size_t smem, cudaStream_t st, cudaLaunchConfig_t* cfg,
+                           cudaLaunchAttribute* attr) {
+    cudaError_t e = cudaFuncSetAttribute(cg_cluster_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)kClusterSmem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(cg_cluster_kernel<LAY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    *cfg = {};
+    cfg->gridDim = dim3((unsigned)s.P);
+    cfg->blockDim = dim3((unsigned)s.threads);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)s.P;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+    return e;
+}
+
+// Whether the current device can hold the largest cluster; asked once per device.
+bool device_takes_cluster() {
+    constexpr int kMaxDev = 64;
+    static int cache[kMaxDev] = {};  // 0 not asked, 1 yes, 2 no
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) {
+        cudaGetLastError();
+        return false;
+    }
+    int v = __atomic_load_n(&cache[dev], __ATOMIC_RELAXED);
+    if (v == 0) {
+        LoopShape s;
+        s.P = kClusterMax;
+        s.threads = kClusterThreads;
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        int clusters = 0;
+        v = cluster_config<2>(s, kClusterSmem, nullptr, &cfg, attr) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, cg_cluster_kernel<2>, &cfg) == cudaSuccess && clusters > 0
+                ? 1
+                : 2;
+        cudaGetLastError();
+        __atomic_store_n(&cache[dev], v, __ATOMIC_RELAXED);
+    }
+    return v == 1;
+}
+
+template <int LAY>
+cudaError_t cluster_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    const cudaError_t e = cluster_config<LAY>(s, a.smem, st, &cfg, attr);
+    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, cg_cluster_kernel<LAY>, a) : e;
+}
+}  // namespace
+
+// FP64 operations of an iteration up to which 16 SMs finish before 152 do:
+// the cluster form wins by 25 % at 56,000 (7-point 16^3) and 23 % at 126,000
+// (27-point 16^3); at 112,000 (7-point 20^3) both take 9 us, and at 251,000
+// (27-point 20^3) the grid form is ahead, 11.1 against 11.9 us.
+constexpr int64_t kClusterWork = 130000;
+
+bool cg_cluster_fits(int n, int64_t stored) {
+    if (n <= 0 || stored + 7 * (int64_t)n > kClusterWork) return false;
+    const LoopShape s = cluster_shape(n);
+    if (s.fixed + 16 * (size_t)(stored / s.P) + 1024 > kClusterSmem) return false;
+    return device_takes_cluster();
+}
+
+cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a) {
+    const LoopShape s = cluster_shape(a.n);
+    a.nslices = (a.n + 31) / 32;
+    a.rows = s.rows;
+    a.matBytes = (int)((kClusterSmem - s.fixed) / 16 * 16);
+    a.smem = s.fixed + (size_t)a.matBytes;
+    if (layout == 0) return cluster_launch<0>(st, s, a);
+    if (layout == 1) return cluster_launch<1>(st, s, a);
+    return cluster_launch<2>(st, s, a);
+}
+
+// The vectors have to fit in shared memory (875,000 rows on 152 SMs), and at
+// most 6.5 entries per row may have to be read from L2 or HBM in every
+// iteration: the stream runs with 14 warps per SM, where the SpMV kernels of
+// the graph loop have 48.  7-point 80^3 (half of the matrix streamed): 26.7 us
+// against 31.3; 27-point 54^3 (9 entries per row by this count) 25.5 against
+// 27.7, 60^3 (15) 34.6 against 33.0 and 70^3 51 against 40.
+bool cg_loop_fits(int n, int64_t stored, int entryBytes, int numSms) {
+    if (n <= 0) return false;
+    const LoopShape s = loop_shape(n, numSms);
+    if (s.fixed > kLoopSmem) return false;
+    const int64_t resident = (int64_t)((kLoopSmem - s.fixed) / (size_t)entryBytes) * s.P;
+    return 2 * (stored - resident) <= 13 * (int64_t)n;
+}
+
+size_t cg_loop_sync_bytes(int numSms) { return 128 * sizeof(uint32_t) + 3 * sizeof(ulonglong2) * 2 * (size_t)numSms; }
+
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a) {
+    const LoopShape s = loop_shape(a.n, numSms);
+    a.nslices = (a.n + 31) / 32;
+    a.rows = s.rows;
+    a.counters = static_cast<uint32_t*>(sync);
+    a.posts = reinterpret_cast<ulonglong2*>(a.counters + 128);
+    // A CTA whose part of the matrix fits in the rest copies it there.
+    a.matBytes = (int)((kLoopSmem - s.fixed) / 16 * 16);
+    a.smem = s.fixed + (size_t)a.matBytes;
+    if (layout == 0) return loop_launch<0>(st, s, a);
+    if (layout == 1) return loop_launch<1>(st, s, a);
+    return loop_launch<2>(st, s, a);
+}
+
+}  // namespace xjpcg

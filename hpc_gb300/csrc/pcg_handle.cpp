@@ -159,6 +159,7 @@ void PcgHandle::init(int device) {
     check(cudaStreamSynchronize(m_stream), "sync");
     m_useGraph = envInt("XJPCG_HOST_LOOP", 0) == 0;
     m_fusedUpdate = envInt("XJPCG_FUSED_UPDATE", 1) != 0;
+    m_loopKernelEnv = envInt("XJPCG_LOOP_KERNEL", -1);
     m_forcedLanes = envInt("XJPCG_SPMV_LANES", 0);
     m_forcedCfg = envInt("XJPCG_SPMV_CFG", -1);
     m_faultAlloc = envIs("XJPCG_FAULT", "alloc");
@@ -1007,6 +1008,61 @@ int PcgHandle::cgSpmvMode() const {
                                                                                          : kSpmvCgDot;
 }
 
+// Whether the fp64 loop runs as one kernel (cg_loop.cu), and which: 0 no, 1
+// over the grid, 2 in one cluster.  It reads a sliced copy, whichever is built;
+// the choice depends on the matrix alone, so that repeated solves agree bit
+// for bit.  A forced SpMV layout keeps the loop of that layout's kernel (unless
+// XJPCG_LOOP_KERNEL=1), as the host-driven loop and the separate vector kernels
+// keep theirs.
+int PcgHandle::loopKernel(uint32_t maxIter, int* layout) {
+    const bool forced = m_forcedCfg >= 0 || m_forcedLanes != 0;
+    if (!m_useGraph || !m_fusedUpdate || m_loopKernelEnv == 0 || maxIter > 0xfffffff0u) return 0;
+    if (forced && (m_loopKernelEnv != 1 || !(isSell(m_spmvCfg) || isPat(m_spmvCfg)))) return 0;
+    if (!cg_loop_fits((int)m_n, 0, 1, m_numSms) || !ensureSell()) return 0;  // too large, or rows too uneven
+    if (forced)
+        *layout = isPat(m_spmvCfg) ? 2 : (isSellNarrow(m_spmvCfg) ? 1 : 0);
+    else
+        *layout = m_psState == 1 ? 2 : (m_sellNarrow ? 1 : 0);
+    if (cg_cluster_fits((int)m_n, m_sellTotal)) return 2;
+    return cg_loop_fits((int)m_n, m_sellTotal, m_sellNarrow ? 10 : 12, m_numSms) ? 1 : 0;
+}
+
+// One launch for the vector init, one for the loop.
+void PcgHandle::launchLoopKernel(int form, int layout, uint32_t maxIter) {
+    const int n = (int)m_n, n4 = (int)m_n4;
+    CgState* st = m_state.as<CgState>();
+    check(cg_init_launch(vec_grid(n4, m_numSms), m_stream, n, n4, m_b.as<double>(), m_diag.as<double>(),
+                         m_x.as<double>(), m_r.as<double>(), m_p.as<double>(), m_J.as<double>(), m_Ap.as<double>(),
+                         st, m_partials.as<double>()),
+          "init kernel");
+    const bool pat = layout == 2;
+    LoopArgs a;
+    a.n = n;
+    a.n2 = n4 / 2;
+    a.sliceOff = pat ? m_psSliceOff.as<int>() : m_sliceOff.as<int>();
+    a.sval = pat ? m_psVal.as<double>() : m_sellVal.as<double>();
+    a.col32 = m_sellCol.as<int>();
+    a.col16 = m_sellNarrow ? m_sellCol16.as<int16_t>() : nullptr;
+    a.patLen = m_psPatLen.as<int>();
+    a.patIdx = m_psPatIdx.as<int>();
+    a.patOff = m_psPatOff.as<int>();
+    a.genOff = m_psGenOff.as<int>();
+    a.pat = m_psPat.as<int>();
+    a.gcol = m_psGcol.as<int>();
+    a.x = m_x.as<double>();
+    a.p = m_p.as<double>();
+    a.r = m_r.as<double>();
+    a.J = m_J.as<double>();
+    a.state = st;
+    if (form == 2) {
+        check(cg_cluster_launch(m_stream, layout, a), "cluster loop kernel");
+        return;
+    }
+    a.tag0 = m_loopTag;
+    m_loopTag += maxIter + 1u;
+    check(cg_loop_launch(m_stream, layout, m_numSms, m_loopSync.p, a), "loop kernel");
+}
+
 // The mixed loop's FP32 update after its SpMV: the fused cooperative kernel
 // (update, refresh decision, and the p update when no refresh is due), or,
 // with XJPCG_FUSED_UPDATE=0, the update kernel alone (with pUpdate, the p
@@ -1065,15 +1121,28 @@ Results PcgHandle::run(uint32_t maxIter, double tol) {
     const int n = (int)m_n, n4 = (int)m_n4;
     CgState* st = m_state.as<CgState>();
     double* part = m_partials.as<double>();
-    if (m_useGraph) {
+    int loopLayout = 0;
+    const int loopForm = loopKernel(maxIter, &loopLayout);
+    m_lastOneKernel = loopForm != 0;
+    if (m_useGraph && loopForm == 0) {
         buildGraph();
         cmd.useCond = 1;
         cmd.condHandle = (uint64_t)m_cond;
     }
+    if (loopForm == 1) {
+        alloc(m_loopSync, cg_loop_sync_bytes(m_numSms), "loop kernel posts");
+        // Tags tell this solve's posts from earlier ones'; a launch uses at
+        // most maxIter + 1 of them.  The counters start from 0 each time.
+        const bool wrap = m_loopTag == 0 || (uint64_t)m_loopTag + maxIter + 2 > 0xffffffffull;
+        check(cudaMemsetAsync(m_loopSync.p, 0, wrap ? cg_loop_sync_bytes(m_numSms) : 512, m_stream), "memset");
+        if (wrap) m_loopTag = 1;
+    }
     faultPoint("graph launch");
     check(cudaMemcpyAsync(st, &cmd, sizeof(CgState), cudaMemcpyHostToDevice, m_stream), "state upload");
     check(cudaEventRecord(m_ev0, m_stream), "event");
-    if (m_useGraph) {
+    if (loopForm != 0) {
+        launchLoopKernel(loopForm, loopLayout, maxIter);
+    } else if (m_useGraph) {
         check(cudaGraphLaunch(m_exec, m_stream), "graph launch");
     } else {
         // Host-driven loop: batches of iterations, kernels skip once done.
@@ -2016,7 +2085,8 @@ void PcgHandle::fillInfo(XJPCG_GbInfo_t* info) const {
     info->rrLast = m_lastState.rr;
     info->solveMs = m_lastMs;
     info->loopMode = m_useGraph ? 1u : 0u;
-    info->loopUnroll = m_useGraph ? (uint32_t)kLoopUnroll : 16u;  // the host loop issues batches of 16
+    // 0: the last fp64 solve ran its loop in one kernel; the host loop issues batches of 16
+    info->loopUnroll = m_lastOneKernel ? 0u : (m_useGraph ? (uint32_t)kLoopUnroll : 16u);
     info->kernelsPerIter = m_fusedUpdate ? 2u : 3u;
     if (m_batchCfg >= 0) {
         int t = 0, l = 0;

@@ -206,6 +206,8 @@ class PcgHandle {
                        int mode, const uint32_t* done);
     void ensureVectors(uint32_t n);
     void buildGraph();
+    int loopKernel(uint32_t maxIter, int* layout);
+    void launchLoopKernel(int form, int layout, uint32_t maxIter);
     int cgSpmvMode() const;
     void mixedUpdate(int n4, int vg, CgState* st, double* part, bool pUpdate = true);
     void iterationTail(int n4, CgState* st, double* part);
@@ -284,6 +286,8 @@ class PcgHandle {
     DevBuf m_b, m_diag, m_x, m_r, m_p, m_J, m_Ap;
     DevBuf m_state, m_partials, m_records;
     uint64_t m_recCap = 0;
+    DevBuf m_loopSync;       // counters and posts of the persistent loop kernel
+    uint32_t m_loopTag = 0;  // next unused tag; 0: m_loopSync is to be cleared
     DevBuf m_scratchY;
     // mixed precision
     DevBuf m_state32, m_r32, m_p32, m_d32, m_Ap32, m_J32;
@@ -324,6 +328,7 @@ class PcgHandle {
     cudaGraphConditionalHandle m_condOuter = 0, m_condInner = 0;
     bool m_useGraph = true;
     bool m_fusedUpdate = true;  // XJPCG_FUSED_UPDATE
+    int m_loopKernelEnv = -1;   // XJPCG_LOOP_KERNEL: 0 never, 1 also with a forced sliced layout
     bool m_faultAlloc = false, m_faultLaunch = false, m_initDone = false;  // XJPCG_FAULT hooks
     size_t m_guardBytes = 0;                                   // XJPCG_GUARD_BYTES
     std::vector<std::pair<DevBuf*, std::string>> m_guarded;    // buffers allocated with guards
@@ -333,6 +338,7 @@ class PcgHandle {
     CgState m_lastState{};
     float m_lastMs = 0.f;
     uint32_t m_lastOuter = 0, m_lastInner = 0;
+    bool m_lastOneKernel = false;
 };
 
 }  // namespace xjpcg

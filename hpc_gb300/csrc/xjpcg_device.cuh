@@ -15,6 +15,25 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
     return t;
 }
 
+// The 64-byte record of iteration k (a ring once the buffer is full).
+__device__ __forceinline__ void write_record(CgState* s, uint32_t k, double rr, double rz, double alpha,
+                                             double beta) {
+    if (s->records == nullptr || s->recCap < 2) return;
+    const uint32_t slot = (k + 1u < s->recCap) ? k + 1u : 1u + (k % (s->recCap - 1u));
+    IterRecord rec;
+    rec.id = 0;
+    rec.iter = k;
+    rec.vecSize = s->vecSize;
+    rec.maxIter = s->maxIterP1;
+    rec.tols = s->tols;
+    rec.res = rr;
+    rec.rz = rz;
+    rec.alpha = alpha;
+    rec.beta = beta;
+    rec.clock = globaltimer_ns();
+    s->records[slot] = rec;
+}
+
 // ---------------------------------------------------------------------------
 // Deterministic reductions.  Every sum below has a fixed association order for
 // a fixed launch shape, so results are bitwise stable run to run.

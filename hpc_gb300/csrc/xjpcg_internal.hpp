@@ -164,6 +164,36 @@ cudaError_t cg_update_launch(int grid, cudaStream_t st, int n4, double* r, doubl
 cudaError_t cg_pupdate_launch(int grid, cudaStream_t st, int n4, double* x, double* p, const double* z,
                               CgState* state);
 
+// ---- the fp64 loop as one kernel (cg_loop.cu) ----
+struct LoopArgs {
+    int n = 0, n2 = 0;              // rows; pairs of the padded vectors
+    const int* sliceOff = nullptr;  // sliced layout (of all three kinds)
+    const double* sval = nullptr;
+    const int* col32 = nullptr;      // layout 0
+    const int16_t* col16 = nullptr;  // layout 1
+    const int *patLen = nullptr, *patIdx = nullptr, *patOff = nullptr, *genOff = nullptr, *pat = nullptr,
+              *gcol = nullptr;  // layout 2
+    double *x = nullptr, *p = nullptr;
+    const double *r = nullptr, *J = nullptr;
+    CgState* state = nullptr;
+
+    uint32_t tag0 = 0;  // tags tag0 .. tag0 + iterations - 1 are this launch's own
+    // set by cg_loop_launch
+    int nslices = 0, rows = 0, matBytes = 0;
+    size_t smem = 0;
+    uint32_t* counters = nullptr;
+    ulonglong2* posts = nullptr;
+};
+// stored: entries of the sliced copy; entryBytes: of one of them, its column included
+bool cg_loop_fits(int n, int64_t stored, int entryBytes, int numSms);
+// the same in one cluster of up to 16 CTAs, for small systems
+bool cg_cluster_fits(int n, int64_t stored);
+cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a);
+size_t cg_loop_sync_bytes(int numSms);
+// layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
+// offsets; sync: cg_loop_sync_bytes bytes, the first 512 cleared before each launch.
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a);
+
 // ---- mixed precision, reliable updates (mixed_kernels.cu) ----
 cudaError_t rel_init_launch(int grid, cudaStream_t s, int n, int n4, const double* b, const double* diag, double* x,
                             float* d, float* J, float* r, float* p, CgState* st, double* partials);

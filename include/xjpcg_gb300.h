@@ -31,7 +31,7 @@ typedef struct {
     double bb;             /* b.b of the last solve */
     double rrLast;         /* recursive r.r after the last iteration */
     double solveMs;        /* device time of the last solve (CUDA events) */
-    uint32_t loopMode;     /* 1 = conditional-graph loop, 0 = host-driven */
+    uint32_t loopMode;     /* 1 = loop on the device (conditional graph, or one kernel), 0 = host-driven */
     uint32_t spmvLayout;   /* 0 = CSR staged through shared memory, 1 = sliced (SELL-32), 2 = merge path,
                               3 = sliced with int16 column offsets, 4 = sliced with rows sorted by
                               length (long rows one warp each), 5 = sliced with column offsets
@@ -49,7 +49,8 @@ typedef struct {
     double uploadMs;       /* device time of the last COO matrix upload (H2D, part of m_matProc) */
     double uploadIdxMs;    /* of which the row and column index copies (on the handle's stream) */
     double uploadValMs;    /* of which the value copy (on the side stream, from its start) */
-    uint32_t loopUnroll;   /* iterations per pass of a graph loop's body (kernels past the stop return at once) */
+    uint32_t loopUnroll;   /* iterations per pass of a graph loop's body (kernels past the stop return at once);
+                              0 = the last fp64 solve ran as two launches, the init and the whole loop */
     uint32_t kernelsPerIter; /* kernels per fp64 iteration: 2 (SpMV, fused vector kernel) or 3 (separate) */
 } XJPCG_GbInfo_t;
 
