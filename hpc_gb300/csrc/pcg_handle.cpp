@@ -71,7 +71,11 @@ bool DevBuf::ensure(size_t b, uint64_t* generation, size_t guardBytes) {
 PcgHandle::~PcgHandle() {
     if (m_exec) cudaGraphExecDestroy(m_exec);
     if (m_mixedExec) cudaGraphExecDestroy(m_mixedExec);
-    if (m_batchExec) cudaGraphExecDestroy(m_batchExec);
+    for (int c = 0; c < kBatchClasses; ++c) {
+        if (m_batchStream[c]) cudaStreamDestroy(m_batchStream[c]);
+        if (m_batchJoin[c]) cudaEventDestroy(m_batchJoin[c]);
+    }
+    if (m_batchFork) cudaEventDestroy(m_batchFork);
     if (m_ev0) cudaEventDestroy(m_ev0);
     if (m_ev1) cudaEventDestroy(m_ev1);
     if (m_evUp0) cudaEventDestroy(m_evUp0);
@@ -1729,6 +1733,179 @@ namespace {
 __attribute__((unused)) uint64_t mixKey(uint64_t h, uint64_t v) { return (h ^ v) * 0x100000001b3ull; }
 }  // namespace
 
+// One stream per number of CTAs per system, the larger ahead of the smaller.
+void PcgHandle::batchStreams() {
+    if (m_batchFork == nullptr) {
+        int lowest = 0, highest = 0;
+        check(cudaDeviceGetStreamPriorityRange(&lowest, &highest), "stream priorities");
+        for (int c = 0; c < kBatchClasses; ++c) {
+            check(cudaStreamCreateWithPriority(&m_batchStream[c], cudaStreamNonBlocking, std::max(highest, lowest - c)),
+                  "cudaStreamCreate");
+            check(cudaEventCreateWithFlags(&m_batchJoin[c], cudaEventDisableTiming), "cudaEventCreate");
+        }
+        check(cudaEventCreateWithFlags(&m_batchFork, cudaEventDisableTiming), "cudaEventCreate");
+    }
+}
+
+// Checks the batch's arrays on the device and leaves them in in.*: the
+// caller's own device arrays (when aligned to their elements), or copies of
+// the host arrays in the handle's buffers.
+void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
+                           const double* values, const double* diag, const double* b, bool onDevice, BatchInput& in) {
+    // the system offsets are few: checked on the host
+    in.sys.resize(nsys + 1);
+    check(cudaMemcpy(in.sys.data(), sysRow, sizeof(int32_t) * (nsys + 1), onDevice ? cudaMemcpyDeviceToHost
+                                                                                    : cudaMemcpyHostToHost),
+          "system offsets");
+    if (in.sys[0] != 0) throw InvalidValue("system row offsets must start at 0.");
+    for (uint32_t s = 0; s < nsys; ++s)
+        if (in.sys[s + 1] - in.sys[s] <= 0) throw InvalidValue("every system needs at least one row.");
+    const int total = in.sys[nsys];
+    alloc(m_bSysRow, sizeof(int32_t) * (nsys + 1), "batch offsets");
+    alloc(m_bWidth, sizeof(int32_t) * (2 * (size_t)nsys + 1), "batch widths");
+    check(cudaMemcpyAsync(m_bSysRow.p, in.sys.data(), sizeof(int32_t) * (nsys + 1), cudaMemcpyHostToDevice, m_stream),
+          "H2D");
+    check(cudaMemsetAsync(m_bWidth.p, 0, sizeof(int32_t) * nsys, m_stream), "memset");
+    check(cudaMemsetAsync(m_flags.p, 0, sizeof(int), m_stream), "memset");
+    auto place = [&](DevBuf& buf, const void* src, size_t elem, size_t count, const char* what) -> const void* {
+        if (onDevice && reinterpret_cast<uintptr_t>(src) % elem == 0) return src;
+        alloc(buf, elem * (count + 4), what);
+        check(cudaMemcpyAsync(buf.p, src, elem * count, onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
+                              m_stream),
+              what);
+        return buf.p;
+    };
+    in.rowptr = static_cast<const int*>(place(m_bRowptr, rowPtr, 4, (size_t)total + 1, "batch row pointers"));
+    // the row pointers are checked before any column is read through them
+    int* const entry = m_bWidth.as<int>() + nsys;
+    check(batch_check_rows(m_stream, (int)nsys, total, m_bSysRow.as<int>(), in.rowptr, entry, m_flags.as<int>()),
+          "row pointer check");
+    int flag = 0;
+    in.entry.resize(nsys + 1);
+    check(cudaMemcpyAsync(&flag, m_flags.p, sizeof(int), cudaMemcpyDeviceToHost, m_stream), "D2H");
+    check(cudaMemcpyAsync(in.entry.data(), entry, sizeof(int32_t) * (nsys + 1), cudaMemcpyDeviceToHost, m_stream), "D2H");
+    check(cudaStreamSynchronize(m_stream), "sync");
+    if (flag & 1) throw InvalidValue("row pointers must start at 0.");
+    if (flag & 2) throw InvalidValue("row pointers are not monotone.");
+    const size_t nnz = (size_t)in.entry[nsys];
+    in.col = static_cast<const int*>(place(m_bCol, colIdx, 4, nnz, "batch columns"));
+    in.val = static_cast<const double*>(place(m_bVal, values, 8, nnz, "batch values"));
+    in.b = static_cast<const double*>(place(m_bB, b, 8, (size_t)total, "batch b"));
+    in.diag = static_cast<const double*>(place(m_bDiag, diag, 8, (size_t)total, "batch diag"));
+    check(batch_widths(m_stream, (int)nsys, total, m_bSysRow.as<int>(), in.rowptr, in.col, m_bWidth.as<int>(),
+                       m_flags.as<int>()),
+          "column check");
+    in.width.resize(nsys);
+    check(cudaMemcpyAsync(&flag, m_flags.p, sizeof(int), cudaMemcpyDeviceToHost, m_stream), "D2H");
+    check(cudaMemcpyAsync(in.width.data(), m_bWidth.p, sizeof(int32_t) * nsys, cudaMemcpyDeviceToHost, m_stream), "D2H");
+    check(cudaStreamSynchronize(m_stream), "sync");
+    if (flag & 4) throw InvalidValue("a column index lies outside its system.");
+}
+
+// The batch with every system in shared memory (batched_cluster.cu).  False
+// when that is not the way for it (nothing has run then).
+bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol, bool mixed) {
+    const uint32_t nsys = (uint32_t)in.width.size();
+    const std::vector<int32_t>&hSys = in.sys, &width = in.width;
+    BatchClusterArgs a;
+    a.sysRow = m_bSysRow.as<int>();
+    a.rowptr = in.rowptr;
+    a.col = in.col;
+    a.val = in.val;
+    a.b = in.b;
+    a.diag = in.diag;
+    // Class of a system: 0 .. 4 small CTAs, 1, 2, 4, 8 or 16 of them, 5 .. 9 wide
+    // ones.  The first that holds it; while the GPU has room, twice the CTAs.
+    auto ctasOf = [](int c) { return 1 << (c % 5); };
+    auto smsOf = [&](int c) { return ctasOf(c) / (c < 5 ? (mixed ? 6.0 : 5.0) : (mixed ? 3.0 : 2.0)); };
+    auto fits = [&](uint32_t s, int c) {
+        const int n = hSys[s + 1] - hSys[s];
+        const int rows = 32 * (((n + 31) / 32 + ctasOf(c) - 1) / ctasOf(c));
+        return rows <= batch_cluster_rows(mixed, c < 5) &&
+               batch_cluster_smem(mixed, n, std::max(1, width[s]), ctasOf(c)) <= batch_cluster_room(mixed, c < 5);
+    };
+    std::vector<uint8_t> cls(nsys);
+    double sms = 0.0;
+    for (uint32_t s = 0; s < nsys; ++s) {
+        int c = 0;
+        while (c < kBatchClasses && !fits(s, c)) ++c;
+        if (c == kBatchClasses || hSys[s + 1] - hSys[s] > 65536) return false;
+        cls[s] = (uint8_t)c;
+        sms += smsOf(c);
+    }
+    for (bool more = true; more && 2.0 * sms <= m_numSms;) {
+        more = false;
+        sms = 0.0;
+        for (uint32_t s = 0; s < nsys; ++s) {
+            if (cls[s] % 5 < 4 && hSys[s + 1] - hSys[s] > 128 * ctasOf(cls[s])) {
+                ++cls[s];
+                more = true;
+            }
+            sms += smsOf(cls[s]);
+        }
+    }
+    // sms: SMs that the batch would fill at once.  A system advances faster here
+    // than on one CTA of the other kernels, but takes up to twice (FP64) the
+    // SMs' time, so this is the way until the SMs run out of time.  fp64 / mixed,
+    // kernel ms here against there, and how often the batch fills the GPU:
+    //   60 systems of 1,000 - 5,000 rows    3.3 / 2.0    7.8 / 4.7   0.5 / 0.8
+    //   900 of 100 - 400                    0.95 / 0.48  0.95 / 0.81 1.2 / 1.0
+    //   700 of 300 - 2,000                  3.9 / 2.3    4.0 / 2.8   2.2 / 1.9
+    //   600 of 1,000 - 2,500                8.4          5.6         3.7
+    //   300 of 200 - 20,000                 24.6 / 10    18 / 14     4.1 / 3.5
+    //   2,000 of 200 - 20,000               145 / 57     66 / 37     28 / 24
+    if (sms > (mixed ? 4.0 : 2.5) * m_numSms) return false;
+    alloc(m_bOrder, sizeof(int32_t) * nsys, "batch order");
+    std::vector<int32_t> order(nsys);
+    for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
+    // by class, the largest first in each
+    std::stable_sort(order.begin(), order.end(), [&](int32_t p, int32_t q) {
+        if (cls[p] != cls[q]) return cls[p] > cls[q];
+        return hSys[p + 1] - hSys[p] > hSys[q + 1] - hSys[q];
+    });
+    check(cudaMemcpyAsync(m_bOrder.p, order.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice, m_stream), "H2D");
+    a.width = m_bWidth.as<int>();
+    a.x = m_bX.as<double>();
+    a.res = m_bRes.as<BatchResult>();
+    a.maxIterP1 = maxIter + 1u;
+    a.tol = tol;
+    {
+        const double delta = envDouble("XJPCG_RELIABLE_DELTA", 0.01);
+        a.delta2 = delta * delta;
+    }
+    batchStreams();
+    faultPoint("graph launch");
+    check(cudaEventRecord(m_ev0, m_stream), "event");
+    // a system whose kernel gave up leaves its result as it is: failed
+    check(cudaMemsetAsync(m_bRes.p, 0xff, sizeof(BatchResult) * nsys, m_stream), "memset");
+    check(cudaEventRecord(m_batchFork, m_stream), "event");
+    cudaError_t err = cudaSuccess;
+    m_batchClusterCtas = 0;
+    for (uint32_t at = 0; at < nsys;) {
+        const int c = cls[order[at]], teamOf = ctasOf(c);
+        uint32_t end = at;
+        size_t smem = 0;
+        for (; end < nsys && cls[order[end]] == c; ++end) {
+            const int s = order[end];
+            smem = std::max(smem, batch_cluster_smem(mixed, hSys[s + 1] - hSys[s], std::max(1, width[s]), teamOf));
+        }
+        a.order = m_bOrder.as<int>() + at;
+        a.ctas = teamOf;
+        if (err == cudaSuccess) err = cudaStreamWaitEvent(m_batchStream[c], m_batchFork, 0);
+        if (err == cudaSuccess) err = batch_cluster_launch(m_batchStream[c], mixed, c < 5, (int)(end - at), smem, a);
+        // joined whatever happened: nothing of the batch outlives the call
+        cudaEventRecord(m_batchJoin[c], m_batchStream[c]);
+        cudaStreamWaitEvent(m_stream, m_batchJoin[c], 0);
+        m_batchClusterCtas += (int)(end - at) * teamOf;
+        at = end;
+    }
+    check(cudaEventRecord(m_ev1, m_stream), "event");
+    check(cudaEventSynchronize(m_ev1), "event");
+    check(err, "batched cluster kernel");
+    check(cudaEventElapsedTime(&m_batchMs, m_ev0, m_ev1), "event");
+    return true;
+}
+
 uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
                                const double* values, const double* diag, const double* b, double* x,
                                uint32_t maxIter, double tol, int precision, BatchResult* results, bool onDevice) {
@@ -1736,68 +1913,56 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     if (nsys == 0) throw InvalidValue("number of systems is zero.");
     if (precision != 0 && precision != 1) throw InvalidValue("precision must be 0 (fp64) or 1 (mixed).");
     const bool mixed = precision == 1;
-    // System and row offsets are small: validate them on the host.
-    std::vector<int32_t> hSys(nsys + 1);
-    check(cudaMemcpy(hSys.data(), sysRow, sizeof(int32_t) * (nsys + 1), onDevice ? cudaMemcpyDeviceToHost
-                                                                                  : cudaMemcpyHostToHost),
-          "system offsets");
-    if (hSys[0] != 0) throw InvalidValue("system row offsets must start at 0.");
-    int maxN = 0;
-    for (uint32_t s = 0; s < nsys; ++s) {
-        const int ns = hSys[s + 1] - hSys[s];
-        if (ns <= 0) throw InvalidValue("every system needs at least one row.");
-        maxN = std::max(maxN, ns);
-    }
+    BatchInput in;
+    batchInput(nsys, sysRow, rowPtr, colIdx, values, diag, b, onDevice, in);
+    const std::vector<int32_t>&hSys = in.sys, &entry = in.entry;
     const int total = hSys[nsys];
-    std::vector<int32_t> hRp((size_t)total + 1);
-    check(cudaMemcpy(hRp.data(), rowPtr, sizeof(int32_t) * ((size_t)total + 1),
-                     onDevice ? cudaMemcpyDeviceToHost : cudaMemcpyHostToHost),
-          "row pointers");
-    if (hRp[0] != 0) throw InvalidValue("row pointers must start at 0.");
-    int maxRowLen = 0;
-    for (int i = 0; i < total; ++i) {
-        if (hRp[i + 1] < hRp[i]) throw InvalidValue("row pointers are not monotone.");
-        maxRowLen = std::max(maxRowLen, hRp[i + 1] - hRp[i]);
-    }
-    const int64_t nnz = hRp[total];
+    const int64_t nnz = entry[nsys];
+    int maxN = 0;
+    for (uint32_t s = 0; s < nsys; ++s) maxN = std::max(maxN, hSys[s + 1] - hSys[s]);
+    const int maxRowLen = *std::max_element(in.width.begin(), in.width.end());
+    alloc(m_bX, sizeof(double) * ((size_t)total + 4), "batch vector");
+    alloc(m_bRes, sizeof(BatchResult) * nsys, "batch results");
+    // Forced kernel shapes and layouts take the kernels they name.
+    const int forced = envInt("XJPCG_BATCH_CFG", -1);
+    const bool forcedShape = forced >= 0 || envInt("XJPCG_BATCH_SLICED", 1) == 0 || envInt("XJPCG_BATCH_PATTERNS", 1) == 0;
+    m_batchClusterCtas = 0;
+    if (!forcedShape && envInt("XJPCG_BATCH_CLUSTERS", 1) != 0 && batchClusters(in, maxIter, tol, mixed))
+        return batchResults(nsys, total, x, tol, results, onDevice);
     // Queue order: largest systems first so the long solves start early.
     std::vector<int32_t> order(nsys);
     for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
-    std::stable_sort(order.begin(), order.end(), [&](int32_t a, int32_t c) {
-        return (hRp[hSys[a + 1]] - hRp[hSys[a]]) > (hRp[hSys[c + 1]] - hRp[hSys[c]]);
-    });
-    const size_t vb = sizeof(double) * ((size_t)total + 4), fb = sizeof(float) * ((size_t)total + 4);
-    alloc(m_bSysRow, sizeof(int32_t) * (nsys + 1), "batch offsets");
-    alloc(m_bOrder, sizeof(int32_t) * nsys, "batch order");
-    alloc(m_bRowptr, sizeof(int32_t) * ((size_t)total + 1), "batch row pointers");
-    alloc(m_bCol, sizeof(int32_t) * ((size_t)nnz + 4), "batch columns");
-    alloc(m_bVal, sizeof(double) * ((size_t)nnz + 4), "batch values");
-    for (DevBuf* v : {&m_bB, &m_bDiag, &m_bX, &m_bR, &m_bAp, &m_bJ, &m_bP}) alloc(*v, vb, "batch vector");
-    if (mixed) {
-        alloc(m_bVal32, sizeof(float) * ((size_t)nnz + 4), "batch fp32 values");
-        for (DevBuf* v : {&m_bR32, &m_bD32, &m_bAp32, &m_bJ32, &m_bP32}) alloc(*v, fb, "batch vector");
+    std::stable_sort(order.begin(), order.end(),
+                     [&](int32_t a, int32_t c) { return entry[a + 1] - entry[a] > entry[c + 1] - entry[c]; });
+    // Systems too long for one CTA next to the batch's average share can go to
+    // teams of CTAs: their work, entries x sqrt(rows) for want of iteration
+    // counts, is above a quarter of the work per SM.  fp64 / mixed ms with 0.40 /
+    // 0.30 / 0.22 of it: 1,024 systems of 200 - 20,000 rows 45.8 / 46.3 / 46.3 and
+    // 24.3 / 23.9 / 24.6; 2,000 of them 71 / 67 / 63 and 32.0 / 33.6 / 35.2.
+    std::vector<uint8_t> isLong(nsys, 0);
+    {
+        auto workOf = [&](uint32_t i) {
+            const double n = hSys[i + 1] - hSys[i];
+            return ((double)(entry[i + 1] - entry[i]) + 7.0 * n) * std::sqrt(n);
+        };
+        double allWork = 0.0;
+        for (uint32_t i = 0; i < nsys; ++i) allWork += workOf(i);
+        const double share = 0.25 * allWork / m_numSms;
+        for (uint32_t i = 0; i < nsys; ++i) isLong[i] = workOf(i) > share && hSys[i + 1] - hSys[i] > 2048 ? 1 : 0;
     }
-    alloc(m_bRes, sizeof(BatchResult) * nsys, "batch results");
+    std::vector<int32_t> teamOrder(order);
+    std::stable_sort(teamOrder.begin(), teamOrder.end(), [&](int32_t p, int32_t q) { return isLong[p] < isLong[q]; });
+    uint32_t singles = (uint32_t)std::count(isLong.begin(), isLong.end(), 0);
+    const size_t vb = sizeof(double) * ((size_t)total + 4), fb = sizeof(float) * ((size_t)total + 4);
+    alloc(m_bOrder, sizeof(int32_t) * 2 * nsys, "batch order");
+    for (DevBuf* v : {&m_bR, &m_bAp, &m_bJ, &m_bP}) alloc(*v, vb, "batch vector");
+    if (mixed)
+        for (DevBuf* v : {&m_bR32, &m_bD32, &m_bAp32, &m_bJ32, &m_bP32}) alloc(*v, fb, "batch vector");
     alloc(m_bQueue, 16, "batch queue");
-    const cudaMemcpyKind k = onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
-    check(cudaMemcpyAsync(m_bSysRow.p, hSys.data(), sizeof(int32_t) * (nsys + 1), cudaMemcpyHostToDevice, m_stream),
-          "H2D");
     check(cudaMemcpyAsync(m_bOrder.p, order.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice, m_stream), "H2D");
-    check(cudaMemcpyAsync(m_bRowptr.p, hRp.data(), sizeof(int32_t) * ((size_t)total + 1), cudaMemcpyHostToDevice,
+    check(cudaMemcpyAsync(m_bOrder.as<int>() + nsys, teamOrder.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice,
                           m_stream),
           "H2D");
-    check(cudaMemcpyAsync(m_bCol.p, colIdx, sizeof(int32_t) * nnz, k, m_stream), "copy columns");
-    check(cudaMemcpyAsync(m_bVal.p, values, sizeof(double) * nnz, k, m_stream), "copy values");
-    check(cudaMemcpyAsync(m_bB.p, b, sizeof(double) * total, k, m_stream), "copy b");
-    check(cudaMemcpyAsync(m_bDiag.p, diag, sizeof(double) * total, k, m_stream), "copy diag");
-    check(batch_validate_columns(m_stream, (int)nsys, m_bSysRow.as<int>(), m_bRowptr.as<int>(), m_bCol.as<int>(),
-                                 m_flags.as<int>()),
-          "column check");
-    int bad = 0;
-    check(cudaMemcpyAsync(&bad, m_flags.p, sizeof(int), cudaMemcpyDeviceToHost, m_stream), "D2H");
-    check(cudaStreamSynchronize(m_stream), "sync");
-    if (bad) throw InvalidValue("a column index lies outside its system.");
-    if (mixed) check(convert_f64_to_f32(m_stream, nnz, m_bVal.as<double>(), m_bVal32.as<float>()), "fp32 values");
 
     // Per-system SELL-32 copy for the sliced kernels: 32-row slices of each
     // system, values slice-column-major, 16-bit local columns.  Offered when
@@ -1822,7 +1987,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
               "H2D");
         check(cudaMemsetAsync(m_bsLen.p, 0, sizeof(int32_t) * ((size_t)nsl + 1), m_stream), "memset");
         check(batch_sell_widths(m_stream, (int)nsys, nsl, m_bSysRow.as<int>(), m_bsBase.as<int>(),
-                                m_bRowptr.as<int>(), m_bCol.as<int>(), m_bsLen.as<int>(), m_bsOff.as<int>(),
+                                in.rowptr, in.col, m_bsLen.as<int>(), m_bsOff.as<int>(),
                                 m_bsScan.as<int>(), m_bsPatLen.as<int>(), m_bsPatOff.as<int>(),
                                 envInt("XJPCG_BATCH_PATTERNS", 1) != 0),
               "batch slices");
@@ -1840,30 +2005,34 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         if (mixed) {
             alloc(m_bsVal32, sizeof(float) * ((size_t)stored + 32), "batch sliced fp32 values");
             check(batch_sell_fill<float>(m_stream, (int)nsys, nsl, m_bSysRow.as<int>(), m_bsBase.as<int>(),
-                                         m_bRowptr.as<int>(), m_bCol.as<int>(), m_bVal.as<double>(), m_bsOff.as<int>(),
+                                         in.rowptr, in.col, in.val, m_bsOff.as<int>(),
                                          m_bsPatLen.as<int>(), m_bsPatOff.as<int>(), m_bsVal32.as<float>(),
                                          m_bsCol.as<uint16_t>()),
                   "batch sliced fp32 fill");
         } else {
             alloc(m_bsVal, sizeof(double) * ((size_t)stored + 32), "batch sliced values");
             check(batch_sell_fill<double>(m_stream, (int)nsys, nsl, m_bSysRow.as<int>(), m_bsBase.as<int>(),
-                                          m_bRowptr.as<int>(), m_bCol.as<int>(), m_bVal.as<double>(),
+                                          in.rowptr, in.col, in.val,
                                           m_bsOff.as<int>(), m_bsPatLen.as<int>(), m_bsPatOff.as<int>(),
                                           m_bsVal.as<double>(), m_bsCol.as<uint16_t>()),
                   "batch sliced fill");
         }
     }
 
+    if (!sliced) singles = nsys;  // the team kernels read the sliced copy
+    const bool csr = !sliced || (forced >= 0 && !batch_config_sliced(forced % batch_num_configs()));
+    if (mixed && csr) {  // the CSR kernels read FP32 values
+        alloc(m_bVal32, sizeof(float) * ((size_t)nnz + 4), "batch fp32 values");
+        check(convert_f64_to_f32(m_stream, nnz, in.val, m_bVal32.as<float>()), "fp32 values");
+    }
     BatchLaunch L;
-    L.nsys = (int)nsys;
     L.sysRow = m_bSysRow.as<int>();
-    L.order = m_bOrder.as<int>();
-    L.rowptr = m_bRowptr.as<int>();
-    L.col = m_bCol.as<int>();
-    L.val = m_bVal.as<double>();
-    L.val32 = mixed ? m_bVal32.as<float>() : nullptr;
-    L.b = m_bB.as<double>();
-    L.diag = m_bDiag.as<double>();
+    L.rowptr = in.rowptr;
+    L.col = in.col;
+    L.val = in.val;
+    L.val32 = mixed && csr ? m_bVal32.as<float>() : nullptr;
+    L.b = in.b;
+    L.diag = in.diag;
     L.x = m_bX.as<double>();
     L.r = m_bR.as<double>();
     L.Ap = m_bAp.as<double>();
@@ -1908,15 +2077,22 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         rows = std::min(maxN, rows);
         if (std::find(smemRows.begin(), smemRows.end(), rows) == smemRows.end()) smemRows.push_back(rows);
     }
+    // 0: no teams, 1: always, -1: where they are faster
+    const int teamsEnv = envInt("XJPCG_BATCH_TEAMS", forcedShape ? 0 : -1);
     const uint64_t key = mixKey(mixKey(mixKey(nsys, (uint64_t)total), (uint64_t)nnz),
-                                (uint64_t)precision + 7 + (sliced ? 1000 : 0));
-    const int forced = envInt("XJPCG_BATCH_CFG", -1);
-    auto runOnce = [&](int cfg, int rows, float* ms) {
+                                (uint64_t)precision + 7 + (sliced ? 1000 : 0) + 10000 * (uint64_t)(teamsEnv + 1));
+    // One batch; teams: CTAs per long system, 0 for none.
+    auto runOnce = [&](int cfg, int rows, int teams, float* ms) {
         check(cudaMemsetAsync(m_bQueue.p, 0, 16, m_stream), "memset queue");
         check(cudaEventRecord(m_ev0, m_stream), "event");
         int grid = 0;
-        check(batch_launch(cfg, mixed, m_numSms, rows, m_stream, L, &grid), "batched kernel");
+        L.order = m_bOrder.as<int>() + (teams ? nsys : 0);
+        L.nsys = (int)(teams ? singles : nsys);
+        const cudaError_t err =
+            teams ? batch_team_launch(m_stream, mixed, teams, m_numSms, rows, L, (int)(nsys - singles), &grid)
+                  : batch_launch(cfg, mixed, m_numSms, rows, m_stream, L, &grid);
         check(cudaEventRecord(m_ev1, m_stream), "event");
+        check(err, "batched kernel");
         check(cudaEventSynchronize(m_ev1), "event");
         check(cudaEventElapsedTime(ms, m_ev0, m_ev1), "event");
         m_batchGrid = grid;
@@ -1925,51 +2101,50 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     if (forced >= 0 && forced < ncfg * (int)smemRows.size()) {
         m_batchCfg = forced % ncfg;
         m_batchSmemRows = smemRows[forced / ncfg];
+        m_batchTeams = teamsEnv == 1 && singles < nsys ? 4 : 0;
     } else if (m_batchKey != key || m_batchCfg < 0) {
+        // The sliced shapes (the CSR ones where there is no sliced copy: on
+        // 1,024 systems they took 1.1 to 1.9 times as long), with and without
+        // teams.
         m_batchTuneMs.assign((size_t)ncfg * smemRows.size(), -1.f);
         float best = 1e30f;
+        auto consider = [&](int c, int rows, int teams, float* told) {
+            float ms = 0;
+            runOnce(c, rows, teams, &ms);
+            *told = *told < 0.f ? ms : std::min(*told, ms);
+            if (ms < best) {
+                best = ms;
+                m_batchCfg = c;
+                m_batchSmemRows = rows;
+                m_batchTeams = teams;
+            }
+        };
+        const bool canTeam = singles < nsys && teamsEnv != 0;
         for (size_t si = 0; si < smemRows.size(); ++si)
             for (int c = 0; c < ncfg; ++c) {
-                if (batch_config_sliced(c) && !sliced) continue;
-                float ms = 0;
-                runOnce(c, smemRows[si], &ms);
-                m_batchTuneMs[si * ncfg + c] = ms;
-                if (ms < best) {
-                    best = ms;
-                    m_batchCfg = c;
-                    m_batchSmemRows = smemRows[si];
-                }
+                if (batch_config_sliced(c) != sliced || (canTeam && teamsEnv == 1)) continue;
+                consider(c, smemRows[si], 0, &m_batchTuneMs[si * ncfg + c]);
             }
+        if (canTeam) {  // 512-thread CTAs, 4,096 rows or 44 KB of p
+            int c512 = 0;
+            for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
+                batch_config_shape(c, &t, &g);
+                if (batch_config_sliced(c) && t == 512) c512 = c;
+            }
+            float unused = -1.f;
+            for (int rows : {std::min(maxN, 4096), std::min(maxN, (int)(44 * 1024 / esz))})
+                for (int teams : {2, 4, 8}) consider(c512, rows, teams, &unused);
+        }
         m_batchKey = key;
     }
-    // The production launch is a CUDA graph (queue reset + persistent
-    // kernel), instantiated once per shape and buffer set.
-    const uint64_t gkey = mixKey(mixKey(mixKey(key, (uint64_t)m_batchCfg), (uint64_t)m_batchSmemRows), m_generation);
-    if (!m_batchExec || m_batchExecKey != gkey) {
-        if (m_batchExec) {
-            cudaGraphExecDestroy(m_batchExec);
-            m_batchExec = nullptr;
-        }
-        cudaGraph_t g = nullptr;
-        check(cudaStreamBeginCapture(m_stream, cudaStreamCaptureModeThreadLocal), "capture");
-        int grid = 0;
-        cudaError_t e1 = cudaMemsetAsync(m_bQueue.p, 0, 16, m_stream);
-        cudaError_t e2 = e1 == cudaSuccess ? batch_launch(m_batchCfg, mixed, m_numSms, m_batchSmemRows, m_stream, L, &grid)
-                                           : e1;
-        cudaError_t e3 = cudaStreamEndCapture(m_stream, &g);
-        check(e2, "batched kernel capture");
-        check(e3, "capture end");
-        check(cudaGraphInstantiate(&m_batchExec, g, 0), "graph instantiate");
-        cudaGraphDestroy(g);
-        m_batchGrid = grid;
-        m_batchExecKey = gkey;
-    }
-    faultPoint("graph launch");
-    check(cudaEventRecord(m_ev0, m_stream), "event");
-    check(cudaGraphLaunch(m_batchExec, m_stream), "graph launch");
-    check(cudaEventRecord(m_ev1, m_stream), "event");
-    check(cudaEventSynchronize(m_ev1), "event");
-    check(cudaEventElapsedTime(&m_batchMs, m_ev0, m_ev1), "event");
+    faultPoint("batched launch");
+    runOnce(m_batchCfg, m_batchSmemRows, m_batchTeams, &m_batchMs);
+    return batchResults(nsys, total, x, tol, results, onDevice);
+}
+
+// Results and x of the batch that has run; the number of systems that failed.
+uint32_t PcgHandle::batchResults(uint32_t nsys, int total, double* x, double tol, BatchResult* results,
+                                 bool onDevice) {
     std::vector<BatchResult> hr(nsys);
     check(cudaMemcpyAsync(results ? (void*)results : (void*)hr.data(), m_bRes.p, sizeof(BatchResult) * nsys,
                           cudaMemcpyDeviceToHost, m_stream),
@@ -2095,8 +2270,13 @@ void PcgHandle::fillInfo(XJPCG_GbInfo_t* info) const {
         info->batchLanes = (uint32_t)l;
         info->batchSliced = batch_config_sliced(m_batchCfg) ? 1u : 0u;
     }
-    info->batchSmemRows = (uint32_t)m_batchSmemRows;
-    info->batchGrid = (uint32_t)m_batchGrid;
+    if (m_batchClusterCtas > 0) {
+        info->batchThreads = 256u;
+        info->batchLanes = 1u;
+        info->batchSliced = 1u;
+    }
+    info->batchSmemRows = m_batchClusterCtas > 0 ? 0u : (uint32_t)m_batchSmemRows;
+    info->batchGrid = (uint32_t)(m_batchClusterCtas > 0 ? m_batchClusterCtas : m_batchGrid);
     info->batchMs = m_batchMs;
     const int c32 = m_spmvCfg32 >= 0 ? m_spmvCfg32 : m_spmvCfg;
     info->spmvLayout32 = layoutCode(c32);

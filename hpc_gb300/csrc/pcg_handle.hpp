@@ -207,6 +207,17 @@ class PcgHandle {
     void ensureVectors(uint32_t n);
     void buildGraph();
     int loopKernel(uint32_t maxIter, int* layout);
+    // A batch's arrays on the device, and what the host needs of them.
+    struct BatchInput {
+        std::vector<int32_t> sys, entry, width;  // first row and entry of each system (and the ends), longest row
+        const int *rowptr = nullptr, *col = nullptr;
+        const double *val = nullptr, *diag = nullptr, *b = nullptr;
+    };
+    void batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
+                    const double* values, const double* diag, const double* b, bool onDevice, BatchInput& in);
+    bool batchClusters(const BatchInput& in, uint32_t maxIter, double tol, bool mixed);
+    void batchStreams();
+    uint32_t batchResults(uint32_t nsys, int total, double* x, double tol, BatchResult* results, bool onDevice);
     void launchLoopKernel(int form, int layout, uint32_t maxIter);
     int cgSpmvMode() const;
     void mixedUpdate(int n4, int vg, CgState* st, double* part, bool pUpdate = true);
@@ -316,8 +327,12 @@ class PcgHandle {
     uint64_t m_batchKey = 0;
     float m_batchMs = 0.f;
     std::vector<float> m_batchTuneMs;
-    cudaGraphExec_t m_batchExec = nullptr;  // queue reset + persistent kernel
-    uint64_t m_batchExecKey = 0;
+    DevBuf m_bWidth;                                     // longest row of each system
+    static constexpr int kBatchClasses = 10;             // 1, 2, 4, 8, 16 small CTAs per system, then wide ones
+    cudaStream_t m_batchStream[kBatchClasses] = {};      // one per class, created on first use
+    cudaEvent_t m_batchFork = nullptr, m_batchJoin[kBatchClasses] = {};
+    int m_batchClusterCtas = 0;                          // CTAs of the last cluster batch, 0: the other kernels ran
+    int m_batchTeams = 0;                                // the tuner's choice: CTAs per long system, 0: one each
 
     // graph
     cudaGraphExec_t m_exec = nullptr;

@@ -253,8 +253,32 @@ struct BatchLaunch {
     const int* sysPat = nullptr;  // per system: pattern length, then kBatchPatMax offsets
 };
 int batch_num_configs();
-cudaError_t batch_validate_columns(cudaStream_t st, int nsys, const int* sysRow, const int* rowptr, const int* col,
-                                   int* flag);
+// Systems held in shared memory, one CTA or cluster each (batched_cluster.cu).
+struct BatchClusterArgs {
+    const int* sysRow = nullptr;
+    const int* order = nullptr;  // the systems of this launch
+    const int* width = nullptr;  // longest row of each system
+    const int* rowptr = nullptr;
+    const int* col = nullptr;
+    const double *val = nullptr, *b = nullptr, *diag = nullptr;
+    double* x = nullptr;
+    BatchResult* res = nullptr;
+    uint32_t maxIterP1 = 0;
+    double tol = 0.0, delta2 = 0.0;
+    int ctas = 1;  // CTAs per system: 1 .. 16
+};
+int batch_cluster_rows(bool mixed, bool small);     // most rows of a CTA
+size_t batch_cluster_room(bool mixed, bool small);  // most shared memory of a CTA
+size_t batch_cluster_smem(bool mixed, int n, int width, int ctas);
+// a.ctas CTAs per system, small or wide
+cudaError_t batch_cluster_launch(cudaStream_t st, bool mixed, bool small, int systems, size_t smem,
+                                 const BatchClusterArgs& a);
+// flag |= 1: rowptr[0] != 0, 2: not monotone; entry[s] = rowptr[sysRow[s]], nsys + 1 of them
+cudaError_t batch_check_rows(cudaStream_t st, int nsys, int total, const int* sysRow, const int* rowptr, int* entry,
+                             int* flag);
+// width[s]: longest row of system s (cleared before); flag |= 4: a column outside its system
+cudaError_t batch_widths(cudaStream_t st, int nsys, int total, const int* sysRow, const int* rowptr, const int* col,
+                         int* width, int* flag);
 void batch_config_shape(int cfg, int* threads, int* lanes);
 bool batch_config_sliced(int cfg);  // the kernel reads the per-system SELL-32 copy
 // Shared column offsets per slice of the batched SELL-32 copy: at most this
@@ -271,6 +295,9 @@ template <typename VT>
 cudaError_t batch_sell_fill(cudaStream_t st, int nsys, int nslices, const int* sysRow, const int* sliceBase,
                             const int* rowptr, const int* col, const double* val, const int* sliceOff,
                             const int* patLen, const int* patOff, VT* sval, uint16_t* scol);
+// the nteam systems after the first nsys of L.order on clusters of ctas (2, 4, 8) CTAs, then the others
+cudaError_t batch_team_launch(cudaStream_t st, bool mixed, int ctas, int numSms, int smemRows, const BatchLaunch& L,
+                              int nteam, int* gridOut);
 cudaError_t batch_launch(int cfg, bool mixed, int numSms, int smemRows, cudaStream_t st, const BatchLaunch& L,
                          int* gridOut);
 
