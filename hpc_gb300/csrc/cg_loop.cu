@@ -23,11 +23,12 @@
 //             32^3   14.7 /  9.5 /  -                 16^3  16.9 / 10.9 / 8.4
 //             48^3   18.1 / 12.3 /  -                 32^3  18.0 / 11.7 /  -
 //             64^3   25.5 / 17.5 /  -                 48^3  24.2 / 17.9 /  -
-//             80^3   31.3 / 26.7 /  -                 60^3  33.0 / 34.6 /  -
+//             80^3   31.3 / 26.7 /  -                 60^3  32.7 / 30.2 /  -
 //
 // Every row is summed in its stored order, as in the sliced SpMV kernels; the
 // dot products are summed per thread, per warp, per CTA and over the CTAs, in
-// an order that depends on n alone, so a solve is bitwise reproducible.
+// an order that depends on n and the entries stored, not on the layout, so a solve
+// is bitwise reproducible.
 #include <algorithm>
 
 #include "xjpcg_device.cuh"
@@ -36,9 +37,9 @@
 namespace xjpcg {
 
 namespace {
-constexpr int kLoopThreads = 448;   // at most; 144 registers (512 threads spilled and took 3 to 6 % longer)
 constexpr int kVecThreads = 256;    // threads that update r and z: enough to fill the FP64 pipe, and every warp costs two sums
 constexpr int kCols = 8;            // stored columns per step of a row: their loads go out together
+constexpr int kPipeCols = 7;        // the same where the next step is loaded ahead (27 = 7 + 7 + 7 + 6)
 constexpr int kPosts = 5;           // posts a lane reads at once: 152 CTAs in one step
 constexpr uint64_t kLoopBudgetNs = 2000000000ull;  // 2 s
 constexpr size_t kLoopSmem = 226 * 1024;
@@ -126,6 +127,11 @@ __device__ __forceinline__ double grid_total(double s, ulonglong2* posts, uint32
 }
 }  // namespace
 
+struct Cols {
+    double v[kPipeCols];
+    int c[kPipeCols];
+};
+
 // CTA q owns a contiguous run of slices (so neighbouring rows' gathers meet in
 // its L1).  Per iteration:
 //   Ap = A p into sz, p.Ap        -> grid sum, alpha
@@ -134,8 +140,9 @@ __device__ __forceinline__ double grid_total(double s, ulonglong2* posts, uint32
 //   p = z + beta p, also to global -> barrier (release / acquire)
 // Only the last needs fences: the posts of the sums carry their own tags.
 // LAY: 0 int32 columns, 1 int16 offsets, 2 slice-shared offsets.
-template <int LAY>
-__global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
+// NT: threads at most.  PIPE: rows beyond shared memory load a step ahead.
+template <int LAY, int NT, bool PIPE>
+__global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
     __shared__ double sAlpha, sBeta, sRz, sRr;
     __shared__ int sGo[3], sOn;
@@ -219,6 +226,31 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     int nwUp = 1;
     while (nwUp < nw) nwUp *= 2;
 
+    // PIPE: the first streamed step of an iteration is loaded before the barrier
+    // that ends the one before, as it does not depend on p
+    const int firstStreamed = nOn + (wid - nOn % nw + nw) % nw;
+    auto ahead = [&](Cols& c, int ls, int j) {
+        const int4 md = meta[ls];
+        const int rem = md.y - j, row = row0 + ls * 32 + lane;
+        const double* vp = a.sval + md.x + j * 32 + lane;
+        if (rem >= kPipeCols) {
+#pragma unroll
+            for (int u = 0; u < kPipeCols; ++u) {
+                c.v[u] = ld_val(vp + u * 32);
+                c.c[u] = column(md, row, j + u);
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < kPipeCols; ++u)
+                if (u < rem) {
+                    c.v[u] = ld_val(vp + u * 32);
+                    c.c[u] = column(md, row, j + u);
+                }
+        }
+    };
+    Cols colsA, colsB;
+    if (PIPE && firstStreamed < ns) ahead(colsA, firstStreamed, 0);
+
     uint32_t k = 0;
     bool ok = true;
     for (;;) {
@@ -254,7 +286,49 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
             sz[r] = row < a.n ? acc : 0.0;
             if (row < a.n) dacc = fma(sp[r], acc, dacc);
         }
-        for (; ls < ns; ls += nw) {
+        if (PIPE) {
+            // the others stream: the next step's values and columns are on their
+            // way while this one's p is gathered and summed
+            double acc = 0.0;
+            int j = 0;
+            auto step = [&](const Cols& c, Cols& next) {
+                const int rem = meta[ls].y - j;
+                double xv[kPipeCols];
+                if (rem >= kPipeCols) {
+#pragma unroll
+                    for (int u = 0; u < kPipeCols; ++u) xv[u] = a.p[c.c[u]];
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kPipeCols; ++u)
+                        if (u < rem) xv[u] = a.p[c.c[u]];
+                }
+                const bool last = rem <= kPipeCols;
+                const int lsn = last ? ls + nw : ls, jn = last ? 0 : j + kPipeCols;
+                if (lsn < ns) ahead(next, lsn, jn);
+                if (rem >= kPipeCols) {
+#pragma unroll
+                    for (int u = 0; u < kPipeCols; ++u) acc = fma(c.v[u], xv[u], acc);
+                } else {
+#pragma unroll
+                    for (int u = 0; u < kPipeCols; ++u)
+                        if (u < rem) acc = fma(c.v[u], xv[u], acc);
+                }
+                if (last) {
+                    const int r = ls * 32 + lane;
+                    sz[r] = row0 + r < a.n ? acc : 0.0;
+                    if (row0 + r < a.n) dacc = fma(sp[r], acc, dacc);
+                    acc = 0.0;
+                }
+                ls = lsn;
+                j = jn;
+            };
+            while (ls < ns) {
+                step(colsA, colsB);
+                if (ls >= ns) break;
+                step(colsB, colsA);
+            }
+        }
+        for (; !PIPE && ls < ns; ls += nw) {
             const int4 md = meta[ls];
             const int r = ls * 32 + lane, row = row0 + r;
             double acc = 0.0;
@@ -398,6 +472,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
         }
         if (!go) break;
         __syncthreads();
+        if (PIPE && firstStreamed < ns) ahead(colsA, firstStreamed, 0);
         if (tid == 0) {
             fence_gpu();
             arrive(a.counters + 96);
@@ -632,21 +707,30 @@ struct LoopShape {
     size_t fixed;  // shared memory besides the matrix
 };
 
-LoopShape loop_shape(int n, int numSms) {
+LoopShape loop_shape(int n, int numSms, int threads) {
     LoopShape s;
     const int nslices = (n + 31) / 32;
     s.P = std::min(numSms, nslices);
     const int ns = (nslices + s.P - 1) / s.P;
     s.rows = 32 * ns;
-    s.threads = std::max(64, std::min(kLoopThreads, 32 * ns));
+    s.threads = std::max(64, std::min(threads, 32 * ns));
     s.fixed = sizeof(double) * (5 * (size_t)s.rows + 64) + sizeof(int4) * (size_t)ns +
               sizeof(int) * (size_t)((ns + 3) / 4 * 4);
     return s;
 }
 
-template <int LAY>
+// How a system is run: threads per CTA, and how rows beyond shared memory load.
+//   whole  all of the matrix in shared memory: 448 threads, most registers
+//   short  rows of up to 10 entries: 512 threads (7-point 80^3 26.7 us against
+//          30.1 with 448, 86^3 31.4, 92^3 36.1; the graph loop 31.3, 36.2, 38.2)
+//   long   384 threads, a step ahead (27-point 54^3 22.9 us against 25.6 with 448
+//          and no step ahead, 60^3 30.2 against 34.6; the graph loop 28.7, 32.7)
+enum : int { kModeWhole = 0, kModeShort = 1, kModeLong = 2 };
+int mode_threads(int mode) { return mode == kModeWhole ? 448 : (mode == kModeShort ? 512 : 384); }
+
+template <int LAY, int NT, bool PIPE>
 cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
-    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY, NT, PIPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kLoopSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -659,7 +743,14 @@ cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY>, a);
+    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY, NT, PIPE>, a);
+}
+
+template <int LAY>
+cudaError_t loop_launch_mode(int mode, cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
+    if (mode == kModeWhole) return loop_launch<LAY, 448, false>(st, s, a);
+    if (mode == kModeShort) return loop_launch<LAY, 512, false>(st, s, a);
+    return loop_launch<LAY, 384, true>(st, s, a);
 }
 }  // namespace
 
@@ -757,24 +848,30 @@ cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a) {
     return cluster_launch<2>(st, s, a);
 }
 
-// The vectors have to fit in shared memory (875,000 rows on 152 SMs), and at
-// most 6.5 entries per row may have to be read from L2 or HBM in every
-// iteration: the stream runs with 14 warps per SM, where the SpMV kernels of
-// the graph loop have 48.  7-point 80^3 (half of the matrix streamed): 26.7 us
-// against 31.3; 27-point 54^3 (9 entries per row by this count) 25.5 against
-// 27.7, 60^3 (15) 34.6 against 33.0 and 70^3 51 against 40.
-bool cg_loop_fits(int n, int64_t stored, int entryBytes, int numSms) {
-    if (n <= 0) return false;
-    const LoopShape s = loop_shape(n, numSms);
-    if (s.fixed > kLoopSmem) return false;
-    const int64_t resident = (int64_t)((kLoopSmem - s.fixed) / (size_t)entryBytes) * s.P;
-    return 2 * (stored - resident) <= 13 * (int64_t)n;
+// -1: no.  The vectors have to fit in shared memory (875,000 rows on 152 SMs).
+// What of the matrix does not fit beside them is read from L2 or HBM in every
+// iteration, by 12 to 16 warps per SM with little L1 left, where the SpMV kernels
+// of the graph loop have 48 warps and all of L1: short rows gain up to the
+// vectors' limit (see mode_threads), long ones while half of their entries stay
+// (27-point 60^3, 12 of 27 streamed: 30.2 us against 32.7; 70^3, 17 of 27
+// streamed: 45.7 against 39.8).
+// The mode itself does not depend on the layout (the sums' order follows from the
+// number of threads): it is the one for the smallest.
+int cg_loop_mode(int n, int64_t stored, double entryBytes, int numSms) {
+    if (n <= 0) return -1;
+    const LoopShape s = loop_shape(n, numSms, 512);
+    if (s.fixed > kLoopSmem) return -1;
+    const double room = (double)(kLoopSmem - s.fixed) * s.P, total = (double)stored;
+    const bool shortRows = stored <= 10 * (int64_t)n;
+    if (total - room / entryBytes > (shortRows ? 6.5 * n : 0.5 * total)) return -1;
+    if (total - room / kLoopPatEntry <= 0.02 * total) return kModeWhole;
+    return shortRows ? kModeShort : kModeLong;
 }
 
 size_t cg_loop_sync_bytes(int numSms) { return 128 * sizeof(uint32_t) + 3 * sizeof(ulonglong2) * 2 * (size_t)numSms; }
 
-cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a) {
-    const LoopShape s = loop_shape(a.n, numSms);
+cudaError_t cg_loop_launch(cudaStream_t st, int mode, int layout, int numSms, void* sync, LoopArgs a) {
+    const LoopShape s = loop_shape(a.n, numSms, mode_threads(mode));
     a.nslices = (a.n + 31) / 32;
     a.rows = s.rows;
     a.counters = static_cast<uint32_t*>(sync);
@@ -782,9 +879,9 @@ cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, 
     // A CTA whose part of the matrix fits in the rest copies it there.
     a.matBytes = (int)((kLoopSmem - s.fixed) / 16 * 16);
     a.smem = s.fixed + (size_t)a.matBytes;
-    if (layout == 0) return loop_launch<0>(st, s, a);
-    if (layout == 1) return loop_launch<1>(st, s, a);
-    return loop_launch<2>(st, s, a);
+    if (layout == 0) return loop_launch_mode<0>(mode, st, s, a);
+    if (layout == 1) return loop_launch_mode<1>(mode, st, s, a);
+    return loop_launch_mode<2>(mode, st, s, a);
 }
 
 }  // namespace xjpcg

@@ -27,6 +27,10 @@ SYSTEMS = {
     "wide_plane": ((3, 190, 191), True, "grid"),  # columns beyond int16 offsets
     "matrix_just_on_chip": ((47, 48, 49), False, "grid"),
     "matrix_partly_on_chip": ((79, 80, 81), True, "grid"),
+    "long_rows_streamed": ((54, 55, 57), False, "grid"),
+    "half_of_long_rows_streamed": ((60, 60, 61), False, "grid"),
+    "width_18_streamed": ((2, 310, 311), False, "grid"),  # 7 + 7 + 4 entries a row, no int16 offsets
+    "too_much_streamed": ((70, 70, 71), False, "graph"),
     "vectors_too_large": ((96, 97, 97), True, "graph"),
 }
 
@@ -70,7 +74,8 @@ def test_loop_kernel_matches_the_host_loop(gpu_lib, name):
     host = _solves(s, {"XJPCG_SPMV_LANES": "-1", "XJPCG_HOST_LOOP": "1"}, calls)
     default = _solves(s, {}, calls)
     runs = [default]
-    for lanes in ("-1", "-5") if name == "wide_plane" else ("-1", "-3", "-5"):
+    layouts = {"wide_plane": ("-1", "-5"), "width_18_streamed": ("-1", "-5"), "half_of_long_rows_streamed": ()}
+    for lanes in layouts.get(name, ("-1", "-3", "-5")):
         runs.append(_solves(s, {"XJPCG_SPMV_LANES": lanes, "XJPCG_LOOP_KERNEL": "1"}, calls))
     for run in runs:
         (ra, reca, ia), (rb, _, _), (rc, _, _) = run
