@@ -7,23 +7,37 @@
 // barrier over 152 SMs 1,600 and a cluster barrier 370 (all measured).  As two
 // kernels per iteration in a graph, with a grid barrier inside the second, an
 // iteration took 14 to 15 us however small the system.  Here one launch runs
-// all iterations: r, x, z = J r, p and J never leave shared memory, nor does
-// the part of the matrix that fits beside them; only p is also written to
-// global memory, for the other CTAs' gathers.
+// all iterations, and r, x, z = J r, p and (if it fits) J never leave shared
+// memory; p is also written to global memory, for the other CTAs' gathers.
 //
 // Two forms:
 //   cg_cluster_kernel  one cluster of up to 16 CTAs; p is gathered, and the
-//                      sums are exchanged, through distributed shared memory.
-//                      Three cluster barriers per iteration.
+//                      sums are exchanged, through distributed shared memory;
+//                      so is the matrix kept on the chip if it fits.  Three
+//                      cluster barriers per iteration.
 //   cg_loop_kernel     one CTA per SM, cooperative; sums go through posts and
-//                      counters in global memory.
+//                      counters in global memory, the matrix streams from L2.
+//
+// A larger system is bound by FP64 issue (14 operations per row and iteration
+// with 7 entries in a row, 34 with 27; 2 per clock and SM) as long as loads and
+// the 64-cycle FMAs of a row overlap.  With 12 warps per SM they do so only when
+// each warp works on three steps at once: columns of one on their way, values
+// and p of the next, sums of the one before, instruction by instruction.  7-point
+// 96^3 33.2 us per iteration: 27,700 cycles for the product (23,300 of issue at
+// the least), 14,700 for r and z, 6,900 for x and p, the rest waiting for sums.
+// Loading values and columns a step ahead but gathering when needed took 48.7
+// us, the three stages one after another 39.2.  Keeping the matrix in what is
+// left of shared memory gained nothing over streaming it (7-point 32^3 9.5 us
+// either way, 64^3 16.9 and 16.8; 27-point 48^3 17.9 and 17.4).
 //
 // Measured, us per iteration (two kernels per iteration / loop / cluster):
-//   7-point   16^3   14.7 /  8.8 / 6.9      27-point   8^3  15.1 / 13.1 / 6.5
-//             32^3   14.7 /  9.5 /  -                 16^3  16.9 / 10.9 / 8.4
-//             48^3   18.1 / 12.3 /  -                 32^3  18.0 / 11.7 /  -
-//             64^3   25.5 / 17.5 /  -                 48^3  24.2 / 17.9 /  -
-//             80^3   31.3 / 26.7 /  -                 60^3  32.7 / 30.2 /  -
+//   7-point   16^3   14.7 /  8.8 / 6.7      27-point   8^3  15.1 / 13.1 / 6.5
+//             32^3   14.9 /  9.6 /  -                 16^3  16.9 / 10.9 / 8.4
+//             48^3   18.1 / 12.4 /  -                 32^3  18.6 / 11.6 /  -
+//             64^3   25.1 / 16.7 /  -                 48^3  24.6 / 17.4 /  -
+//             80^3   33.1 / 23.2 /  -                 60^3  32.7 / 24.8 /  -
+//             96^3   42.2 / 33.2 /  -                 80^3  50.3 / 43.5 /  -
+//            102^3   44.9 / 37.7 /  -                 96^3  73.5 / 69.0 /  -
 //
 // Every row is summed in its stored order, as in the sliced SpMV kernels; the
 // dot products are summed per thread, per warp, per CTA and over the CTAs, in
@@ -37,9 +51,10 @@
 namespace xjpcg {
 
 namespace {
+constexpr int kLoopThreads = 384;   // 168 registers; with 512 (128 registers) the pipelined steps spill
 constexpr int kVecThreads = 256;    // threads that update r and z: enough to fill the FP64 pipe, and every warp costs two sums
-constexpr int kCols = 8;            // stored columns per step of a row: their loads go out together
-constexpr int kPipeCols = 7;        // the same where the next step is loaded ahead (27 = 7 + 7 + 7 + 6)
+constexpr int kStep = 7;            // stored columns per step of a row (27 = 7 + 7 + 7 + 6)
+constexpr int kCols = 8;            // the same in the cluster form
 constexpr int kPosts = 5;           // posts a lane reads at once: 152 CTAs in one step
 constexpr uint64_t kLoopBudgetNs = 2000000000ull;  // 2 s
 constexpr size_t kLoopSmem = 226 * 1024;
@@ -127,9 +142,16 @@ __device__ __forceinline__ double grid_total(double s, ulonglong2* posts, uint32
 }
 }  // namespace
 
-struct Cols {
-    double v[kPipeCols];
-    int c[kPipeCols];
+// One step of a row, up to kStep stored columns.
+struct Step {
+    double v[kStep], x[kStep];
+    int ls, rem;  // slice; its columns from this step's first on
+};
+// A step's place in the matrix.
+struct StepAt {
+    int ls, rem;
+    int v, c;    // of its values; of its columns
+    int shared;  // columns: offsets shared by the slice
 };
 
 // CTA q owns a contiguous run of slices (so neighbouring rows' gathers meet in
@@ -140,12 +162,11 @@ struct Cols {
 //   p = z + beta p, also to global -> barrier (release / acquire)
 // Only the last needs fences: the posts of the sums carry their own tags.
 // LAY: 0 int32 columns, 1 int16 offsets, 2 slice-shared offsets.
-// NT: threads at most.  PIPE: rows beyond shared memory load a step ahead.
-template <int LAY, int NT, bool PIPE>
-__global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
+template <int LAY>
+__global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
     __shared__ double sAlpha, sBeta, sRz, sRr;
-    __shared__ int sGo[3], sOn;
+    __shared__ int sGo[3];
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
     const int q = blockIdx.x, P = gridDim.x;
     const int s0 = (int)((int64_t)a.nslices * q / P), s1 = (int)((int64_t)a.nslices * (q + 1) / P);
@@ -155,10 +176,8 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
     double* const sz = sx + a.rows;
     double* const sp = sz + a.rows;
     double* const sj = sp + a.rows;
-    double* const part = sj + a.rows;  // 2 per warp
+    double* const part = sj + (a.jOnChip ? a.rows : 0);  // 2 per warp
     int4* const meta = reinterpret_cast<int4*>(part + 64);
-    int* const place = reinterpret_cast<int*>(meta + a.rows / 32);
-    unsigned char* const mat = reinterpret_cast<unsigned char*>(place + (a.rows / 32 + 3) / 4 * 4);
 
     for (int i = tid; i < pairs; i += nt) {
         const int e = row0 / 2 + i;
@@ -166,7 +185,7 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
         const double2 zero = make_double2(0.0, 0.0);
         reinterpret_cast<double2*>(sr)[i] = in ? reinterpret_cast<const double2*>(a.r)[e] : zero;
         reinterpret_cast<double2*>(sp)[i] = in ? reinterpret_cast<const double2*>(a.p)[e] : zero;
-        reinterpret_cast<double2*>(sj)[i] = in ? reinterpret_cast<const double2*>(a.J)[e] : zero;
+        if (a.jOnChip) reinterpret_cast<double2*>(sj)[i] = in ? reinterpret_cast<const double2*>(a.J)[e] : zero;
         reinterpret_cast<double2*>(sx)[i] = zero;
     }
     // slice records: {first value, columns, pattern or first column, shared offsets?}
@@ -181,75 +200,61 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
     }
     if (tid == 0) sRz = a.state->rz;
     __syncthreads();
-    // The first nOn slices, as many as fit, stay in shared memory (place: their
-    // bytes there, values then columns).
-    if (tid == 0) {
-        int at = 0, i = 0;
-        for (; i < ns; ++i) {
-            const int4 md = meta[i];
-            const int bytes = 256 * md.y + (md.w ? (4 * md.y + 15) / 16 * 16 : (LAY == 1 ? 64 : 128) * md.y);
-            if (at + bytes > a.matBytes) break;
-            place[i] = at;
-            at += bytes;
-        }
-        sOn = i;
-    }
-    __syncthreads();
-    const int nOn = sOn;
-    for (int ls = wid; ls < nOn; ls += nw) {
-        const int4 md = meta[ls];
-        double* const v = reinterpret_cast<double*>(mat + place[ls]);
-        int* const c = reinterpret_cast<int*>(v + 32 * md.y);
-        for (int j = 0; j < md.y; ++j) {
-            v[j * 32 + lane] = a.sval[md.x + j * 32 + lane];
-            if (LAY == 0)
-                c[j * 32 + lane] = a.col32[md.z + j * 32 + lane];
-            else if (LAY == 1)
-                reinterpret_cast<int16_t*>(c)[j * 32 + lane] = a.col16[md.z + j * 32 + lane];
-            else if (!md.w)
-                c[j * 32 + lane] = a.gcol[md.z + j * 32 + lane];
-        }
-        if (LAY == 2 && md.w)
-            for (int j = lane; j < md.y; j += 32) c[j] = a.pat[md.z + j];
-    }
-    auto column = [&](const int4& md, int row, int j) {
-        if (LAY == 0) return __ldcs(a.col32 + md.z + j * 32 + lane);
-        if (LAY == 1) return min(row, a.n - 1) + __ldcs(a.col16 + md.z + j * 32 + lane);
-        return md.w ? row + __ldg(a.pat + md.z + j) : __ldcs(a.gcol + md.z + j * 32 + lane);
-    };
     __syncthreads();
     const double tols = a.state->tols;
     const uint32_t maxIterP1 = a.state->maxIterP1;
     double2* const p2 = reinterpret_cast<double2*>(a.p) + row0 / 2;
     const int have2 = max(0, min(pairs, a.n2 - row0 / 2));  // pairs of this CTA that exist
 
+    // shared or global, read through one pointer
+    const double2* const j2 = a.jOnChip ? reinterpret_cast<const double2*>(sj) : reinterpret_cast<const double2*>(a.J) + row0 / 2;
+    const int vecStride = min(nt, kVecThreads);
+
     int nwUp = 1;
     while (nwUp < nw) nwUp *= 2;
 
-    // PIPE: the first streamed step of an iteration is loaded before the barrier
-    // that ends the one before, as it does not depend on p
-    const int firstStreamed = nOn + (wid - nOn % nw + nw) % nw;
-    auto ahead = [&](Cols& c, int ls, int j) {
-        const int4 md = meta[ls];
-        const int rem = md.y - j, row = row0 + ls * 32 + lane;
-        const double* vp = a.sval + md.x + j * 32 + lane;
-        if (rem >= kPipeCols) {
-#pragma unroll
-            for (int u = 0; u < kPipeCols; ++u) {
-                c.v[u] = ld_val(vp + u * 32);
-                c.c[u] = column(md, row, j + u);
-            }
-        } else {
-#pragma unroll
-            for (int u = 0; u < kPipeCols; ++u)
-                if (u < rem) {
-                    c.v[u] = ld_val(vp + u * 32);
-                    c.c[u] = column(md, row, j + u);
-                }
-        }
+    // A step passes through three stages: its columns are loaded, then its values
+    // and p, then the products are summed.  A warp has one step in each.
+    int cols[kStep];
+    Step A, B;
+    auto slice = [&](int ls) {
+        const int4 md = meta[min(ls, ns - 1)];
+        StepAt t;
+        t.ls = ls;
+        t.rem = ls < ns ? md.y : 0;
+        t.v = md.x + lane;
+        t.shared = LAY == 2 ? md.w : 0;
+        t.c = t.shared ? md.z : md.z + lane;
+        return t;
     };
-    Cols colsA, colsB;
-    if (PIPE && firstStreamed < ns) ahead(colsA, firstStreamed, 0);
+    auto next = [&](const StepAt& t) {
+        if (t.rem <= kStep) return slice(t.ls + nw);
+        StepAt l = t;
+        l.rem -= kStep;
+        l.v += kStep * 32;
+        l.c += t.shared ? kStep : kStep * 32;
+        return l;
+    };
+    auto load_col = [&](const StepAt& t, int u) {
+        if (LAY == 0) return __ldcs(a.col32 + t.c + u * 32);
+        if (LAY == 1) return (int)__ldcs(a.col16 + t.c + u * 32);
+        return __ldg((t.shared ? a.pat : a.gcol) + t.c + (t.shared ? u : u * 32));
+    };
+    auto base_of = [&](const StepAt& t) {
+        const int row = row0 + t.ls * 32 + lane;
+        return a.p + (LAY == 0 ? 0 : (LAY == 1 ? min(row, a.n - 1) : (t.shared ? row : 0)));
+    };
+    auto start = [&]() {
+        if (wid >= ns) return;
+        const StepAt t = slice(wid);
+#pragma unroll
+        for (int u = 0; u < kStep; ++u)
+            if (u < t.rem) {
+                cols[u] = load_col(t, u);
+                A.v[u] = ld_val(a.sval + t.v + u * 32);
+            }
+    };
+    start();
 
     uint32_t k = 0;
     bool ok = true;
@@ -257,116 +262,68 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
         const uint32_t target = (k + 1u) * (uint32_t)P, tag = a.tag0 + k;
         // ---- Ap = A p (kept in sz) and this thread's part of p.Ap ----
         double dacc = 0.0;
-        int ls = wid;
-        for (; ls < nOn; ls += nw) {
-            const int4 md = meta[ls];
-            const int r = ls * 32 + lane, row = row0 + r, at = place[ls];
+        if (wid < ns) {
             double acc = 0.0;
+            StepAt pos = slice(wid);
+            A.ls = wid;
+            A.rem = pos.rem;
             {
-                const double* const v = reinterpret_cast<const double*>(mat + at) + lane;
-                const int* const c = reinterpret_cast<const int*>(mat + at + 256 * md.y);
-                const int base = LAY == 1 ? min(row, a.n - 1) : row;
-                for (int j = 0; j < md.y; j += kCols) {
-                    double xv[kCols];
+                const double* const pb = base_of(pos);
+                const StepAt l = next(pos);
 #pragma unroll
-                    for (int u = 0; u < kCols; ++u)
-                        if (j + u < md.y) {
-                            int col;
-                            if (LAY == 1)
-                                col = base + reinterpret_cast<const int16_t*>(c)[(j + u) * 32 + lane];
-                            else
-                                col = LAY == 2 && md.w ? base + c[j + u] : c[(j + u) * 32 + lane];
-                            xv[u] = a.p[col];
-                        }
-#pragma unroll
-                    for (int u = 0; u < kCols; ++u)
-                        if (j + u < md.y) acc = fma(v[(j + u) * 32], xv[u], acc);
+                for (int u = 0; u < kStep; ++u) {
+                    if (u < pos.rem) A.x[u] = pb[cols[u]];
+                    if (u < l.rem) cols[u] = load_col(l, u);
                 }
+                pos = l;
             }
-            sz[r] = row < a.n ? acc : 0.0;
-            if (row < a.n) dacc = fma(sp[r], acc, dacc);
-        }
-        if (PIPE) {
-            // the others stream: the next step's values and columns are on their
-            // way while this one's p is gathered and summed
-            double acc = 0.0;
-            int j = 0;
-            auto step = [&](const Cols& c, Cols& next) {
-                const int rem = meta[ls].y - j;
-                double xv[kPipeCols];
-                if (rem >= kPipeCols) {
-#pragma unroll
-                    for (int u = 0; u < kPipeCols; ++u) xv[u] = a.p[c.c[u]];
-                } else {
-#pragma unroll
-                    for (int u = 0; u < kPipeCols; ++u)
-                        if (u < rem) xv[u] = a.p[c.c[u]];
-                }
-                const bool last = rem <= kPipeCols;
-                const int lsn = last ? ls + nw : ls, jn = last ? 0 : j + kPipeCols;
-                if (lsn < ns) ahead(next, lsn, jn);
-                if (rem >= kPipeCols) {
-#pragma unroll
-                    for (int u = 0; u < kPipeCols; ++u) acc = fma(c.v[u], xv[u], acc);
-                } else {
-#pragma unroll
-                    for (int u = 0; u < kPipeCols; ++u)
-                        if (u < rem) acc = fma(c.v[u], xv[u], acc);
-                }
-                if (last) {
-                    const int r = ls * 32 + lane;
-                    sz[r] = row0 + r < a.n ? acc : 0.0;
-                    if (row0 + r < a.n) dacc = fma(sp[r], acc, dacc);
-                    acc = 0.0;
-                }
-                ls = lsn;
-                j = jn;
+            auto finish = [&](const Step& f) {
+                if (f.rem > kStep) return;  // more of the slice to come
+                const int r = f.ls * 32 + lane;
+                const bool in = row0 + r < a.n;
+                sz[r] = in ? acc : 0.0;
+                if (in) dacc = fma(sp[r], acc, dacc);
+                acc = 0.0;
             };
-            while (ls < ns) {
-                step(colsA, colsB);
-                if (ls >= ns) break;
-                step(colsB, colsA);
-            }
-        }
-        for (; !PIPE && ls < ns; ls += nw) {
-            const int4 md = meta[ls];
-            const int r = ls * 32 + lane, row = row0 + r;
-            double acc = 0.0;
-            {
-                const double* vp = a.sval + md.x + lane;
-                int j = 0;
-                for (; j + kCols <= md.y; j += kCols) {
-                    double v[kCols];
-                    int c[kCols];
+            auto step = [&](const Step& f, Step& g) {  // pos: g's place
+                if (pos.ls >= ns) {  // f is the warp's last
 #pragma unroll
-                    for (int u = 0; u < kCols; ++u) {
-                        v[u] = ld_val(vp + u * 32);
-                        c[u] = column(md, row, j + u);
+                    for (int u = 0; u < kStep; ++u)
+                        if (u < f.rem) acc = fma(f.v[u], f.x[u], acc);
+                    finish(f);
+                    return false;
+                }
+                const StepAt l = next(pos);
+                const double* const pb = base_of(pos);
+                const double* const vp = a.sval + pos.v;
+                g.ls = pos.ls;
+                g.rem = pos.rem;
+                // the stages' instructions alternate, as a dependent FMA takes 64 cycles
+                if (min(min(f.rem, pos.rem), l.rem) >= kStep) {
+#pragma unroll
+                    for (int u = 0; u < kStep; ++u) {
+                        g.x[u] = pb[cols[u]];
+                        g.v[u] = ld_val(vp + u * 32);
+                        cols[u] = load_col(l, u);
+                        acc = fma(f.v[u], f.x[u], acc);
                     }
+                } else {
 #pragma unroll
-                    for (int u = 0; u < kCols; ++u) acc = fma(v[u], a.p[c[u]], acc);
-                    vp += kCols * 32;
-                }
-                const int rem = md.y - j;
-                if (rem > 0) {
-                    double v[kCols - 1], xv[kCols - 1];
-                    int c[kCols - 1];
-#pragma unroll
-                    for (int u = 0; u < kCols - 1; ++u)
-                        if (u < rem) {
-                            v[u] = ld_val(vp + u * 32);
-                            c[u] = column(md, row, j + u);
+                    for (int u = 0; u < kStep; ++u) {
+                        if (u < pos.rem) {
+                            g.x[u] = pb[cols[u]];
+                            g.v[u] = ld_val(vp + u * 32);
                         }
-#pragma unroll
-                    for (int u = 0; u < kCols - 1; ++u)
-                        if (u < rem) xv[u] = a.p[c[u]];
-#pragma unroll
-                    for (int u = 0; u < kCols - 1; ++u)
-                        if (u < rem) acc = fma(v[u], xv[u], acc);
+                        if (u < l.rem) cols[u] = load_col(l, u);
+                        if (u < f.rem) acc = fma(f.v[u], f.x[u], acc);
+                    }
                 }
+                finish(f);
+                pos = l;
+                return true;
+            };
+            while (step(A, B) && step(B, A)) {
             }
-            sz[r] = row < a.n ? acc : 0.0;
-            if (row < a.n) dacc = fma(sp[r], acc, dacc);
         }
         dacc = warp_sum(dacc);
         if (lane == 0) part[wid] = dacc;
@@ -388,9 +345,12 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
         const double alpha = sAlpha;
         // ---- r -= alpha Ap, z = J r ----
         double rr = 0.0, rz = 0.0;
-        for (int i = tid; i < have2 && tid < kVecThreads; i += min(nt, kVecThreads)) {
+        double2 jn = make_double2(0.0, 0.0);
+        if (tid < min(have2, kVecThreads)) jn = j2[tid];
+        for (int i = tid; i < have2 && tid < kVecThreads; i += vecStride) {
             double2 rv = reinterpret_cast<double2*>(sr)[i];
-            const double2 av = reinterpret_cast<double2*>(sz)[i], jv = reinterpret_cast<double2*>(sj)[i];
+            const double2 av = reinterpret_cast<double2*>(sz)[i], jv = jn;
+            if (i + vecStride < have2) jn = j2[i + vecStride];
             rv.x = fma(-alpha, av.x, rv.x);
             rv.y = fma(-alpha, av.y, rv.y);
             const double2 zv = make_double2(rv.x * jv.x, rv.y * jv.y);
@@ -472,7 +432,7 @@ __global__ void __launch_bounds__(NT, 1) cg_loop_kernel(LoopArgs a) {
         }
         if (!go) break;
         __syncthreads();
-        if (PIPE && firstStreamed < ns) ahead(colsA, firstStreamed, 0);
+        start();
         if (tid == 0) {
             fence_gpu();
             arrive(a.counters + 96);
@@ -704,57 +664,41 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
 namespace {
 struct LoopShape {
     int P, rows, threads;
+    bool jOnChip;  // grid form: J in shared memory as well
     size_t fixed;  // shared memory besides the matrix
 };
 
-LoopShape loop_shape(int n, int numSms, int threads) {
+LoopShape loop_shape(int n, int numSms) {
     LoopShape s;
     const int nslices = (n + 31) / 32;
     s.P = std::min(numSms, nslices);
     const int ns = (nslices + s.P - 1) / s.P;
     s.rows = 32 * ns;
-    s.threads = std::max(64, std::min(threads, 32 * ns));
-    s.fixed = sizeof(double) * (5 * (size_t)s.rows + 64) + sizeof(int4) * (size_t)ns +
-              sizeof(int) * (size_t)((ns + 3) / 4 * 4);
+    s.threads = std::max(64, std::min(kLoopThreads, 32 * ns));
+    const size_t other = sizeof(double) * 64 + sizeof(int4) * (size_t)ns;
+    s.jOnChip = sizeof(double) * 5 * (size_t)s.rows + other <= kLoopSmem;
+    s.fixed = sizeof(double) * (s.jOnChip ? 5 : 4) * (size_t)s.rows + other;
     return s;
 }
 
-// How a system is run: threads per CTA, and how rows beyond shared memory load.
-//   whole  all of the matrix in shared memory: 448 threads, most registers
-//   short  rows of up to 10 entries: 512 threads (7-point 80^3 26.7 us against
-//          30.1 with 448, 86^3 31.4, 92^3 36.1; the graph loop 31.3, 36.2, 38.2)
-//   long   384 threads, a step ahead (27-point 54^3 22.9 us against 25.6 with 448
-//          and no step ahead, 60^3 30.2 against 34.6; the graph loop 28.7, 32.7)
-enum : int { kModeWhole = 0, kModeShort = 1, kModeLong = 2 };
-int mode_threads(int mode) { return mode == kModeWhole ? 448 : (mode == kModeShort ? 512 : 384); }
-
-template <int LAY, int NT, bool PIPE>
+template <int LAY>
 cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
-    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY, NT, PIPE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kLoopSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)s.P);
     cfg.blockDim = dim3((unsigned)s.threads);
-    cfg.dynamicSmemBytes = a.smem;
+    cfg.dynamicSmemBytes = s.fixed;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY, NT, PIPE>, a);
+    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY>, a);
 }
 
-template <int LAY>
-cudaError_t loop_launch_mode(int mode, cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
-    if (mode == kModeWhole) return loop_launch<LAY, 448, false>(st, s, a);
-    if (mode == kModeShort) return loop_launch<LAY, 512, false>(st, s, a);
-    return loop_launch<LAY, 384, true>(st, s, a);
-}
-}  // namespace
-
-namespace {
 // The cluster form: its CTAs' rows and shared memory.
 LoopShape cluster_shape(int n) {
     LoopShape s;
@@ -848,40 +792,21 @@ cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a) {
     return cluster_launch<2>(st, s, a);
 }
 
-// -1: no.  The vectors have to fit in shared memory (875,000 rows on 152 SMs).
-// What of the matrix does not fit beside them is read from L2 or HBM in every
-// iteration, by 12 to 16 warps per SM with little L1 left, where the SpMV kernels
-// of the graph loop have 48 warps and all of L1: short rows gain up to the
-// vectors' limit (see mode_threads), long ones while half of their entries stay
-// (27-point 60^3, 12 of 27 streamed: 30.2 us against 32.7; 70^3, 17 of 27
-// streamed: 45.7 against 39.8).
-// The mode itself does not depend on the layout (the sums' order follows from the
-// number of threads): it is the one for the smallest.
-int cg_loop_mode(int n, int64_t stored, double entryBytes, int numSms) {
-    if (n <= 0) return -1;
-    const LoopShape s = loop_shape(n, numSms, 512);
-    if (s.fixed > kLoopSmem) return -1;
-    const double room = (double)(kLoopSmem - s.fixed) * s.P, total = (double)stored;
-    const bool shortRows = stored <= 10 * (int64_t)n;
-    if (total - room / entryBytes > (shortRows ? 6.5 * n : 0.5 * total)) return -1;
-    if (total - room / kLoopPatEntry <= 0.02 * total) return kModeWhole;
-    return shortRows ? kModeShort : kModeLong;
-}
+// The vectors have to fit in shared memory, all but J (1,079,808 rows on 152 SMs; J too up to 865,792).
+bool cg_loop_fits(int n, int numSms) { return n > 0 && loop_shape(n, numSms).fixed <= kLoopSmem; }
 
 size_t cg_loop_sync_bytes(int numSms) { return 128 * sizeof(uint32_t) + 3 * sizeof(ulonglong2) * 2 * (size_t)numSms; }
 
-cudaError_t cg_loop_launch(cudaStream_t st, int mode, int layout, int numSms, void* sync, LoopArgs a) {
-    const LoopShape s = loop_shape(a.n, numSms, mode_threads(mode));
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a) {
+    const LoopShape s = loop_shape(a.n, numSms);
     a.nslices = (a.n + 31) / 32;
     a.rows = s.rows;
+    a.jOnChip = s.jOnChip ? 1 : 0;
     a.counters = static_cast<uint32_t*>(sync);
     a.posts = reinterpret_cast<ulonglong2*>(a.counters + 128);
-    // A CTA whose part of the matrix fits in the rest copies it there.
-    a.matBytes = (int)((kLoopSmem - s.fixed) / 16 * 16);
-    a.smem = s.fixed + (size_t)a.matBytes;
-    if (layout == 0) return loop_launch_mode<0>(mode, st, s, a);
-    if (layout == 1) return loop_launch_mode<1>(mode, st, s, a);
-    return loop_launch_mode<2>(mode, st, s, a);
+    if (layout == 0) return loop_launch<0>(st, s, a);
+    if (layout == 1) return loop_launch<1>(st, s, a);
+    return loop_launch<2>(st, s, a);
 }
 
 }  // namespace xjpcg

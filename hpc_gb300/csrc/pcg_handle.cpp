@@ -550,6 +550,7 @@ bool PcgHandle::ensurePat() {
                                m_psGcol.as<int>(), true),
           "shared-offset fill");
     m_psTotal = tot[0];
+    m_psGeneral = tot[1];
     m_psState = 1;
     m_ps32Valid = false;
     return true;
@@ -1012,31 +1013,29 @@ int PcgHandle::cgSpmvMode() const {
                                                                                          : kSpmvCgDot;
 }
 
-// Whether the fp64 loop runs as one kernel (cg_loop.cu), and which: -1 no, 0 .. 2
-// over the grid (cg_loop_mode), 3 in one cluster.  It reads a sliced copy, whichever is built;
+// Whether the fp64 loop runs as one kernel (cg_loop.cu), and which: 0 no, 1
+// over the grid, 2 in one cluster.  It reads a sliced copy, whichever is built;
 // the choice depends on the matrix alone, so that repeated solves agree bit
 // for bit.  A forced SpMV layout keeps the loop of that layout's kernel (unless
 // XJPCG_LOOP_KERNEL=1), as the host-driven loop and the separate vector kernels
 // keep theirs.
 int PcgHandle::loopKernel(uint32_t maxIter, int* layout) {
     const bool forced = m_forcedCfg >= 0 || m_forcedLanes != 0;
-    if (!m_useGraph || !m_fusedUpdate || m_loopKernelEnv == 0 || maxIter > 0xfffffff0u) return -1;
-    if (forced && (m_loopKernelEnv != 1 || !(isSell(m_spmvCfg) || isPat(m_spmvCfg)))) return -1;
-    if (cg_loop_mode((int)m_n, 0, 1.0, m_numSms) < 0 || !ensureSell()) return -1;  // too large, or rows too uneven
+    if (!m_useGraph || !m_fusedUpdate || m_loopKernelEnv == 0 || maxIter > 0xfffffff0u) return 0;
+    if (forced && (m_loopKernelEnv != 1 || !(isSell(m_spmvCfg) || isPat(m_spmvCfg)))) return 0;
+    if (!cg_loop_fits((int)m_n, m_numSms) || !ensureSell()) return 0;  // too large, or rows too uneven
+    // Gathers that are not coalesced want the graph loop's 48 warps per SM and L1
+    // once the vectors take most of the shared memory.  Random columns, us per
+    // iteration (this kernel / graph loop): 200,000 rows of 14 25.7 / 34.4, 500,000
+    // of 14 50.3 / 54.8 and of 30 85.2 / 84.1, 900,000 of 14 117 / 83.  Slices
+    // whose rows share their offsets (stencils) gain at every size.
+    constexpr uint32_t kLoopAnyColumns = 450000;
+    if (m_n > kLoopAnyColumns && !forced && (!ensurePat() || 10 * m_psGeneral > m_psTotal)) return 0;
     if (forced)
         *layout = isPat(m_spmvCfg) ? 2 : (isSellNarrow(m_spmvCfg) ? 1 : 0);
     else
         *layout = m_psState == 1 ? 2 : (m_sellNarrow ? 1 : 0);
-    if (cg_cluster_fits((int)m_n, m_sellTotal)) return 3;
-    int mode = cg_loop_mode((int)m_n, m_sellTotal, m_sellNarrow ? 10.0 : 12.0, m_numSms);
-    const bool longRows = m_sellTotal > 10 * (int64_t)m_n;
-    if (mode != 0 && !forced && (mode < 0 || longRows) &&
-        cg_loop_mode((int)m_n, m_sellTotal, kLoopPatEntry, m_numSms) >= 0 && ensurePat()) {
-        // shared offsets leave room for more of the matrix
-        *layout = 2;
-        mode = cg_loop_mode((int)m_n, m_psTotal, kLoopPatEntry, m_numSms);
-    }
-    return mode;
+    return cg_cluster_fits((int)m_n, m_sellTotal) ? 2 : 1;
 }
 
 // One launch for the vector init, one for the loop.
@@ -1066,13 +1065,13 @@ void PcgHandle::launchLoopKernel(int form, int layout, uint32_t maxIter) {
     a.r = m_r.as<double>();
     a.J = m_J.as<double>();
     a.state = st;
-    if (form == 3) {
+    if (form == 2) {
         check(cg_cluster_launch(m_stream, layout, a), "cluster loop kernel");
         return;
     }
     a.tag0 = m_loopTag;
     m_loopTag += maxIter + 1u;
-    check(cg_loop_launch(m_stream, form, layout, m_numSms, m_loopSync.p, a), "loop kernel");
+    check(cg_loop_launch(m_stream, layout, m_numSms, m_loopSync.p, a), "loop kernel");
 }
 
 // The mixed loop's FP32 update after its SpMV: the fused cooperative kernel
@@ -1135,13 +1134,13 @@ Results PcgHandle::run(uint32_t maxIter, double tol) {
     double* part = m_partials.as<double>();
     int loopLayout = 0;
     const int loopForm = loopKernel(maxIter, &loopLayout);
-    m_lastOneKernel = loopForm >= 0;
-    if (m_useGraph && loopForm < 0) {
+    m_lastOneKernel = loopForm != 0;
+    if (m_useGraph && loopForm == 0) {
         buildGraph();
         cmd.useCond = 1;
         cmd.condHandle = (uint64_t)m_cond;
     }
-    if (loopForm >= 0 && loopForm < 3) {
+    if (loopForm == 1) {
         alloc(m_loopSync, cg_loop_sync_bytes(m_numSms), "loop kernel posts");
         // Tags tell this solve's posts from earlier ones'; a launch uses at
         // most maxIter + 1 of them.  The counters start from 0 each time.
@@ -1152,7 +1151,7 @@ Results PcgHandle::run(uint32_t maxIter, double tol) {
     faultPoint("graph launch");
     check(cudaMemcpyAsync(st, &cmd, sizeof(CgState), cudaMemcpyHostToDevice, m_stream), "state upload");
     check(cudaEventRecord(m_ev0, m_stream), "event");
-    if (loopForm >= 0) {
+    if (loopForm != 0) {
         launchLoopKernel(loopForm, loopLayout, maxIter);
     } else if (m_useGraph) {
         check(cudaGraphLaunch(m_exec, m_stream), "graph launch");

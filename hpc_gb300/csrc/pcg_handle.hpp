@@ -256,7 +256,7 @@ class PcgHandle {
     DevBuf m_psSliceOff, m_psPatLen, m_psPatNew, m_psPatIdx, m_psPatOff, m_psGenOff, m_psPat, m_psGcol, m_psVal,
         m_psVal32;
     int m_psState = 0;  // 0 not built, 1 built, 2 not offered
-    int64_t m_psTotal = 0;
+    int64_t m_psTotal = 0, m_psGeneral = 0;  // stored entries; those in slices without shared offsets
     bool m_ps32Valid = false;
     // length-sorted sliced copy (irregular rows)
     DevBuf m_ssSorted, m_ssHist, m_ssStart, m_ssSliceOff, m_ssCol, m_ssVal, m_ssVal32;

@@ -183,18 +183,16 @@ struct LoopArgs {
     size_t smem = 0;
     uint32_t* counters = nullptr;
     ulonglong2* posts = nullptr;
+    int jOnChip = 0;
 };
-// How the grid form would run a system (-1: not at all); stored: entries of the
-// sliced copy, entryBytes: of one of them, its column included.
-constexpr double kLoopPatEntry = 8.25;  // a value, and a little more than 1/32 of an offset
-int cg_loop_mode(int n, int64_t stored, double entryBytes, int numSms);
+bool cg_loop_fits(int n, int numSms);  // the grid form
 // the same in one cluster of up to 16 CTAs, for small systems
 bool cg_cluster_fits(int n, int64_t stored);
 cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a);
 size_t cg_loop_sync_bytes(int numSms);
-// mode: of cg_loop_mode; layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
+// layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
 // offsets; sync: cg_loop_sync_bytes bytes, the first 512 cleared before each launch.
-cudaError_t cg_loop_launch(cudaStream_t st, int mode, int layout, int numSms, void* sync, LoopArgs a);
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a);
 
 // ---- mixed precision, reliable updates (mixed_kernels.cu) ----
 cudaError_t rel_init_launch(int grid, cudaStream_t s, int n, int n4, const double* b, const double* diag, double* x,
