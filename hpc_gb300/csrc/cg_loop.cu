@@ -33,11 +33,11 @@
 // Measured, us per iteration (two kernels per iteration / loop / cluster):
 //   7-point   16^3   14.7 /  8.8 / 6.7      27-point   8^3  15.1 / 13.1 / 6.5
 //             32^3   14.9 /  9.6 /  -                 16^3  16.9 / 10.9 / 8.4
-//             48^3   18.1 / 12.4 /  -                 32^3  18.6 / 11.6 /  -
+//             48^3   18.1 / 12.4 /  -                 32^3  18.6 / 11.5 /  -
 //             64^3   25.1 / 16.7 /  -                 48^3  24.6 / 17.4 /  -
-//             80^3   33.1 / 23.2 /  -                 60^3  32.7 / 24.8 /  -
-//             96^3   42.2 / 33.2 /  -                 80^3  50.3 / 43.5 /  -
-//            102^3   44.9 / 37.7 /  -                 96^3  73.5 / 69.0 /  -
+//             80^3   33.1 / 23.2 /  -                 60^3  32.7 / 23.9 /  -
+//             96^3   42.2 / 33.2 /  -                 80^3  50.3 / 40.5 /  -
+//            102^3   44.9 / 37.7 /  -                 96^3  73.5 / 63.4 /  -
 //
 // Every row is summed in its stored order, as in the sliced SpMV kernels; the
 // dot products are summed per thread, per warp, per CTA and over the CTAs, in
@@ -53,7 +53,7 @@ namespace xjpcg {
 namespace {
 constexpr int kLoopThreads = 384;   // 168 registers; with 512 (128 registers) the pipelined steps spill
 constexpr int kVecThreads = 256;    // threads that update r and z: enough to fill the FP64 pipe, and every warp costs two sums
-constexpr int kStep = 7;            // stored columns per step of a row (27 = 7 + 7 + 7 + 6)
+constexpr int kStep[2] = {7, 9};    // stored columns per step of a row
 constexpr int kCols = 8;            // the same in the cluster form
 constexpr int kPosts = 5;           // posts a lane reads at once: 152 CTAs in one step
 constexpr uint64_t kLoopBudgetNs = 2000000000ull;  // 2 s
@@ -142,9 +142,10 @@ __device__ __forceinline__ double grid_total(double s, ulonglong2* posts, uint32
 }
 }  // namespace
 
-// One step of a row, up to kStep stored columns.
+// One step of a row, up to K stored columns.
+template <int K>
 struct Step {
-    double v[kStep], x[kStep];
+    double v[K], x[K];
     int ls, rem;  // slice; its columns from this step's first on
 };
 // A step's place in the matrix.
@@ -162,7 +163,8 @@ struct StepAt {
 //   p = z + beta p, also to global -> barrier (release / acquire)
 // Only the last needs fences: the posts of the sums carry their own tags.
 // LAY: 0 int32 columns, 1 int16 offsets, 2 slice-shared offsets.
-template <int LAY>
+// K: stored columns per step.
+template <int LAY, int K>
 __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
     __shared__ double sAlpha, sBeta, sRz, sRr;
@@ -215,8 +217,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
 
     // A step passes through three stages: its columns are loaded, then its values
     // and p, then the products are summed.  A warp has one step in each.
-    int cols[kStep];
-    Step A, B;
+    int cols[K];
+    Step<K> A, B;
     auto slice = [&](int ls) {
         const int4 md = meta[min(ls, ns - 1)];
         StepAt t;
@@ -228,11 +230,11 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
         return t;
     };
     auto next = [&](const StepAt& t) {
-        if (t.rem <= kStep) return slice(t.ls + nw);
+        if (t.rem <= K) return slice(t.ls + nw);
         StepAt l = t;
-        l.rem -= kStep;
-        l.v += kStep * 32;
-        l.c += t.shared ? kStep : kStep * 32;
+        l.rem -= K;
+        l.v += K * 32;
+        l.c += t.shared ? K : K * 32;
         return l;
     };
     auto load_col = [&](const StepAt& t, int u) {
@@ -248,7 +250,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
         if (wid >= ns) return;
         const StepAt t = slice(wid);
 #pragma unroll
-        for (int u = 0; u < kStep; ++u)
+        for (int u = 0; u < K; ++u)
             if (u < t.rem) {
                 cols[u] = load_col(t, u);
                 A.v[u] = ld_val(a.sval + t.v + u * 32);
@@ -271,24 +273,24 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
                 const double* const pb = base_of(pos);
                 const StepAt l = next(pos);
 #pragma unroll
-                for (int u = 0; u < kStep; ++u) {
+                for (int u = 0; u < K; ++u) {
                     if (u < pos.rem) A.x[u] = pb[cols[u]];
                     if (u < l.rem) cols[u] = load_col(l, u);
                 }
                 pos = l;
             }
-            auto finish = [&](const Step& f) {
-                if (f.rem > kStep) return;  // more of the slice to come
+            auto finish = [&](const Step<K>& f) {
+                if (f.rem > K) return;  // more of the slice to come
                 const int r = f.ls * 32 + lane;
                 const bool in = row0 + r < a.n;
                 sz[r] = in ? acc : 0.0;
                 if (in) dacc = fma(sp[r], acc, dacc);
                 acc = 0.0;
             };
-            auto step = [&](const Step& f, Step& g) {  // pos: g's place
+            auto step = [&](const Step<K>& f, Step<K>& g) {  // pos: g's place
                 if (pos.ls >= ns) {  // f is the warp's last
 #pragma unroll
-                    for (int u = 0; u < kStep; ++u)
+                    for (int u = 0; u < K; ++u)
                         if (u < f.rem) acc = fma(f.v[u], f.x[u], acc);
                     finish(f);
                     return false;
@@ -299,9 +301,9 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
                 g.ls = pos.ls;
                 g.rem = pos.rem;
                 // the stages' instructions alternate, as a dependent FMA takes 64 cycles
-                if (min(min(f.rem, pos.rem), l.rem) >= kStep) {
+                if (min(min(f.rem, pos.rem), l.rem) >= K) {
 #pragma unroll
-                    for (int u = 0; u < kStep; ++u) {
+                    for (int u = 0; u < K; ++u) {
                         g.x[u] = pb[cols[u]];
                         g.v[u] = ld_val(vp + u * 32);
                         cols[u] = load_col(l, u);
@@ -309,7 +311,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
                     }
                 } else {
 #pragma unroll
-                    for (int u = 0; u < kStep; ++u) {
+                    for (int u = 0; u < K; ++u) {
                         if (u < pos.rem) {
                             g.x[u] = pb[cols[u]];
                             g.v[u] = ld_val(vp + u * 32);
@@ -681,9 +683,9 @@ LoopShape loop_shape(int n, int numSms) {
     return s;
 }
 
-template <int LAY>
+template <int LAY, int K>
 cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
-    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(cg_loop_kernel<LAY, K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kLoopSmem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
@@ -696,7 +698,12 @@ cudaError_t loop_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) 
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY>, a);
+    return cudaLaunchKernelEx(&cfg, cg_loop_kernel<LAY, K>, a);
+}
+
+template <int LAY>
+cudaError_t loop_launch_steps(int step, cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
+    return step == kStep[1] ? loop_launch<LAY, kStep[1]>(st, s, a) : loop_launch<LAY, kStep[0]>(st, s, a);
 }
 
 // The cluster form: its CTAs' rows and shared memory.
@@ -797,16 +804,28 @@ bool cg_loop_fits(int n, int numSms) { return n > 0 && loop_shape(n, numSms).fix
 
 size_t cg_loop_sync_bytes(int numSms) { return 128 * sizeof(uint32_t) + 3 * sizeof(ulonglong2) * 2 * (size_t)numSms; }
 
-cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a) {
+// Steps of 9 where rows of the mean length take fewer of them than of 7: a step
+// costs its instructions besides the products, and one with columns to spare
+// more (27-point 96^3: 63.4 us per iteration with 9 = 3 steps, 69.1 with 7; 7-point
+// 96^3: 40.2 with 9, 33.6 with 7).  Not where a warp has one slice at most, and
+// the wait for a step's own loads counts (27-point 32^3: 12.0 with 9, 11.5 with 7).
+static int loop_step(int n, int64_t stored, const LoopShape& s) {
+    const int64_t rows = ((int64_t)n + 31) / 32 * 32, mean = (stored + rows - 1) / rows;
+    const bool fewer = (mean + kStep[1] - 1) / kStep[1] < (mean + kStep[0] - 1) / kStep[0];
+    return fewer && s.rows > s.threads ? kStep[1] : kStep[0];
+}
+
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, int64_t stored, void* sync, LoopArgs a) {
     const LoopShape s = loop_shape(a.n, numSms);
+    const int step = loop_step(a.n, stored, s);
     a.nslices = (a.n + 31) / 32;
     a.rows = s.rows;
     a.jOnChip = s.jOnChip ? 1 : 0;
     a.counters = static_cast<uint32_t*>(sync);
     a.posts = reinterpret_cast<ulonglong2*>(a.counters + 128);
-    if (layout == 0) return loop_launch<0>(st, s, a);
-    if (layout == 1) return loop_launch<1>(st, s, a);
-    return loop_launch<2>(st, s, a);
+    if (layout == 0) return loop_launch_steps<0>(step, st, s, a);
+    if (layout == 1) return loop_launch_steps<1>(step, st, s, a);
+    return loop_launch_steps<2>(step, st, s, a);
 }
 
 }  // namespace xjpcg

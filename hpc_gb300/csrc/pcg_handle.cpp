@@ -1071,7 +1071,7 @@ void PcgHandle::launchLoopKernel(int form, int layout, uint32_t maxIter) {
     }
     a.tag0 = m_loopTag;
     m_loopTag += maxIter + 1u;
-    check(cg_loop_launch(m_stream, layout, m_numSms, m_loopSync.p, a), "loop kernel");
+    check(cg_loop_launch(m_stream, layout, m_numSms, pat ? m_psTotal : m_sellTotal, m_loopSync.p, a), "loop kernel");
 }
 
 // The mixed loop's FP32 update after its SpMV: the fused cooperative kernel

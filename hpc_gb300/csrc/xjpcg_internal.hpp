@@ -190,9 +190,9 @@ bool cg_loop_fits(int n, int numSms);  // the grid form
 bool cg_cluster_fits(int n, int64_t stored);
 cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a);
 size_t cg_loop_sync_bytes(int numSms);
-// layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
+// stored: entries of the layout; layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
 // offsets; sync: cg_loop_sync_bytes bytes, the first 512 cleared before each launch.
-cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, void* sync, LoopArgs a);
+cudaError_t cg_loop_launch(cudaStream_t st, int layout, int numSms, int64_t stored, void* sync, LoopArgs a);
 
 // ---- mixed precision, reliable updates (mixed_kernels.cu) ----
 cudaError_t rel_init_launch(int grid, cudaStream_t s, int n, int n4, const double* b, const double* diag, double* x,

@@ -27,7 +27,8 @@ SYSTEMS = {
     "wide_plane": ((3, 190, 191), True, "grid"),  # columns beyond int16 offsets
     "matrix_just_on_chip": ((47, 48, 49), False, "grid"),
     "matrix_partly_on_chip": ((79, 80, 81), True, "grid"),
-    "steps_of_7_7_4": ((2, 310, 311), False, "grid"),  # no int16 offsets
+    "steps_of_9": ((2, 310, 311), False, "grid"),  # 18 entries a row, no int16 offsets
+    "steps_of_7_and_5": ((2, 2, 7001), False, "grid"),
     "empty_slices": ((20, 21, 23), False, "grid"),
     "J_just_on_chip": ((94, 95, 96), True, "grid"),
     "J_not_on_chip": ((96, 97, 97), True, "grid"),
@@ -77,7 +78,7 @@ def test_loop_kernel_matches_the_host_loop(gpu_lib, name):
     host = _solves(s, {"XJPCG_SPMV_LANES": "-1", "XJPCG_HOST_LOOP": "1"}, calls)
     default = _solves(s, {}, calls)
     runs = [default]
-    for lanes in ("-1", "-5") if name in ("wide_plane", "steps_of_7_7_4") else ("-1", "-3", "-5"):
+    for lanes in ("-1", "-5") if name in ("wide_plane", "steps_of_9") else ("-1", "-3", "-5"):
         runs.append(_solves(s, {"XJPCG_SPMV_LANES": lanes, "XJPCG_LOOP_KERNEL": "1"}, calls))
     for run in runs:
         (ra, reca, ia), (rb, _, _), (rc, _, _) = run
