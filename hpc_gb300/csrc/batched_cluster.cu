@@ -583,11 +583,11 @@ __global__ void batch_rows_kernel(int nsys, int total, const int* __restrict__ s
         if (rowptr[r + 1] < rowptr[r]) atomicOr(flag, 2);
 }
 
-// One thread per row: the longest row of every system, and flag bit 4 for a
-// column outside its system.
+// One thread per row: the longest row of every system, how far its columns reach
+// from the diagonal, and flag bit 4 for a column outside its system.
 __global__ void batch_widths_kernel(int nsys, int total, const int* __restrict__ sysRow,
                                     const int* __restrict__ rowptr, const int* __restrict__ col, int* __restrict__ width,
-                                    int* flag) {
+                                    int* __restrict__ reach, int* flag) {
     for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < total; r += gridDim.x * blockDim.x) {
         int lo = 0, hi = nsys - 1;  // the system of row r
         while (lo < hi) {
@@ -599,11 +599,18 @@ __global__ void batch_widths_kernel(int nsys, int total, const int* __restrict__
         }
         const int n = sysRow[lo + 1] - sysRow[lo];
         const int e0 = rowptr[r], e1 = rowptr[r + 1];
+        const int row = r - sysRow[lo];
+        int far = 0;
         bool bad = false;
-        for (int e = e0; e < e1; ++e) bad = bad || (unsigned)col[e] >= (unsigned)n;
+        for (int e = e0; e < e1; ++e) {
+            const int c = col[e];
+            bad = bad || (unsigned)c >= (unsigned)n;
+            far = max(far, bad ? 0 : abs(c - row));
+        }
         if (bad) atomicOr(flag, 4);
         // most rows are as long as the longest: look before the atomic
         if (*(volatile int*)&width[lo] < e1 - e0) atomicMax(&width[lo], e1 - e0);
+        if (*(volatile int*)&reach[lo] < far) atomicMax(&reach[lo], far);
     }
 }
 
@@ -615,9 +622,9 @@ cudaError_t batch_check_rows(cudaStream_t st, int nsys, int total, const int* sy
 }
 
 cudaError_t batch_widths(cudaStream_t st, int nsys, int total, const int* sysRow, const int* rowptr, const int* col,
-                         int* width, int* flag) {
+                         int* width, int* reach, int* flag) {
     batch_widths_kernel<<<std::max(1, std::min((total + 255) / 256, device_sm_count() * 8)), 256, 0, st>>>(
-        nsys, total, sysRow, rowptr, col, width, flag);
+        nsys, total, sysRow, rowptr, col, width, reach, flag);
     return cudaGetLastError();
 }
 

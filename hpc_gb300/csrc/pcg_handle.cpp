@@ -1769,10 +1769,10 @@ void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* 
         if (in.sys[s + 1] - in.sys[s] <= 0) throw InvalidValue("every system needs at least one row.");
     const int total = in.sys[nsys];
     alloc(m_bSysRow, sizeof(int32_t) * (nsys + 1), "batch offsets");
-    alloc(m_bWidth, sizeof(int32_t) * (2 * (size_t)nsys + 1), "batch widths");
+    alloc(m_bWidth, sizeof(int32_t) * (3 * (size_t)nsys + 1), "batch widths");  // widths, reaches, entries
     check(cudaMemcpyAsync(m_bSysRow.p, in.sys.data(), sizeof(int32_t) * (nsys + 1), cudaMemcpyHostToDevice, m_stream),
           "H2D");
-    check(cudaMemsetAsync(m_bWidth.p, 0, sizeof(int32_t) * nsys, m_stream), "memset");
+    check(cudaMemsetAsync(m_bWidth.p, 0, sizeof(int32_t) * 2 * nsys, m_stream), "memset");
     check(cudaMemsetAsync(m_flags.p, 0, sizeof(int), m_stream), "memset");
     auto place = [&](DevBuf& buf, const void* src, size_t elem, size_t count, const char* what) -> const void* {
         if (onDevice && reinterpret_cast<uintptr_t>(src) % elem == 0) return src;
@@ -1784,7 +1784,7 @@ void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* 
     };
     in.rowptr = static_cast<const int*>(place(m_bRowptr, rowPtr, 4, (size_t)total + 1, "batch row pointers"));
     // the row pointers are checked before any column is read through them
-    int* const entry = m_bWidth.as<int>() + nsys;
+    int* const entry = m_bWidth.as<int>() + 2 * (size_t)nsys;
     check(batch_check_rows(m_stream, (int)nsys, total, m_bSysRow.as<int>(), in.rowptr, entry, m_flags.as<int>()),
           "row pointer check");
     int flag = 0;
@@ -1800,13 +1800,25 @@ void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* 
     in.b = static_cast<const double*>(place(m_bB, b, 8, (size_t)total, "batch b"));
     in.diag = static_cast<const double*>(place(m_bDiag, diag, 8, (size_t)total, "batch diag"));
     check(batch_widths(m_stream, (int)nsys, total, m_bSysRow.as<int>(), in.rowptr, in.col, m_bWidth.as<int>(),
-                       m_flags.as<int>()),
+                       m_bWidth.as<int>() + nsys, m_flags.as<int>()),
           "column check");
-    in.width.resize(nsys);
+    in.width.resize(2 * (size_t)nsys);  // and the reaches behind them
     check(cudaMemcpyAsync(&flag, m_flags.p, sizeof(int), cudaMemcpyDeviceToHost, m_stream), "D2H");
-    check(cudaMemcpyAsync(in.width.data(), m_bWidth.p, sizeof(int32_t) * nsys, cudaMemcpyDeviceToHost, m_stream), "D2H");
+    check(cudaMemcpyAsync(in.width.data(), m_bWidth.p, sizeof(int32_t) * 2 * nsys, cudaMemcpyDeviceToHost, m_stream),
+          "D2H");
     check(cudaStreamSynchronize(m_stream), "sync");
     if (flag & 4) throw InvalidValue("a column index lies outside its system.");
+    // Work of a system: FP64 operations per iteration times the iterations, which
+    // follow the number of steps that a value needs across the system: rows over
+    // the columns' reach (the square root of the rows in 2 dimensions, the cube root
+    // in 3), and not above the square root.  On 1,024 grids of 200 - 20,000 rows the
+    // iterations were 5.0 to 9.0 times that, and 1.2 to 6.4 times the square root.
+    in.work.resize(nsys);
+    for (uint32_t s = 0; s < nsys; ++s) {
+        const double n = in.sys[s + 1] - in.sys[s], reach = std::max(1, in.width[nsys + s]);
+        in.work[s] = ((double)(in.entry[s + 1] - in.entry[s]) + 7.0 * n) * std::min(std::sqrt(n), n / reach);
+    }
+    in.width.resize(nsys);
 }
 
 // The batch with every system in shared memory (batched_cluster.cu).  False
@@ -1865,10 +1877,10 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
     alloc(m_bOrder, sizeof(int32_t) * nsys, "batch order");
     std::vector<int32_t> order(nsys);
     for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
-    // by class, the largest first in each
+    // by class, the longest first in each
     std::stable_sort(order.begin(), order.end(), [&](int32_t p, int32_t q) {
         if (cls[p] != cls[q]) return cls[p] > cls[q];
-        return hSys[p + 1] - hSys[p] > hSys[q + 1] - hSys[q];
+        return in.work[p] > in.work[q];
     });
     check(cudaMemcpyAsync(m_bOrder.p, order.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice, m_stream), "H2D");
     a.width = m_bWidth.as<int>();
@@ -1936,26 +1948,23 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     m_batchClusterCtas = 0;
     if (!forcedShape && envInt("XJPCG_BATCH_CLUSTERS", 1) != 0 && batchClusters(in, maxIter, tol, mixed))
         return batchResults(nsys, total, x, tol, results, onDevice);
-    // Queue order: largest systems first so the long solves start early.
+    // Queue order: the longest solves first.
     std::vector<int32_t> order(nsys);
     for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
     std::stable_sort(order.begin(), order.end(),
-                     [&](int32_t a, int32_t c) { return entry[a + 1] - entry[a] > entry[c + 1] - entry[c]; });
+                     [&](int32_t a, int32_t c) { return in.work[a] > in.work[c]; });
     // Systems too long for one CTA next to the batch's average share can go to
-    // teams of CTAs: their work, entries x sqrt(rows) for want of iteration
-    // counts, is above a quarter of the work per SM.  fp64 / mixed ms with 0.40 /
-    // 0.30 / 0.22 of it: 1,024 systems of 200 - 20,000 rows 45.8 / 46.3 / 46.3 and
-    // 24.3 / 23.9 / 24.6; 2,000 of them 71 / 67 / 63 and 32.0 / 33.6 / 35.2.
+    // teams of CTAs: their work is above 0.35 of the work per SM.  fp64 / mixed ms
+    // with 0.15, 0.25, 0.35, 0.50 of it: 1,024 systems of 200 - 20,000 rows 45.9 /
+    // 24.6, 45.0 / 24.3, 42.3 / 24.9, 42.9 / 24.1; 2,000 of them 63.9 / 36.0, 62.8 /
+    // 35.3, 62.4 / 33.9, 61.8 / 32.8; 600 of 1,000 - 8,000 16.0 / 11.9, 15.2 / 11.1,
+    // 14.4 / 10.3, 15.4 / 10.0.
     std::vector<uint8_t> isLong(nsys, 0);
     {
-        auto workOf = [&](uint32_t i) {
-            const double n = hSys[i + 1] - hSys[i];
-            return ((double)(entry[i + 1] - entry[i]) + 7.0 * n) * std::sqrt(n);
-        };
         double allWork = 0.0;
-        for (uint32_t i = 0; i < nsys; ++i) allWork += workOf(i);
-        const double share = 0.25 * allWork / m_numSms;
-        for (uint32_t i = 0; i < nsys; ++i) isLong[i] = workOf(i) > share && hSys[i + 1] - hSys[i] > 2048 ? 1 : 0;
+        for (uint32_t i = 0; i < nsys; ++i) allWork += in.work[i];
+        const double share = 0.35 * allWork / m_numSms;
+        for (uint32_t i = 0; i < nsys; ++i) isLong[i] = in.work[i] > share && hSys[i + 1] - hSys[i] > 2048 ? 1 : 0;
     }
     std::vector<int32_t> teamOrder(order);
     std::stable_sort(teamOrder.begin(), teamOrder.end(), [&](int32_t p, int32_t q) { return isLong[p] < isLong[q]; });

@@ -210,6 +210,7 @@ class PcgHandle {
     // A batch's arrays on the device, and what the host needs of them.
     struct BatchInput {
         std::vector<int32_t> sys, entry, width;  // first row and entry of each system (and the ends), longest row
+        std::vector<double> work;                // of each system, a guess
         const int *rowptr = nullptr, *col = nullptr;
         const double *val = nullptr, *diag = nullptr, *b = nullptr;
     };

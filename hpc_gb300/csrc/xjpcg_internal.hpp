@@ -276,9 +276,10 @@ cudaError_t batch_cluster_launch(cudaStream_t st, bool mixed, bool small, int sy
 // flag |= 1: rowptr[0] != 0, 2: not monotone; entry[s] = rowptr[sysRow[s]], nsys + 1 of them
 cudaError_t batch_check_rows(cudaStream_t st, int nsys, int total, const int* sysRow, const int* rowptr, int* entry,
                              int* flag);
-// width[s]: longest row of system s (cleared before); flag |= 4: a column outside its system
+// width[s], reach[s]: longest row of system s, and how far columns lie from the
+// diagonal (cleared before); flag |= 4: a column outside its system
 cudaError_t batch_widths(cudaStream_t st, int nsys, int total, const int* sysRow, const int* rowptr, const int* col,
-                         int* width, int* flag);
+                         int* width, int* reach, int* flag);
 void batch_config_shape(int cfg, int* threads, int* lanes);
 bool batch_config_sliced(int cfg);  // the kernel reads the per-system SELL-32 copy
 // Shared column offsets per slice of the batched SELL-32 copy: at most this
