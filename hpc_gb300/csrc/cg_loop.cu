@@ -31,13 +31,15 @@
 // either way, 64^3 16.9 and 16.8; 27-point 48^3 17.9 and 17.4).
 //
 // Measured, us per iteration (two kernels per iteration / loop / cluster):
-//   7-point   16^3   14.7 /  8.8 / 6.7      27-point   8^3  15.1 / 13.1 / 6.5
-//             32^3   14.9 /  9.6 /  -                 16^3  16.9 / 10.9 / 8.4
-//             48^3   18.1 / 12.4 /  -                 32^3  18.6 / 11.5 /  -
-//             64^3   25.1 / 16.7 /  -                 48^3  24.6 / 17.4 /  -
-//             80^3   33.1 / 23.2 /  -                 60^3  32.7 / 23.9 /  -
-//             96^3   42.2 / 33.2 /  -                 80^3  50.3 / 40.5 /  -
-//            102^3   44.9 / 37.7 /  -                 96^3  73.5 / 63.4 /  -
+//   7-point   16^3   14.7 /  8.8 / 5.7      27-point   8^3  15.1 / 13.1 / 6.3
+//             24^3   15.1 /  8.9 / 8.5                16^3  16.9 / 10.2 / 7.6
+//             32^3   14.9 /  9.5 /  -                 32^3  18.6 / 11.3 /  -
+//             48^3   18.1 / 12.0 /  -                 48^3  24.6 / 16.9 /  -
+//             64^3   25.1 / 16.4 /  -                 60^3  32.7 / 23.6 /  -
+//             80^3   33.1 / 23.1 /  -                 80^3  50.3 / 40.7 /  -
+//             96^3   42.2 / 33.2 /  -                 96^3  73.5 / 63.6 /  -
+//            102^3   44.9 / 37.9 /  -                102^3  81.7 / 73.5 /  -
+// (sums by a shuffle tree in every warp: cluster 16^3 6.6, 20^3 9.0 against 7.2)
 //
 // Every row is summed in its stored order, as in the sliced SpMV kernels; the
 // dot products are summed per thread, per warp, per CTA and over the CTAs, in
@@ -88,6 +90,25 @@ __device__ __forceinline__ double lanes_sum(double v, int count) {
     for (int o = 16; o > 0; o >>= 1)
         if (o < count) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
+}
+
+// This thread's warp, as a value that the compiler knows to be the same in all
+// lanes: shuffles under a test of it need no reconvergence.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// Sum of the values that nw warps' threads left in shared memory, by one warp:
+// over the lanes in groups of `width`, in each group's first lane.  A warp-wide add
+// holds the SM's FP64 pipe for 16 cycles: a shuffle tree in each of 8 warps is 40
+// of them, this is 12 for all.
+__device__ __forceinline__ double threads_sum(const double* v, int nw, int lane, int width = 32) {
+    double s[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) s[u] = u < nw ? v[u * 32 + lane] : 0.0;
+    for (int w = 4; w < nw; w += 4)
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (w + u < nw) s[u] += v[(w + u) * 32 + lane];
+    return lanes_sum((s[0] + s[1]) + (s[2] + s[3]), width);
 }
 
 // A CTA's total to every CTA and back, by one warp: the sum of all CTAs'
@@ -169,7 +190,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
     __shared__ double sAlpha, sBeta, sRz, sRr;
     __shared__ int sGo[3];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wid = warp_index(), nt = blockDim.x, nw = nt >> 5;
     const int q = blockIdx.x, P = gridDim.x;
     const int s0 = (int)((int64_t)a.nslices * q / P), s1 = (int)((int64_t)a.nslices * (q + 1) / P);
     const int ns = s1 - s0, pairs = ns * 16, row0 = s0 * 32;
@@ -178,8 +199,8 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     double* const sz = sx + a.rows;
     double* const sp = sz + a.rows;
     double* const sj = sp + a.rows;
-    double* const part = sj + (a.jOnChip ? a.rows : 0);  // 2 per warp
-    int4* const meta = reinterpret_cast<int4*>(part + 64);
+    double* const part = sj + (a.jOnChip ? a.rows : 0);  // 1 per thread
+    int4* const meta = reinterpret_cast<int4*>(part + kLoopThreads);
 
     for (int i = tid; i < pairs; i += nt) {
         const int e = row0 / 2 + i;
@@ -211,9 +232,6 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
     // shared or global, read through one pointer
     const double2* const j2 = a.jOnChip ? reinterpret_cast<const double2*>(sj) : reinterpret_cast<const double2*>(a.J) + row0 / 2;
     const int vecStride = min(nt, kVecThreads);
-
-    int nwUp = 1;
-    while (nwUp < nw) nwUp *= 2;
 
     // A step passes through three stages: its columns are loaded, then its values
     // and p, then the products are summed.  A warp has one step in each.
@@ -327,11 +345,10 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
             while (step(A, B) && step(B, A)) {
             }
         }
-        dacc = warp_sum(dacc);
-        if (lane == 0) part[wid] = dacc;
+        part[tid] = dacc;
         __syncthreads();
         if (wid == 0) {
-            double s = lanes_sum(lane < nw ? part[lane] : 0.0, nwUp);
+            double s = threads_sum(part, nw, lane);
             s = grid_total(s, a.posts, a.counters, target, tag, lane, ok);
             if (lane == 0) {
                 const double al = sRz / s;
@@ -364,16 +381,14 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
             reinterpret_cast<double2*>(sz)[i] = zv;
         }
         if (tid < kVecThreads) {
-            rr = warp_sum(rr);
-            rz = warp_sum(rz);
-            if (lane == 0) {
-                part[wid] = rr;
-                part[32 + wid] = rz;
-            }
+            // the lower lanes go on with r.r, the upper with r.z
+            const double other = __shfl_xor_sync(0xffffffffu, lane < 16 ? rz : rr, 16);
+            part[tid] = (lane < 16 ? rr : rz) + other;
         }
         __syncthreads();
         if (wid < 2) {
-            double s = lanes_sum(lane < min(nw, kVecThreads / 32) ? part[32 * wid + lane] : 0.0, min(nwUp, kVecThreads / 32));
+            double s = threads_sum(part, min(nw, kVecThreads / 32), lane, 16);
+            s = __shfl_sync(0xffffffffu, s, 16 * wid);
             s = grid_total(s, a.posts + (1 + wid) * P, a.counters + (1 + wid) * 32, target, tag, lane, ok);
             if (lane == 0) {
                 if (wid == 0) {
@@ -462,7 +477,6 @@ namespace {
 constexpr int kClusterThreads = 512;
 constexpr int kClusterMax = 16;
 constexpr size_t kClusterSmem = 212 * 1024;  // beside 14 KB of static shared memory
-constexpr int kClusterSlots = kClusterMax * (kClusterThreads / 32);
 
 // Every thread of the cluster; distributed shared memory written before is
 // visible after.
@@ -489,26 +503,21 @@ __device__ __forceinline__ void to_all(double* place, double v, int P, int lane)
         asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(map_rank(place, (uint32_t)lane)), "d"(v) : "memory");
 }
 
-__device__ __forceinline__ double slots_sum(const double* slots, int count, int lane) {
-    double s = lane < count ? slots[lane] : 0.0;
-    for (int i = lane + 32; i < count; i += 32) s += slots[i];
-    return warp_sum(s);
-}
 }  // namespace
 
 // One cluster.  R rows per CTA, so a column's owner is column / R.  The matrix
 // part in shared memory holds, per entry, the value and the cluster address of
-// its p, so a gather is one load (about 250 cycles).  Every warp writes its part
-// of a sum to every CTA; after the cluster barrier each CTA adds all of them in
-// the same order.  A CTA always runs to the same decision as the others, and no
+// its p, so a gather is one load (about 250 cycles).  Every CTA writes its part
+// of a sum to every CTA; after the cluster barrier each adds all of them in the
+// same order.  A CTA always runs to the same decision as the others, and no
 // CTA is read or written by another after its last cluster barrier.
 template <int LAY>
 __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
-    __shared__ double slots[3][kClusterSlots];
+    __shared__ double slots[3][kClusterMax], part[2][kClusterThreads];
     __shared__ double sAlpha, sBeta, sRz, sRr;
     __shared__ int sGo[3];
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nt = blockDim.x, nw = nt >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wid = warp_index(), nt = blockDim.x, nw = nt >> 5;
     const int q = blockIdx.x, P = gridDim.x, R = a.rows;
     const int s0 = q * (R / 32), ns = max(0, min(R / 32, a.nslices - s0)), row0 = s0 * 32;
     double* const sr = reinterpret_cast<double*>(loopSmem);
@@ -592,10 +601,12 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
             sz[r] = acc;
             dacc = fma(sp[r], acc, dacc);
         }
-        to_all(&slots[0][q * nw + wid], warp_sum(dacc), P, lane);
+        part[0][tid] = dacc;
+        __syncthreads();
+        if (wid == 0) to_all(&slots[0][q], threads_sum(part[0], nw, lane), P, lane);
         cluster_sync();
         if (wid == 0) {
-            const double s = slots_sum(slots[0], P * nw, lane);
+            const double s = lanes_sum(lane < P ? slots[0][lane] : 0.0, kClusterMax);
             if (lane == 0) {
                 const double al = sRz / s;
                 sAlpha = al;
@@ -615,13 +626,13 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
             sr[i] = rv;
             sz[i] = zv;
         }
-        rr = warp_sum(rr);
-        rz = warp_sum(rz);
-        to_all(&slots[1][q * nw + wid], rr, P, lane);
-        to_all(&slots[2][q * nw + wid], rz, P, lane);
+        part[0][tid] = rr;
+        part[1][tid] = rz;
+        __syncthreads();
+        if (wid < 2) to_all(&slots[1 + wid][q], threads_sum(part[wid], nw, lane), P, lane);
         cluster_sync();
         if (wid < 2) {
-            const double s = slots_sum(slots[1 + wid], P * nw, lane);
+            const double s = lanes_sum(lane < P ? slots[1 + wid][lane] : 0.0, kClusterMax);
             if (lane == 0) {
                 if (wid == 0) {
                     sRr = s;
@@ -677,7 +688,7 @@ LoopShape loop_shape(int n, int numSms) {
     const int ns = (nslices + s.P - 1) / s.P;
     s.rows = 32 * ns;
     s.threads = std::max(64, std::min(kLoopThreads, 32 * ns));
-    const size_t other = sizeof(double) * 64 + sizeof(int4) * (size_t)ns;
+    const size_t other = sizeof(double) * kLoopThreads + sizeof(int4) * (size_t)ns;
     s.jOnChip = sizeof(double) * 5 * (size_t)s.rows + other <= kLoopSmem;
     s.fixed = sizeof(double) * (s.jOnChip ? 5 : 4) * (size_t)s.rows + other;
     return s;
@@ -775,11 +786,11 @@ cudaError_t cluster_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& 
 }
 }  // namespace
 
-// FP64 operations of an iteration up to which 16 SMs finish before 152 do:
-// the cluster form wins by 25 % at 56,000 (7-point 16^3) and 23 % at 126,000
-// (27-point 16^3); at 112,000 (7-point 20^3) both take 9 us, and at 251,000
-// (27-point 20^3) the grid form is ahead, 11.1 against 11.9 us.
-constexpr int64_t kClusterWork = 130000;
+// FP64 operations of an iteration up to which 16 SMs finish before 152 do.  us per
+// iteration, cluster / grid: 7-point 20^3 (112,000) 7.2 / 9.1, 24^3 (194,000) 8.5 /
+// 8.9, 26^3 (246,000) 9.9 / 9.0; 27-point 16^3 (139,000) 7.6 / 10.2, 18^3 (198,000)
+// 9.0 / 10.7, 20^3 (272,000) 10.6 / 10.6.
+constexpr int64_t kClusterWork = 210000;
 
 bool cg_cluster_fits(int n, int64_t stored) {
     if (n <= 0 || stored + 7 * (int64_t)n > kClusterWork) return false;
@@ -799,7 +810,7 @@ cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a) {
     return cluster_launch<2>(st, s, a);
 }
 
-// The vectors have to fit in shared memory, all but J (1,079,808 rows on 152 SMs; J too up to 865,792).
+// The vectors have to fit in shared memory, all but J (1,065,216 rows on 152 SMs; J too up to 856,064).
 bool cg_loop_fits(int n, int numSms) { return n > 0 && loop_shape(n, numSms).fixed <= kLoopSmem; }
 
 size_t cg_loop_sync_bytes(int numSms) { return 128 * sizeof(uint32_t) + 3 * sizeof(ulonglong2) * 2 * (size_t)numSms; }

@@ -21,16 +21,16 @@ SYSTEMS = {
     "one_slice": ((2, 4, 4), False, "cluster"),
     "slice_and_a_row": ((1, 3, 11), True, "cluster"),
     "uneven_rows": ((7, 8, 9), False, "cluster"),
-    "largest_cluster": ((20, 21, 21), True, "cluster"),
-    "smallest_grid": ((22, 22, 23), True, "grid"),
-    "a_slice_per_sm_and_one": ((17, 13, 23), False, "grid"),
+    "largest_cluster": ((24, 24, 25), True, "cluster"),
+    "smallest_grid": ((25, 25, 25), True, "grid"),
+    "a_slice_per_sm_and_one": ((17, 13, 23), False, "cluster"),
     "wide_plane": ((3, 190, 191), True, "grid"),  # columns beyond int16 offsets
     "matrix_just_on_chip": ((47, 48, 49), False, "grid"),
     "matrix_partly_on_chip": ((79, 80, 81), True, "grid"),
     "steps_of_9": ((2, 310, 311), False, "grid"),  # 18 entries a row, no int16 offsets
     "steps_of_7_and_5": ((2, 2, 7001), False, "grid"),
     "empty_slices": ((20, 21, 23), False, "grid"),
-    "J_just_on_chip": ((94, 95, 96), True, "grid"),
+    "J_just_on_chip": ((94, 95, 95), True, "grid"),
     "J_not_on_chip": ((96, 97, 97), True, "grid"),
     "vectors_too_large": ((103, 103, 104), True, "graph"),
 }
