@@ -23,8 +23,8 @@
 // the 64-cycle FMAs of a row overlap.  With 12 warps per SM they do so only when
 // each warp works on three steps at once: columns of one on their way, values
 // and p of the next, sums of the one before, instruction by instruction.  7-point
-// 96^3 33.2 us per iteration: 27,700 cycles for the product (23,300 of issue at
-// the least), 14,700 for r and z, 6,900 for x and p, the rest waiting for sums.
+// 96^3 32.4 us per iteration: 27,700 cycles for the product (23,300 of issue at
+// the least), 14,700 for r and z, 5,000 for p, the rest waiting for sums.
 // Loading values and columns a step ahead but gathering when needed took 48.7
 // us, the three stages one after another 39.2.  Keeping the matrix in what is
 // left of shared memory gained nothing over streaming it (7-point 32^3 9.5 us
@@ -33,12 +33,12 @@
 // Measured, us per iteration (two kernels per iteration / loop / cluster):
 //   7-point   16^3   14.7 /  8.8 / 5.7      27-point   8^3  15.1 / 13.1 / 6.3
 //             24^3   15.1 /  8.9 / 8.5                16^3  16.9 / 10.2 / 7.6
-//             32^3   14.9 /  9.5 /  -                 32^3  18.6 / 11.3 /  -
-//             48^3   18.1 / 12.0 /  -                 48^3  24.6 / 16.9 /  -
-//             64^3   25.1 / 16.4 /  -                 60^3  32.7 / 23.6 /  -
-//             80^3   33.1 / 23.1 /  -                 80^3  50.3 / 40.7 /  -
-//             96^3   42.2 / 33.2 /  -                 96^3  73.5 / 63.6 /  -
-//            102^3   44.9 / 37.9 /  -                102^3  81.7 / 73.5 /  -
+//             32^3   14.9 /  9.5 /  -                 32^3  18.6 / 11.2 /  -
+//             48^3   18.1 / 11.4 /  -                 48^3  24.6 / 16.8 /  -
+//             64^3   25.1 / 15.9 /  -                 60^3  32.7 / 23.1 /  -
+//             80^3   33.1 / 22.1 /  -                 80^3  50.3 / 40.2 /  -
+//             96^3   42.2 / 32.4 /  -                 96^3  73.5 / 61.9 /  -
+//            102^3   44.9 / 37.2 /  -                102^3  81.7 / 72.1 /  -
 // (sums by a shuffle tree in every warp: cluster 16^3 6.6, 20^3 9.0 against 7.2)
 //
 // Every row is summed in its stored order, as in the sliced SpMV kernels; the
@@ -180,7 +180,7 @@ struct StepAt {
 // its L1).  Per iteration:
 //   Ap = A p into sz, p.Ap        -> grid sum, alpha
 //   r -= alpha Ap, z = J r        -> grid sums of r.r and r.z, beta, stop test;
-//                                    the idle warps do x += alpha p meanwhile
+//                                    the other warps do x += alpha p meanwhile
 //   p = z + beta p, also to global -> barrier (release / acquire)
 // Only the last needs fences: the posts of the sums carry their own tags.
 // LAY: 0 int32 columns, 1 int16 offsets, 2 slice-shared offsets.
@@ -386,6 +386,15 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
             part[tid] = (lane < 16 ? rr : rz) + other;
         }
         __syncthreads();
+        auto updateX = [&](int from, int step) {
+            for (int i = from; i < have2; i += step) {
+                double2 xv = reinterpret_cast<double2*>(sx)[i];
+                const double2 pv = reinterpret_cast<double2*>(sp)[i];
+                xv.x = fma(alpha, pv.x, xv.x);
+                xv.y = fma(alpha, pv.y, xv.y);
+                reinterpret_cast<double2*>(sx)[i] = xv;
+            }
+        };
         if (wid < 2) {
             double s = threads_sum(part, min(nw, kVecThreads / 32), lane, 16);
             s = __shfl_sync(0xffffffffu, s, 16 * wid);
@@ -403,13 +412,7 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
             }
         } else {
             // x += alpha p while the sums are on their way
-            for (int i = tid; i < have2; i += nt) {
-                double2 xv = reinterpret_cast<double2*>(sx)[i];
-                const double2 pv = reinterpret_cast<double2*>(sp)[i];
-                xv.x = fma(alpha, pv.x, xv.x);
-                xv.y = fma(alpha, pv.y, xv.y);
-                reinterpret_cast<double2*>(sx)[i] = xv;
-            }
+            updateX(tid - 64, nt - 64);
         }
         if (__syncthreads_or(!ok)) {
             ok = false;
@@ -430,29 +433,24 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
                 st->done = 1u;
             }
         }
+        if (nt == 64) updateX(tid, nt);  // no third warp
+        if (!go) break;
         // ---- p = z + beta p ----
         for (int i = tid; i < have2; i += nt) {
             double2 pv = reinterpret_cast<double2*>(sp)[i];
-            if (wid < 2) {
-                double2 xv = reinterpret_cast<double2*>(sx)[i];
-                xv.x = fma(alpha, pv.x, xv.x);
-                xv.y = fma(alpha, pv.y, xv.y);
-                reinterpret_cast<double2*>(sx)[i] = xv;
-            }
-            if (go) {
-                const double2 zv = reinterpret_cast<double2*>(sz)[i];
-                pv.x = fma(beta, pv.x, zv.x);
-                pv.y = fma(beta, pv.y, zv.y);
-                reinterpret_cast<double2*>(sp)[i] = pv;
-                p2[i] = pv;
-            }
+            const double2 zv = reinterpret_cast<double2*>(sz)[i];
+            pv.x = fma(beta, pv.x, zv.x);
+            pv.y = fma(beta, pv.y, zv.y);
+            reinterpret_cast<double2*>(sp)[i] = pv;
+            p2[i] = pv;
         }
-        if (!go) break;
         __syncthreads();
-        start();
         if (tid == 0) {
             fence_gpu();
             arrive(a.counters + 96);
+        }
+        start();  // after the arrival, which the other CTAs wait for
+        if (tid == 0) {
             ok = wait_count(a.counters + 96, target);
             fence_gpu();
         }
