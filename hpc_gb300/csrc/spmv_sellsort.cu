@@ -18,6 +18,18 @@
 // permutation only decides which lane computes which row; y is written back
 // at the original row index.
 //
+// Hubs: what bounds the kernel are the gathers of x, one L2 sector each (random
+// columns: the SMs fetch at most 0.3 T sectors/s, whatever the number of loads in
+// flight; 2M rows of the Zipf system, 70 M entries, 345 us).  In a symmetric matrix
+// the columns of long rows are gathered most: the first 16,384 of the order take
+// 28 % of the gathers at 2M rows, 39 % at 300,000.  Scattered over x each would hold
+// a whole L1 line; a small kernel copies them side by side (their columns are
+// stored as ~place), and their lines stay in L1.  us without / with: 60,000 rows
+// 55 / 43, 300,007 101 / 76, 1M 204 / 172, 2M 342 / 322.  4,096 to 65,536 hubs differ
+// by 2 %; keeping them in shared memory leaves too few warps, and L1 eviction
+// hints (hubs last, others not at all) were better below 500,000 rows only (71 at
+// 300,007, 375 at 2M: two loads per gather, 128 registers).
+//
 // Work items, in warp-stride order: the long rows (one warp each), then the
 // slices (one lane per row).  kCgDot / kResidual reduce through the same
 // last-block-done grid sum as the other SpMV kernels.
@@ -47,6 +59,12 @@ struct SortAcc<float> {
 };
 
 __device__ __forceinline__ int sort_bin(int len) { return len > kLongRow ? 0 : 1 + (kLongRow - len); }
+
+// x[c], or for c < 0 the copy of hub column ~c.
+template <typename VT, bool HUB>
+__device__ __forceinline__ VT gather(const VT* x, const VT* hubX, int c) {
+    return __ldg(HUB && c < 0 ? hubX + ~c : x + c);
+}
 
 int grid_of(int64_t work, int threads) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((work + threads - 1) / threads, device_sm_count() * 32));
@@ -128,12 +146,48 @@ __global__ void ss_fill_kernel(int n, int nLong, int nSlices, const int* __restr
     }
 }
 
-template <typename VT, int U>
-__global__ void __launch_bounds__(kSortThreads) spmv_sellsort_kernel(
+// Entries of the first nHubs rows of the order (one CTA).
+__global__ void __launch_bounds__(1024) ss_hub_entries_kernel(int nHubs, const int* __restrict__ sorted,
+                                                              const int* __restrict__ rowptr, int* total) {
+    __shared__ int sum;
+    if (threadIdx.x == 0) sum = 0;
+    __syncthreads();
+    int mine = 0;
+    for (int i = threadIdx.x; i < nHubs; i += blockDim.x) mine += rowptr[sorted[i] + 1] - rowptr[sorted[i]];
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&sum, mine);
+    __syncthreads();
+    if (threadIdx.x == 0) *total = sum;
+}
+
+// hubOf[row]: its place if it is one of the first nHubs of the order (else as set before).
+__global__ void ss_hub_index_kernel(int nHubs, const int* __restrict__ sorted, int* __restrict__ hubOf) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nHubs; i += gridDim.x * blockDim.x) hubOf[sorted[i]] = i;
+}
+
+__global__ void ss_recode_kernel(int64_t nnz, const int* __restrict__ col, const int* __restrict__ hubOf,
+                                 int* __restrict__ out) {
+    for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < nnz; j += (int64_t)gridDim.x * blockDim.x) {
+        const int c = col[j], h = __ldg(&hubOf[c]);
+        out[j] = h >= 0 ? ~h : c;
+    }
+}
+
+template <typename VT>
+__global__ void ss_hub_x_kernel(int nHubs, const int* __restrict__ sorted, const VT* __restrict__ x,
+                                VT* __restrict__ hubX, const uint32_t* doneFlag) {
+    if (doneFlag && *(volatile const uint32_t*)doneFlag) return;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nHubs) hubX[i] = x[sorted[i]];
+}
+
+template <typename VT, int U, bool HUB>
+__global__ void __launch_bounds__(kSortThreads, HUB ? 5 : 6) spmv_sellsort_kernel(
     int n, int nLong, int nSlices, const int* __restrict__ sorted, const int* __restrict__ sliceOff,
     const int* __restrict__ scol, const VT* __restrict__ sval, const int* __restrict__ rowptr,
     const int* __restrict__ col, const VT* __restrict__ val, const VT* __restrict__ x, VT* __restrict__ y,
-    const VT* __restrict__ b, CgState* state, double* partials, int mode, const uint32_t* doneFlag) {
+    const VT* __restrict__ b, const VT* __restrict__ hubX, CgState* state, double* partials, int mode,
+    const uint32_t* doneFlag) {
     typedef typename SortAcc<VT>::type AccT;
     if (doneFlag && *(volatile const uint32_t*)doneFlag) return;
     const int lane = threadIdx.x & 31;
@@ -148,6 +202,7 @@ __global__ void __launch_bounds__(kSortThreads) spmv_sellsort_kernel(
             row = sorted[w];
             const int j0 = rowptr[row], j1 = rowptr[row + 1];
             int j = j0 + lane;
+#pragma unroll 1
             for (; j + 32 * (U - 1) < j1; j += 32 * U) {
                 VT v[U];
                 int c[U];
@@ -157,9 +212,9 @@ __global__ void __launch_bounds__(kSortThreads) spmv_sellsort_kernel(
                     c[u] = __ldcs(&col[j + 32 * u]);
                 }
 #pragma unroll
-                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)__ldg(&x[c[u]]), acc);
+                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
             }
-            for (; j < j1; j += 32) acc = fma((AccT)__ldcs(&val[j]), (AccT)__ldg(&x[__ldcs(&col[j])]), acc);
+            for (; j < j1; j += 32) acc = fma((AccT)__ldcs(&val[j]), (AccT)gather<VT, HUB>(x, hubX, __ldcs(&col[j])), acc);
             acc = warp_sum(acc);
             if (lane != 0) continue;
         } else {
@@ -172,6 +227,7 @@ __global__ void __launch_bounds__(kSortThreads) spmv_sellsort_kernel(
             const VT* vp = sval + off + lane;
             const int* cp = scol + off + lane;
             int j = 0;
+#pragma unroll 1
             for (; j + U <= len; j += U) {
                 VT v[U];
                 int c[U];
@@ -181,9 +237,9 @@ __global__ void __launch_bounds__(kSortThreads) spmv_sellsort_kernel(
                     c[u] = __ldcs(cp + (j + u) * 32);
                 }
 #pragma unroll
-                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)__ldg(&x[c[u]]), acc);
+                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
             }
-            for (; j < len; ++j) acc = fma((AccT)__ldcs(vp + j * 32), (AccT)__ldg(&x[__ldcs(cp + j * 32)]), acc);
+            for (; j < len; ++j) acc = fma((AccT)__ldcs(vp + j * 32), (AccT)gather<VT, HUB>(x, hubX, __ldcs(cp + j * 32)), acc);
             if (row < 0) continue;
         }
         if (mode == kSpmvResidual) {
@@ -270,10 +326,10 @@ cudaError_t sellsort_fill(cudaStream_t st, int n, int nLong, const int* rowptr, 
 }
 
 namespace {
-template <typename VT, int U>
+template <typename VT, int U, bool HUB>
 int ss_bps() {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmv_sellsort_kernel<VT, U>, kSortThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmv_sellsort_kernel<VT, U, HUB>, kSortThreads, 0) !=
         cudaSuccess)
         return 0;
     return nb;
@@ -281,29 +337,53 @@ int ss_bps() {
 }  // namespace
 
 template <typename VT>
-int sellsort_grid(int cfg, int n, int nLong, int numSms) {
-    const int bps = sellsort_config_unroll(cfg) == 4 ? ss_bps<VT, 4>() : ss_bps<VT, 8>();
+int sellsort_grid(int cfg, int n, int nLong, int nHubs, int numSms) {
+    const int bps = sellsort_config_unroll(cfg) == 4 ? (nHubs > 0 ? ss_bps<VT, 4, true>() : ss_bps<VT, 4, false>())
+                                                     : (nHubs > 0 ? ss_bps<VT, 8, true>() : ss_bps<VT, 8, false>());
     if (bps <= 0) return 0;
     const int items = nLong + (n - nLong + 31) / 32;
     const int need = (items + kSortThreads / 32 - 1) / (kSortThreads / 32);
     return std::max(1, std::min(need, bps * numSms));
 }
 
+cudaError_t sellsort_hub_entries(cudaStream_t st, int nHubs, const int* sorted, const int* rowptr, int* scratch,
+                                 int* entries) {
+    ss_hub_entries_kernel<<<1, 1024, 0, st>>>(nHubs, sorted, rowptr, scratch);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(entries, scratch, sizeof(int), cudaMemcpyDeviceToHost, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+
+cudaError_t sellsort_recode(cudaStream_t st, int n, int64_t nnz, int nHubs, const int* sorted, const int* col, int* hubOf,
+                            int* out) {
+    const cudaError_t e = cudaMemsetAsync(hubOf, 0xff, sizeof(int) * (size_t)n, st);
+    if (e != cudaSuccess) return e;
+    ss_hub_index_kernel<<<grid_of(nHubs, 256), 256, 0, st>>>(nHubs, sorted, hubOf);
+    ss_recode_kernel<<<grid_of(nnz, 256), 256, 0, st>>>(nnz, col, hubOf, out);
+    return cudaGetLastError();
+}
+
 template <typename VT>
 cudaError_t spmv_sellsort_launch(int cfg, int grid, cudaStream_t st, int n, int nLong, const int* sorted,
                                  const int* sliceOff, const int* scol, const VT* sval, const int* rowptr,
-                                 const int* col, const VT* val, const VT* x, VT* y, const VT* b, CgState* state,
-                                 double* partials, int mode, const uint32_t* doneFlag) {
+                                 const int* col, const VT* val, const VT* x, VT* y, const VT* b, int nHubs, VT* hubX,
+                                 CgState* state, double* partials, int mode, const uint32_t* doneFlag) {
     if (n <= 0) return cudaSuccess;
     const int nSlices = (n - nLong + 31) / 32;
-    if (sellsort_config_unroll(cfg) == 4)
-        spmv_sellsort_kernel<VT, 4><<<grid, kSortThreads, 0, st>>>(n, nLong, nSlices, sorted, sliceOff, scol, sval,
-                                                                   rowptr, col, val, x, y, b, state, partials, mode,
-                                                                   doneFlag);
+    if (nHubs > 0) ss_hub_x_kernel<VT><<<(nHubs + 127) / 128, 128, 0, st>>>(nHubs, sorted, x, hubX, doneFlag);
+    auto go = [&](auto kernel) {
+        kernel<<<grid, kSortThreads, 0, st>>>(n, nLong, nSlices, sorted, sliceOff, scol, sval, rowptr, col, val, x, y,
+                                              b, hubX, state, partials, mode, doneFlag);
+    };
+    if (sellsort_config_unroll(cfg) == 4) {
+        if (nHubs > 0)
+            go(spmv_sellsort_kernel<VT, 4, true>);
+        else
+            go(spmv_sellsort_kernel<VT, 4, false>);
+    } else if (nHubs > 0)
+        go(spmv_sellsort_kernel<VT, 8, true>);
     else
-        spmv_sellsort_kernel<VT, 8><<<grid, kSortThreads, 0, st>>>(n, nLong, nSlices, sorted, sliceOff, scol, sval,
-                                                                   rowptr, col, val, x, y, b, state, partials, mode,
-                                                                   doneFlag);
+        go(spmv_sellsort_kernel<VT, 8, false>);
     return cudaGetLastError();
 }
 
@@ -311,14 +391,15 @@ template cudaError_t sellsort_fill<double>(cudaStream_t, int, int, const int*, c
                                            const int*, int*, double*);
 template cudaError_t sellsort_fill<float>(cudaStream_t, int, int, const int*, const int*, const double*, const int*,
                                           const int*, int*, float*);
-template int sellsort_grid<double>(int, int, int, int);
-template int sellsort_grid<float>(int, int, int, int);
+template int sellsort_grid<double>(int, int, int, int, int);
+template int sellsort_grid<float>(int, int, int, int, int);
 template cudaError_t spmv_sellsort_launch<double>(int, int, cudaStream_t, int, int, const int*, const int*,
                                                   const int*, const double*, const int*, const int*, const double*,
-                                                  const double*, double*, const double*, CgState*, double*, int,
-                                                  const uint32_t*);
+                                                  const double*, double*, const double*, int, double*, CgState*,
+                                                  double*, int, const uint32_t*);
 template cudaError_t spmv_sellsort_launch<float>(int, int, cudaStream_t, int, int, const int*, const int*, const int*,
                                                  const float*, const int*, const int*, const float*, const float*,
-                                                 float*, const float*, CgState*, double*, int, const uint32_t*);
+                                                 float*, const float*, int, float*, CgState*, double*, int,
+                                                 const uint32_t*);
 
 }  // namespace xjpcg

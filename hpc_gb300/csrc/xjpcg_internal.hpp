@@ -122,12 +122,19 @@ template <typename VT>
 cudaError_t sellsort_fill(cudaStream_t st, int n, int nLong, const int* rowptr, const int* col, const double* val,
                           const int* sorted, const int* sliceOff, int* scol, VT* sval);
 template <typename VT>
-int sellsort_grid(int cfg, int n, int nLong, int numSms);
+int sellsort_grid(int cfg, int n, int nLong, int nHubs, int numSms);
+// *entries of the first nHubs rows of the order (scratch: one int).
+cudaError_t sellsort_hub_entries(cudaStream_t st, int nHubs, const int* sorted, const int* rowptr, int* scratch,
+                                 int* entries);
+// out (nnz ints): col with those rows' columns as ~place; hubOf: n ints.
+cudaError_t sellsort_recode(cudaStream_t st, int n, int64_t nnz, int nHubs, const int* sorted, const int* col, int* hubOf,
+                            int* out);
+// nHubs > 0: scol and col are recoded columns, hubX has room for nHubs values.
 template <typename VT>
 cudaError_t spmv_sellsort_launch(int cfg, int grid, cudaStream_t st, int n, int nLong, const int* sorted,
                                  const int* sliceOff, const int* scol, const VT* sval, const int* rowptr,
-                                 const int* col, const VT* val, const VT* x, VT* y, const VT* b, CgState* state,
-                                 double* partials, int mode, const uint32_t* doneFlag);
+                                 const int* col, const VT* val, const VT* x, VT* y, const VT* b, int nHubs, VT* hubX,
+                                 CgState* state, double* partials, int mode, const uint32_t* doneFlag);
 
 // ---- merge-path SpMV (spmv_merge.cu) ----
 // Scratch per matrix: tileRow[ntiles + 1] ints (merge_partition), carryRow[ntiles] ints, carryVal[ntiles] accumulators

@@ -1,0 +1,51 @@
+"""The length-sorted SpMV with hub columns: x at the columns of the longest rows
+is read from a compact copy.  Against long-double row sums, on both sides of the
+size from which the copy is used."""
+import os
+
+import numpy as np
+import pytest
+
+import hpc_gb300 as X
+from hpc_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FROM = 2 * 16384  # rows above which hubs are used
+
+
+@pytest.mark.parametrize("n", [FROM, FROM + 1, 50001])
+def test_spmv_and_solves_with_hub_columns(gpu_lib, n):
+    s = W.zipf_spd(n, hi=1500, seed=n)
+    rows, cols, vals = s.coo()
+    rng = np.random.default_rng(n)
+    env = {"XJPCG_SPMV_LANES": "-4", "XJPCG_GUARD_BYTES": "4096"}
+    os.environ.update(env)
+    try:
+        with X.JPCG() as h:
+            r = h.coo_solve(n, rows, cols, vals, s.diag, s.b, 3000, 1e-10)
+            assert r.status == X.SUCCESS and h.info().spmvLayout == 4
+            v = vals
+            for step in range(2):  # the second with new values
+                x = rng.uniform(-1.0, 1.0, n)
+                y = h.spmv(x)
+                prod = v.astype(np.longdouble) * x[cols]
+                want = np.add.reduceat(prod, s.rowptr[:-1])
+                size = np.add.reduceat(np.abs(prod), s.rowptr[:-1])
+                # every product and sum of a row rounds once
+                assert np.all(np.abs(y - want) <= (np.diff(s.rowptr) + 1) * 2.0**-53 * size)
+                x[cols[s.rowptr[np.argmax(np.diff(s.rowptr))]]] = np.nan
+                bad = np.zeros(n, bool)
+                bad[rows[np.isnan(x[cols])]] = True
+                assert np.array_equal(np.isnan(h.spmv(x)), bad)
+                v = 1.5 * v
+                r = h.coo_solve(n, None, None, v, 1.5 * s.diag, s.b, 3000, 1e-10, mode=X.MODE_KEEP_NZ_LAYOUT)
+                assert r.status == X.SUCCESS
+            m = h.mixed_solve(s.b, 1.5 * s.diag, 3000, 1e-10)
+            assert m.status == X.SUCCESS
+            # converged to 1e-10 each, on a matrix scaled to a condition number of about 1
+            assert np.linalg.norm((m.x - r.x) * np.sqrt(s.diag)) <= 1e-8 * np.linalg.norm(r.x * np.sqrt(s.diag))
+            assert h.check_guards()[1] == 0
+    finally:
+        for k in env:
+            os.environ.pop(k, None)
