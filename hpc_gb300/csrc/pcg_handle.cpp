@@ -500,6 +500,10 @@ bool PcgHandle::isSell(int cfg) const {
 
 bool PcgHandle::isSellNarrow(int cfg) const { return isSell(cfg) && sell_config_narrow(cfg - spmv_num_configs()); }
 
+int PcgHandle::sortedHubs(int cfg) const {
+    return sellsort_config_unroll(cfg - sortedCfg0()) == 8 ? m_ssHubs : 0;
+}
+
 bool PcgHandle::isSorted(int cfg) const { return cfg >= sortedCfg0() && cfg < mergeCfg(); }
 
 bool PcgHandle::isPat(int cfg) const { return cfg >= patCfg0() && cfg < sortedCfg0(); }
@@ -588,8 +592,9 @@ bool PcgHandle::ensureSorted() {
         return false;
     }
     // Hub columns pay where x is larger than an L1 and they take a fifth of the
-    // gathers (28 % at 2M rows of the Zipf system: 6 % faster, 39 % at 300,007: 25 %;
-    // the copy of their x costs a launch, 2.5 us).
+    // gathers (39 % at 300,007 rows of the Zipf system: 11 % faster than the unroll of
+    // 4 without; 28 % at 2M rows: 5 % slower to 3 % faster, which the tuner settles; the
+    // copy of their x costs a launch, 2.5 us).
     m_ssHubs = 0;
     constexpr int kHubs = 16384;
     if (n > 2 * kHubs) {
@@ -607,12 +612,18 @@ bool PcgHandle::ensureSorted() {
             m_ssHubs = kHubs;
         }
     }
-    const int* const col = m_ssHubs > 0 ? m_ssHubCol.as<int>() : m_col.as<int>();
     alloc(m_ssCol, sizeof(int) * ((size_t)total + 32), "sorted sliced columns");
     alloc(m_ssVal, sizeof(double) * ((size_t)total + 32), "sorted sliced values");
-    check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), col, m_val.as<double>(),
+    check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), m_col.as<int>(), m_val.as<double>(),
                                 m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssCol.as<int>(), m_ssVal.as<double>()),
           "sorted sliced fill");
+    if (m_ssHubs > 0) {
+        alloc(m_ssHubScol, sizeof(int) * ((size_t)total + 32), "recoded sliced columns");
+        check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), m_ssHubCol.as<int>(), m_val.as<double>(),
+                                    m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssHubScol.as<int>(),
+                                    m_ssVal.as<double>()),
+              "sorted sliced fill");
+    }
     m_ssLong = nLong;
     m_ssTotal = total;
     m_ssState = 1;
@@ -637,7 +648,7 @@ int PcgHandle::spmvGrid64(int cfg) {
         return merge_tiles((int)m_n, (int64_t)m_nnz);
     }
     if (isSorted(cfg))
-        return ensureSorted() ? sellsort_grid<double>(cfg - sortedCfg0(), (int)m_n, m_ssLong, m_ssHubs, m_numSms) : 0;
+        return ensureSorted() ? sellsort_grid<double>(cfg - sortedCfg0(), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
     if (isPat(cfg)) return ensurePat() ? sellpat_grid<double>(cfg - patCfg0(), (int)m_n, m_numSms) : 0;
     if (!isSell(cfg)) return spmv_grid<double>(cfg, (int)m_n, m_numSms);
     if (!ensureSell() || (isSellNarrow(cfg) && !m_sellNarrow)) return 0;
@@ -650,7 +661,7 @@ int PcgHandle::spmvGrid32(int cfg) {
         return merge_tiles((int)m_n, (int64_t)m_nnz);
     }
     if (isSorted(cfg))
-        return ensureSorted() ? sellsort_grid<float>(cfg - sortedCfg0(), (int)m_n, m_ssLong, m_ssHubs, m_numSms) : 0;
+        return ensureSorted() ? sellsort_grid<float>(cfg - sortedCfg0(), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
     if (isPat(cfg)) return ensurePat() ? sellpat_grid<float>(cfg - patCfg0(), (int)m_n, m_numSms) : 0;
     if (!isSell(cfg)) return spmv_grid<float>(cfg, (int)m_n, m_numSms);
     if (!ensureSell() || (isSellNarrow(cfg) && !m_sellNarrow)) return 0;
@@ -679,11 +690,11 @@ cudaError_t PcgHandle::spmv64(int cfg, int grid, const double* x, double* y, con
                                            m_psGenOff.as<int>(), m_psPat.as<int>(), m_psGcol.as<int>(),
                                            m_psVal.as<double>(), x, y, b, st, part, mode, done);
     if (isSorted(cfg))
-        return spmv_sellsort_launch<double>(cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong,
-                                            m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssCol.as<int>(),
-                                            m_ssVal.as<double>(), m_rowptr.as<int>(),
-                                            m_ssHubs > 0 ? m_ssHubCol.as<int>() : m_col.as<int>(), m_val.as<double>(),
-                                            x, y, b, m_ssHubs, m_ssHubX.as<double>(), st, part, mode, done);
+        return spmv_sellsort_launch<double>(
+            cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
+            (sortedHubs(cfg) > 0 ? m_ssHubScol : m_ssCol).as<int>(), m_ssVal.as<double>(), m_rowptr.as<int>(),
+            (sortedHubs(cfg) > 0 ? m_ssHubCol : m_col).as<int>(), m_val.as<double>(), x, y, b, sortedHubs(cfg),
+            m_ssHubX.as<double>(), st, part, mode, done);
     if (!isSell(cfg))
         return spmv_launch<double>(cfg, grid, m_stream, (int)m_n, m_rowptr.as<int>(), m_col.as<int>(),
                                    m_val.as<double>(), x, y, b, st, part, mode, done);
@@ -709,11 +720,11 @@ cudaError_t PcgHandle::spmv32(int cfg, int grid, const float* x, float* y, const
                                           m_psGenOff.as<int>(), m_psPat.as<int>(), m_psGcol.as<int>(),
                                           m_psVal32.as<float>(), x, y, b, st, part, mode, done);
     if (isSorted(cfg))
-        return spmv_sellsort_launch<float>(cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong,
-                                           m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssCol.as<int>(),
-                                           m_ssVal32.as<float>(), m_rowptr.as<int>(),
-                                           m_ssHubs > 0 ? m_ssHubCol.as<int>() : m_col.as<int>(), m_val32.as<float>(),
-                                           x, y, b, m_ssHubs, m_ssHubX.as<float>(), st, part, mode, done);
+        return spmv_sellsort_launch<float>(
+            cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
+            (sortedHubs(cfg) > 0 ? m_ssHubScol : m_ssCol).as<int>(), m_ssVal32.as<float>(), m_rowptr.as<int>(),
+            (sortedHubs(cfg) > 0 ? m_ssHubCol : m_col).as<int>(), m_val32.as<float>(), x, y, b, sortedHubs(cfg),
+            m_ssHubX.as<float>(), st, part, mode, done);
     if (!isSell(cfg))
         return spmv_launch<float>(cfg, grid, m_stream, (int)m_n, m_rowptr.as<int>(), m_col.as<int>(),
                                   m_val32.as<float>(), x, y, b, st, part, mode, done);

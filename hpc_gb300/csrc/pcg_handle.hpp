@@ -264,8 +264,9 @@ class PcgHandle {
     int m_ssState = 0;  // 0 not built, 1 built, 2 not offered
     int m_ssLong = 0;
     int64_t m_ssTotal = 0;
-    DevBuf m_ssHubOf, m_ssHubCol, m_ssHubX;
-    int m_ssHubs = 0;  // columns whose x the kernels keep in L1
+    DevBuf m_ssHubOf, m_ssHubCol, m_ssHubScol, m_ssHubX;
+    int m_ssHubs = 0;  // columns whose x the unroll of 8 reads from a compact copy
+    int sortedHubs(int cfg) const;
     bool m_ss32Valid = false;
     int m_sellState = 0;  // 0 not built, 1 built, 2 rejected (too much padding)
     DevBuf m_mergeRow, m_mergeVal, m_mergePart;  // merge-path carries and partials

@@ -24,11 +24,15 @@
 // the columns of long rows are gathered most: the first 16,384 of the order take
 // 28 % of the gathers at 2M rows, 39 % at 300,000.  Scattered over x each would hold
 // a whole L1 line; a small kernel copies them side by side (their columns are
-// stored as ~place), and their lines stay in L1.  us without / with: 60,000 rows
-// 55 / 43, 300,007 101 / 76, 1M 204 / 172, 2M 342 / 322.  4,096 to 65,536 hubs differ
-// by 2 %; keeping them in shared memory leaves too few warps, and L1 eviction
-// hints (hubs last, others not at all) were better below 500,000 rows only (71 at
-// 300,007, 375 at 2M: two loads per gather, 128 registers).
+// stored as ~place), and their lines stay in L1.  The unroll of 8 takes hubs, that
+// of 4 (the faster one without) never, so the tuner decides.  us, unroll 4 / unroll
+// 8 with hubs: 60,000 rows 43.5 / 44.6, 300,007 84.5 / 75.4, 1M 175 / 170, 2M 326 -
+// 333 / 315 - 342.  4,096 to 65,536 hubs differ by 2 %; keeping them in shared memory
+// leaves too few warps, and L1 eviction hints (hubs last, others not at all) were
+// better below 500,000 rows only (71 at 300,007, 375 at 2M: two loads per gather,
+// 128 registers).
+// Neither loop over a row's steps is unrolled further: left to the compiler, the
+// unroll of 4 took 55, 101, 204 and 342 us.
 //
 // Work items, in warp-stride order: the long rows (one warp each), then the
 // slices (one lane per row).  kCgDot / kResidual reduce through the same
@@ -338,7 +342,7 @@ int ss_bps() {
 
 template <typename VT>
 int sellsort_grid(int cfg, int n, int nLong, int nHubs, int numSms) {
-    const int bps = sellsort_config_unroll(cfg) == 4 ? (nHubs > 0 ? ss_bps<VT, 4, true>() : ss_bps<VT, 4, false>())
+    const int bps = sellsort_config_unroll(cfg) == 4 ? ss_bps<VT, 4, false>()
                                                      : (nHubs > 0 ? ss_bps<VT, 8, true>() : ss_bps<VT, 8, false>());
     if (bps <= 0) return 0;
     const int items = nLong + (n - nLong + 31) / 32;
@@ -370,17 +374,15 @@ cudaError_t spmv_sellsort_launch(int cfg, int grid, cudaStream_t st, int n, int 
                                  CgState* state, double* partials, int mode, const uint32_t* doneFlag) {
     if (n <= 0) return cudaSuccess;
     const int nSlices = (n - nLong + 31) / 32;
+    if (sellsort_config_unroll(cfg) == 4) nHubs = 0;
     if (nHubs > 0) ss_hub_x_kernel<VT><<<(nHubs + 127) / 128, 128, 0, st>>>(nHubs, sorted, x, hubX, doneFlag);
     auto go = [&](auto kernel) {
         kernel<<<grid, kSortThreads, 0, st>>>(n, nLong, nSlices, sorted, sliceOff, scol, sval, rowptr, col, val, x, y,
                                               b, hubX, state, partials, mode, doneFlag);
     };
-    if (sellsort_config_unroll(cfg) == 4) {
-        if (nHubs > 0)
-            go(spmv_sellsort_kernel<VT, 4, true>);
-        else
-            go(spmv_sellsort_kernel<VT, 4, false>);
-    } else if (nHubs > 0)
+    if (sellsort_config_unroll(cfg) == 4)
+        go(spmv_sellsort_kernel<VT, 4, false>);
+    else if (nHubs > 0)
         go(spmv_sellsort_kernel<VT, 8, true>);
     else
         go(spmv_sellsort_kernel<VT, 8, false>);
