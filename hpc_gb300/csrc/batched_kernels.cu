@@ -767,7 +767,9 @@ __device__ __forceinline__ void fp64_system(const BatchArgs& a, int sys, double*
 }
 
 // Next system of the team (one cluster), or -1: its first CTA asks the queue and
-// tells the others.  A team's last barrier of a system separates two calls.
+// tells the others.  A team's last barrier of a system separates two calls; before
+// the first call the kernel runs one, as a CTA's shared memory may be written by
+// others only once that CTA runs.
 __device__ __forceinline__ int next_team_system(const BatchArgs& a) {
     __shared__ int s_t;
     if (blockIdx.x % (unsigned)a.teamCtas == 0 && threadIdx.x < 32) {
@@ -790,8 +792,10 @@ __global__ void __launch_bounds__(NT, (1024 / NT) > 0 ? 1024 / NT : 1) batched_f
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sPat[kBatchPatMax + 1];
     double* pS = reinterpret_cast<double*>(smem);
-    if (TEAMS)
+    if (TEAMS) {
+        team_barrier<true>();
         for (int sys; (sys = next_team_system(a)) >= 0;) fp64_system<NT, G, SL, true>(a, sys, pS, sPat);
+    }
     for (int sys; (sys = next_system(a)) >= 0;) fp64_system<NT, G, SL, false>(a, sys, pS, sPat);
 }
 
@@ -1014,8 +1018,10 @@ __global__ void __launch_bounds__(NT, (TEAMS ? 1024 : 1536) / NT > 0 ? (TEAMS ? 
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ int sPat[kBatchPatMax + 1];
     float* pS = reinterpret_cast<float*>(smem);
-    if (TEAMS)
+    if (TEAMS) {
+        team_barrier<true>();
         for (int sys; (sys = next_team_system(a)) >= 0;) mixed_system<NT, G, SL, true>(a, sys, pS, sPat);
+    }
     for (int sys; (sys = next_system(a)) >= 0;) mixed_system<NT, G, SL, false>(a, sys, pS, sPat);
 }
 
