@@ -1031,6 +1031,7 @@ template <int NT, int G, bool SL>
 struct BatchInst {
     static cudaError_t launch(bool mixed, int grid, size_t smem, cudaStream_t st, const BatchArgs& a) {
         if (SL && a.sliceOff == nullptr) return cudaErrorInvalidValue;  // no sliced copy
+        if (!SL && mixed && a.val32 == nullptr) return cudaErrorInvalidValue;  // no FP32 values
         if (mixed) {
             cudaError_t e = cudaFuncSetAttribute(batched_mixed_kernel<NT, G, SL>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

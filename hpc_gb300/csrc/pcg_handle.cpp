@@ -2070,17 +2070,11 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     }
 
     if (!sliced) singles = nsys;  // the team kernels read the sliced copy
-    const bool csr = !sliced || (forced >= 0 && !batch_config_sliced(forced % batch_num_configs()));
-    if (mixed && csr) {  // the CSR kernels read FP32 values
-        alloc(m_bVal32, sizeof(float) * ((size_t)nnz + 4), "batch fp32 values");
-        check(convert_f64_to_f32(m_stream, nnz, in.val, m_bVal32.as<float>()), "fp32 values");
-    }
     BatchLaunch L;
     L.sysRow = m_bSysRow.as<int>();
     L.rowptr = in.rowptr;
     L.col = in.col;
     L.val = in.val;
-    L.val32 = mixed && csr ? m_bVal32.as<float>() : nullptr;
     L.b = in.b;
     L.diag = in.diag;
     L.x = m_bX.as<double>();
@@ -2129,10 +2123,17 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     }
     // 0: no teams, 1: always, -1: where they are faster
     const int teamsEnv = envInt("XJPCG_BATCH_TEAMS", forcedShape ? 0 : -1);
-    const uint64_t key = mixKey(mixKey(mixKey(nsys, (uint64_t)total), (uint64_t)nnz),
+    const uint64_t shape = mixKey(mixKey(mixKey(nsys, (uint64_t)total), (uint64_t)nnz), (uint64_t)maxN);
+    const uint64_t key = mixKey(mixKey(shape, nsys - singles),
                                 (uint64_t)precision + 7 + (sliced ? 1000 : 0) + 10000 * (uint64_t)(teamsEnv + 1));
     // One batch; teams: CTAs per long system, 0 for none.
     auto runOnce = [&](int cfg, int rows, int teams, float* ms) {
+        if (mixed && teams == 0 && !batch_config_sliced(cfg) && L.val32 == nullptr) {
+            // the CSR kernels read FP32 values
+            alloc(m_bVal32, sizeof(float) * ((size_t)nnz + 4), "batch fp32 values");
+            check(convert_f64_to_f32(m_stream, nnz, in.val, m_bVal32.as<float>()), "fp32 values");
+            L.val32 = m_bVal32.as<float>();
+        }
         check(cudaMemsetAsync(m_bQueue.p, 0, 16, m_stream), "memset queue");
         check(cudaEventRecord(m_ev0, m_stream), "event");
         int grid = 0;
@@ -2148,11 +2149,13 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         m_batchGrid = grid;
     };
     const int ncfg = batch_num_configs();
+    BatchPlan plan = m_batchPlan;
     if (forced >= 0 && forced < ncfg * (int)smemRows.size()) {
-        m_batchCfg = forced % ncfg;
-        m_batchSmemRows = smemRows[forced / ncfg];
-        m_batchTeams = teamsEnv == 1 && singles < nsys ? 4 : 0;
-    } else if (m_batchKey != key || m_batchCfg < 0) {
+        // for this call alone: the tuner's plan stands beside it
+        plan.cfg = forced % ncfg;
+        plan.smemRows = smemRows[forced / ncfg];
+        plan.teams = teamsEnv == 1 && singles < nsys ? 4 : 0;
+    } else if (m_batchKey != key || plan.cfg < 0) {
         // The sliced shapes (the CSR ones where there is no sliced copy: on
         // 1,024 systems they took 1.1 to 1.9 times as long), with and without
         // teams.
@@ -2164,9 +2167,9 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
             *told = *told < 0.f ? ms : std::min(*told, ms);
             if (ms < best) {
                 best = ms;
-                m_batchCfg = c;
-                m_batchSmemRows = rows;
-                m_batchTeams = teams;
+                plan.cfg = c;
+                plan.smemRows = rows;
+                plan.teams = teams;
             }
         };
         const bool canTeam = singles < nsys && teamsEnv != 0;
@@ -2185,10 +2188,13 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
             for (int rows : {std::min(maxN, 4096), std::min(maxN, (int)(44 * 1024 / esz))})
                 for (int teams : {2, 4, 8}) consider(c512, rows, teams, &unused);
         }
+        m_batchPlan = plan;
         m_batchKey = key;
     }
     faultPoint("batched launch");
-    runOnce(m_batchCfg, m_batchSmemRows, m_batchTeams, &m_batchMs);
+    runOnce(plan.cfg, plan.smemRows, plan.teams, &m_batchMs);
+    m_batchCfg = plan.cfg;
+    m_batchSmemRows = plan.smemRows;
     return batchResults(nsys, total, x, tol, results, onDevice);
 }
 

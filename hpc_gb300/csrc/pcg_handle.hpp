@@ -327,16 +327,21 @@ class PcgHandle {
     DevBuf m_bsBase, m_bsLen, m_bsOff, m_bsScan, m_bsVal, m_bsVal32, m_bsCol;  // per-system SELL-32 copy
     DevBuf m_bsPatLen, m_bsPatOff;  // its slices' shared column offsets
     DevBuf m_bsMeta, m_bsSysPat;    // slice records, and each system's offsets
-    int m_batchCfg = -1, m_batchSmemRows = 0, m_batchGrid = 0;
+    int m_batchCfg = -1, m_batchSmemRows = 0, m_batchGrid = 0;  // of the last batch of the streaming kernels
+    // The tuner's choice for batches of m_batchKey's kind: kernel shape, rows of p
+    // in shared memory, CTAs per long system (0: one each).
+    struct BatchPlan {
+        int cfg = -1, smemRows = 0, teams = 0;
+    };
+    BatchPlan m_batchPlan;
     uint64_t m_batchKey = 0;
     float m_batchMs = 0.f;
     std::vector<float> m_batchTuneMs;
-    DevBuf m_bWidth;                                     // longest row of each system
+    DevBuf m_bWidth;                                     // of each system: longest row, columns' reach, first entry
     static constexpr int kBatchClasses = 10;             // 1, 2, 4, 8, 16 small CTAs per system, then wide ones
     cudaStream_t m_batchStream[kBatchClasses] = {};      // one per class, created on first use
     cudaEvent_t m_batchFork = nullptr, m_batchJoin[kBatchClasses] = {};
     int m_batchClusterCtas = 0;                          // CTAs of the last cluster batch, 0: the other kernels ran
-    int m_batchTeams = 0;                                // the tuner's choice: CTAs per long system, 0: one each
 
     // graph
     cudaGraphExec_t m_exec = nullptr;
