@@ -35,6 +35,7 @@ constexpr int kBcMaxCtas = 16;
 constexpr int kInfoShared = 1 << 16;  // the slice's rows share their column offsets
 constexpr int kInfoLocal = 1 << 17;   // every column of the slice lies in this CTA
 constexpr uint64_t kBcWaitNs = 2000000000ull;  // 2 s
+constexpr uint32_t kBatchLost = 2;             // status of a system whose CTAs lost one another
 
 __device__ __forceinline__ void bc_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
@@ -241,13 +242,28 @@ __device__ __forceinline__ bool wait_posts(uint64_t* bar, uint32_t parity) {
     }
 }
 
+// A wait that gives up.  Shared memory of a CTA that has left may be neither
+// written nor read, so no CTA leaves by itself: the one whose wait ran out marks
+// all CTAs of the cluster with the number of the cluster's next barrier and goes
+// on, with a sum that means nothing, so that the others get its posts.  After
+// every barrier of the cluster all compare the mark with that barrier's number
+// and leave together, whichever place in the code each came to it from.  The
+// missing post may still be on its way: before it leaves, the marking CTA waits
+// for it once more.
+struct Lost {
+    uint32_t mark, parity;
+    uint64_t* late;
+};
+
 // Threads 0 .. 32 NV - 1 return with the sum of value (their warp) in every
 // lane, the others with nothing; the caller syncs the CTA.  Narrow: one warp
 // adds all threads' parts of a value (an FP64 add of a warp holds the pipe for
-// 16 cycles, whoever needs it).  ok turns false when a wait gives up.
+// 16 cycles, whoever needs it).  next: the number of the cluster's next barrier,
+// counted from 1.  mute: the CTA's post to the first one stays out (a test of the
+// wait's limit).
 template <int NT, typename T, int NV, bool MULTI>
 __device__ __forceinline__ T system_sum(const T (&v)[NV], SumBox<NT, T, NV>& box, int q, int C, uint32_t parity,
-                                        bool& ok) {
+                                        Lost& lost, uint32_t next, bool mute = false) {
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
 #pragma unroll
     for (int i = 0; i < NV; ++i) box.part[i][tid] = v[i];
@@ -260,12 +276,25 @@ __device__ __forceinline__ T system_sum(const T (&v)[NV], SumBox<NT, T, NV>& box
         for (int k = 1; k < NT / 32; ++k) t += box.part[wid][lane + 32 * k];
         t = warp_sum(t);
         if (MULTI) {
-            if (lane < C) post(&box.slots[wid][q], &box.bar, (uint32_t)lane, t);
-            ok = wait_posts(&box.bar, parity);
+            if (lane < C && !(mute && lane == 0)) post(&box.slots[wid][q], &box.bar, (uint32_t)lane, t);
+            if (!wait_posts(&box.bar, parity)) {
+                lost.parity = parity;
+                lost.late = &box.bar;
+                if (lane < C)
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(bc_map(&lost.mark, (uint32_t)lane)), "r"(next)
+                                 : "memory");
+            }
             t = warp_sum(lane < C ? box.slots[wid][lane] : T(0));
         }
     }
     return t;
+}
+
+// The end of a system whose CTAs lost one another.
+__device__ __forceinline__ void end_lost(Lost& lost, BatchResult& res, int q) {
+    if (threadIdx.x != 0) return;
+    if (q == 0) res.status = kBatchLost;
+    if (lost.late != nullptr) wait_posts(lost.late, lost.parity);
 }
 
 template <typename VT>
@@ -294,6 +323,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
     __shared__ SumBox<NT, double, 2> boxB;
     __shared__ double sAlpha, sBeta, sRz, sRr;
     __shared__ int sGo[3];
+    __shared__ Lost lost;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int C = MULTI ? a.ctas : 1, q = MULTI ? (int)(blockIdx.x % (unsigned)C) : 0;
     const int sys = a.order[MULTI ? blockIdx.x / (unsigned)C : blockIdx.x];
@@ -302,6 +332,8 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
     const int rows = max(0, min(s.R, s.n - s.row0));
     if (MULTI) {
         if (tid == 0) {
+            lost.mark = 0;
+            lost.late = nullptr;
             mbar_init(&boxA.bar, 1);
             mbar_init(&boxB.bar, 1);
             mbar_fence_init();
@@ -325,18 +357,17 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
         }
     }
     load_rows<double, NT>(s, a.rowptr + r0, a.col, a.val);
-    bool ok = true;
     {
-        const double t = system_sum<NT, double, 2, MULTI>(w2, boxB, q, C, 0u, ok);
+        const double t = system_sum<NT, double, 2, MULTI>(w2, boxB, q, C, 0u, lost, 1u);
         if (tid == 0) sRr = t;
         if (tid == 32) sRz = t;
     }
-    if (__syncthreads_or(!ok)) return;
+    __syncthreads();
     const double rr0 = sRr;
     const double tols = rr0 * a.tol * a.tol;
     system_sync<MULTI>();
     uint32_t k = 0;
-    bool go = true;
+    bool go = !MULTI || lost.mark != 1u;
     while (go) {
         // Ap = A p, p.Ap
         double pAp[1] = {0.0};
@@ -346,13 +377,14 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
 #pragma unroll
         for (int u = 0; u < K; ++u)
             if (tid + u * NT < rows) pAp[0] = fma(p[u], z[u], pAp[0]);
-        const double pApT = system_sum<NT, double, 1, MULTI>(pAp, boxA, q, C, k & 1u, ok);
+        const double pApT = system_sum<NT, double, 1, MULTI>(pAp, boxA, q, C, k & 1u, lost, k + 2u,
+                                                              MULTI && k == a.muteAt && q == C - 1);
         if (tid == 0) {
             const double al = sRz / pApT;
             sAlpha = al;
             sGo[0] = isfinite(al) ? 1 : 0;
         }
-        if (__syncthreads_or(!ok)) return;
+        __syncthreads();
         const double alpha = sAlpha;
         w2[0] = w2[1] = 0.0;
 #pragma unroll
@@ -363,7 +395,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
                 w2[0] = fma(r[u], r[u], w2[0]);
                 w2[1] = fma(r[u], z[u], w2[1]);
             }
-        const double tB = system_sum<NT, double, 2, MULTI>(w2, boxB, q, C, (k + 1u) & 1u, ok);
+        const double tB = system_sum<NT, double, 2, MULTI>(w2, boxB, q, C, (k + 1u) & 1u, lost, k + 2u);
         if (tid == 0) {
             sRr = tB;
             sGo[1] = isfinite(tB) ? (tB >= tols && k + 1u < a.maxIterP1 ? 1 : 0) : 2;
@@ -378,7 +410,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
 #pragma unroll
         for (int u = 0; u < K; ++u)
             if (tid + u * NT < rows) x[u] = fma(alpha, p[u], x[u]);
-        if (__syncthreads_or(!ok)) return;
+        __syncthreads();
         const bool broken = sGo[0] == 0 || sGo[1] == 2 || sGo[2] == 0;
         go = !broken && sGo[1] == 1;
         const double beta = sBeta;
@@ -399,6 +431,11 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
             o.status = broken ? 1u : 0u;
         }
         system_sync<MULTI>();
+        if (MULTI && lost.mark == k + 1u) break;
+    }
+    if (MULTI && lost.mark == k + 1u) {
+        end_lost(lost, a.res[sys], q);
+        return;
     }
 #pragma unroll
     for (int u = 0; u < K; ++u)
@@ -415,6 +452,7 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
     __shared__ SumBox<NT, float, 2> boxB;
     __shared__ double sQ, sT[2];
     __shared__ float sF[2];
+    __shared__ Lost lost;
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int C = MULTI ? a.ctas : 1, q = MULTI ? (int)(blockIdx.x % (unsigned)C) : 0;
     const int sys = a.order[MULTI ? blockIdx.x / (unsigned)C : blockIdx.x];
@@ -423,6 +461,8 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
     const int rows = max(0, min(s.R, s.n - s.row0));
     if (MULTI) {
         if (tid == 0) {
+            lost.mark = 0;
+            lost.late = nullptr;
             mbar_init(&boxR.bar, 1);
             mbar_init(&boxA.bar, 1);
             mbar_init(&boxB.bar, 1);
@@ -455,21 +495,21 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
     }
     v2[1] = (double)rzA;
     load_rows<float, NT>(s, rp, a.col, a.val);
-    bool ok = true;
     {
-        const double t = system_sum<NT, double, 2, MULTI>(v2, boxR, q, C, 0u, ok);
+        const double t = system_sum<NT, double, 2, MULTI>(v2, boxR, q, C, 0u, lost, 1u);
         if (tid == 0) sT[0] = t;
         if (tid == 32) sT[1] = t;
     }
-    if (__syncthreads_or(!ok)) return;
+    __syncthreads();
     const double bb = sT[0];
     double rz = sT[1];
     const double tols = bb * a.tol * a.tol;
     double rrMax = bb, rrTrue = bb;
     uint32_t k = 0, outer = 0;
-    bool bd = false;
+    bool bd = false, stopped = false;
     system_sync<MULTI>();
-    for (;;) {
+    // barriers of the cluster so far: one here, one per iteration and one per refresh
+    while (!MULTI || lost.mark != k + outer + 1u) {
         // Ap = A p (FP32), p.Ap
         float pAp[1] = {0.f};
 #pragma unroll
@@ -478,9 +518,10 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
 #pragma unroll
         for (int u = 0; u < K; ++u)
             if (tid + u * NT < rows) pAp[0] = fmaf(p[u], z[u], pAp[0]);
-        const float pApT = system_sum<NT, float, 1, MULTI>(pAp, boxA, q, C, k & 1u, ok);
+        const float pApT = system_sum<NT, float, 1, MULTI>(pAp, boxA, q, C, k & 1u, lost, k + outer + 2u,
+                                                            MULTI && k == a.muteAt && q == C - 1);
         if (tid == 0) sQ = rz / (double)pApT;
-        if (__syncthreads_or(!ok)) return;
+        __syncthreads();
         const double alphaD = sQ;
         const float alpha = (float)alphaD;
         float w2[2] = {0.f, 0.f};
@@ -493,13 +534,13 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
                 w2[0] = fmaf(r[u], r[u], w2[0]);
                 w2[1] = fmaf(r[u], z[u], w2[1]);
             }
-        const float tB = system_sum<NT, float, 2, MULTI>(w2, boxB, q, C, k & 1u, ok);
+        const float tB = system_sum<NT, float, 2, MULTI>(w2, boxB, q, C, k & 1u, lost, k + outer + 2u);
         if (tid == 0) sF[0] = tB;
         if (tid == 32) {
             sF[1] = tB;
             sQ = (double)tB / rz;  // beta, unless a refresh is due
         }
-        if (__syncthreads_or(!ok)) return;
+        __syncthreads();
         ++k;
         const double rrN = sF[0], rzN = sF[1];
         if (rrN > rrMax) rrMax = rrN;
@@ -516,6 +557,7 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
                     d[u] = 0.f;
                 }
             system_sync<MULTI>();
+            if (MULTI && lost.mark == k + outer + 1u) break;
             double v3[2] = {0.0, 0.0};
             float rzR = 0.f;
 #pragma unroll
@@ -534,13 +576,13 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
             }
             v3[1] = (double)rzR;
             ++outer;
-            const double t = system_sum<NT, double, 2, MULTI>(v3, boxR, q, C, outer & 1u, ok);
+            const double t = system_sum<NT, double, 2, MULTI>(v3, boxR, q, C, outer & 1u, lost, k + outer + 1u);
             if (tid == 0) sT[0] = t;
             if (tid == 32) {
                 sT[1] = t;
                 sQ = t / rz;
             }
-            if (__syncthreads_or(!ok)) return;
+            __syncthreads();
             rrTrue = sT[0];
             rrMax = rrTrue;
             bool stop = !(rrTrue > tols) || k + 1u >= a.maxIterP1;
@@ -549,7 +591,10 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
                 stop = true;
             }
             rz = sT[1];
-            if (stop) break;
+            if (stop) {
+                stopped = true;
+                break;
+            }
         }
         const float beta = (float)sQ;
 #pragma unroll
@@ -560,15 +605,18 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
             }
         system_sync<MULTI>();
     }
-    if (q == 0 && tid == 0) {
-        BatchResult& o = a.res[sys];
-        o.itersRun = k;
-        o.iters = k;
-        o.outer = outer;
-        o.res = sqrt(rrTrue / bb);
-        o.status = bd ? 1u : 0u;
+    if (stopped) {
+        if (q == 0 && tid == 0) {
+            BatchResult& o = a.res[sys];
+            o.itersRun = k;
+            o.iters = k;
+            o.outer = outer;
+            o.res = sqrt(rrTrue / bb);
+            o.status = bd ? 1u : 0u;
+        }
+        system_sync<MULTI>();  // no CTA leaves while a post to it may be on its way
     }
-    system_sync<MULTI>();  // no CTA leaves while a post to it may be on its way
+    if (MULTI && lost.mark == k + outer + 1u) end_lost(lost, a.res[sys], q);
 }
 
 // ---------------------------------------------------------------------------

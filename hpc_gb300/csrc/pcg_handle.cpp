@@ -168,6 +168,7 @@ void PcgHandle::init(int device) {
     m_forcedCfg = envInt("XJPCG_SPMV_CFG", -1);
     m_faultAlloc = envIs("XJPCG_FAULT", "alloc");
     m_faultLaunch = envIs("XJPCG_FAULT", "launch");
+    m_faultPost = envIs("XJPCG_FAULT", "post");
     m_initDone = true;
 }
 
@@ -1926,6 +1927,7 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
         const double delta = envDouble("XJPCG_RELIABLE_DELTA", 0.01);
         a.delta2 = delta * delta;
     }
+    if (m_faultPost) a.muteAt = 3;
     batchStreams();
     faultPoint("graph launch");
     check(cudaEventRecord(m_ev0, m_stream), "event");

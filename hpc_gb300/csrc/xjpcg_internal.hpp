@@ -274,6 +274,7 @@ struct BatchClusterArgs {
     uint32_t maxIterP1 = 0;
     double tol = 0.0, delta2 = 0.0;
     int ctas = 1;  // CTAs per system: 1 .. 16
+    uint32_t muteAt = ~0u;  // fault injection: the iteration in which the last CTA does not post to the first
 };
 int batch_cluster_rows(bool mixed, bool small);     // most rows of a CTA
 size_t batch_cluster_room(bool mixed, bool small);  // most shared memory of a CTA

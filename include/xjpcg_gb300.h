@@ -59,7 +59,8 @@ typedef struct {
     uint32_t iters;    /* fp64: min(K, maxIter) as xJPCG reports it; mixed: inner iterations */
     uint32_t itersRun; /* iterations executed (fp64: K) */
     uint32_t outer;    /* mixed: refinement sweeps */
-    uint32_t status;   /* 0 = ran to its stop rule, 1 = breakdown (non-finite alpha, beta or r.r) */
+    uint32_t status;   /* 0 = ran to its stop rule, 1 = breakdown (non-finite alpha, beta or r.r),
+                          2 or more = a wait of its kernel ran out (the other fields and x are void) */
     double res;        /* fp64: sqrt(r.r / b.b) of the recursive residual; mixed: true relative residual */
 } XJPCG_GbBatchResult_t;
 

@@ -123,3 +123,24 @@ def test_batched_input_errors_are_found_on_the_device(gpu_lib):
             st, msg = call(r, c)
             assert st == X.INVALID_VALUE and word in msg, msg
         assert call(rp, col)[0] == X.SUCCESS
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_lost_post_ends_its_systems_alone(gpu_lib, precision, monkeypatch):
+    # XJPCG_FAULT=post: in one iteration the last CTA of each cluster does not
+    # post its sum to the first, whose wait then runs out (2 s).  The cluster gives
+    # up as one and its system is reported as failed; systems of one CTA (at most
+    # 128 rows) and the handle itself are as before.
+    monkeypatch.setenv("XJPCG_FAULT", "post")
+    monkeypatch.setenv("XJPCG_GUARD_BYTES", "4096")
+    many = [_stencil((10, 11), k) for k in range(400)] + [_stencil((46, 47), 6), _stencil((25, 26, 27), 10)]
+    with X.JPCG() as h:
+        st, xs, res = h.batch_solve(many, 20000, 1e-10, precision=precision)
+        assert st == X.EXECUTION_FAILED
+        assert h.info().batchSmemRows == 0  # solved from shared memory
+        assert [int(r["status"]) for r in res] == [0] * 400 + [2, 2]
+        _check(many[:8], xs[:8], res[:8], precision)
+        # ended in fewer iterations than the dropped one: nothing is lost
+        st, _, res = h.batch_solve(many[-2:], 1, 1e-10, precision=precision)
+        assert [int(r["status"]) for r in res] == [0, 0]
+        assert h.check_guards()[1] == 0
