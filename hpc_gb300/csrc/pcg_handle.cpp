@@ -1790,8 +1790,9 @@ void PcgHandle::batchStreams() {
 }
 
 // Checks the batch's arrays on the device and leaves them in in.*: the
-// caller's own device arrays (when aligned to their elements), or copies of
-// the host arrays in the handle's buffers.
+// caller's own device arrays (when they lie on the handle's device, aligned to
+// their elements), or copies in the handle's buffers: a kernel cannot count on
+// reaching memory of another device or of the host, a copy engine can.
 void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
                            const double* values, const double* diag, const double* b, bool onDevice, BatchInput& in) {
     // the system offsets are few: checked on the host
@@ -1810,7 +1811,13 @@ void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* 
     check(cudaMemsetAsync(m_bWidth.p, 0, sizeof(int32_t) * 2 * nsys, m_stream), "memset");
     check(cudaMemsetAsync(m_flags.p, 0, sizeof(int), m_stream), "memset");
     auto place = [&](DevBuf& buf, const void* src, size_t elem, size_t count, const char* what) -> const void* {
-        if (onDevice && reinterpret_cast<uintptr_t>(src) % elem == 0) return src;
+        if (onDevice && reinterpret_cast<uintptr_t>(src) % elem == 0) {
+            cudaPointerAttributes at = {};
+            if (cudaPointerGetAttributes(&at, src) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+                at.device == m_device)
+                return src;
+            cudaGetLastError();
+        }
         alloc(buf, elem * (count + 4), what);
         check(cudaMemcpyAsync(buf.p, src, elem * count, onDevice ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                               m_stream),

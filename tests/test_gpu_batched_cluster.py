@@ -144,3 +144,34 @@ def test_a_lost_post_ends_its_systems_alone(gpu_lib, precision, monkeypatch):
         st, _, res = h.batch_solve(many[-2:], 1, 1e-10, precision=precision)
         assert [int(r["status"]) for r in res] == [0, 0]
         assert h.check_guards()[1] == 0
+
+
+@pytest.mark.parametrize("place", ["device", "misaligned", "pinned", "host"])
+def test_batched_arrays_wherever_they_lie(gpu_lib, place):
+    # only arrays of the handle's own device, aligned to their elements, are read
+    # in place; everything else that a copy reaches is copied first (memory of
+    # another device among it, which needs a second one to show)
+    import torch
+    batch = [_stencil((9, 10), 1), _stencil((25, 26), 2), _stencil((9, 10, 11), 3)]
+    off = np.cumsum([0] + [s.nnz for s in batch])
+    sys = np.cumsum([0] + [s.n for s in batch]).astype(np.int32)
+    rp = np.concatenate([[0]] + [s.rowptr[1:] + off[k] for k, s in enumerate(batch)]).astype(np.int32)
+    arrays = [rp] + [np.concatenate([getattr(s, f) for s in batch]) for f in ("col", "val", "diag", "b")]
+
+    def put(a):
+        t = torch.from_numpy(a)
+        if place == "misaligned":
+            raw = torch.zeros(a.nbytes + 1, dtype=torch.uint8, device="cuda")
+            raw[1:] = torch.from_numpy(a.view(np.uint8)).cuda()
+            return raw[1:]
+        return t.cuda() if place == "device" else t.pin_memory() if place == "pinned" else t
+
+    held = [put(a) for a in arrays]
+    first, x = torch.from_numpy(sys).cuda(), torch.zeros(int(sys[-1]), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    with X.JPCG() as h:
+        st = h.lib.xJPCG_gbBatchSolve(h.h, 3, first.data_ptr(), *[t.data_ptr() for t in held], x.data_ptr(), 2000, 1e-10,
+                                      0, None, 1)
+        assert st == X.SUCCESS, h.last_message()
+        _, want, _ = h.batch_solve(batch, 2000, 1e-10)
+    assert np.array_equal(x.cpu().numpy(), np.concatenate(want))
