@@ -697,37 +697,75 @@ size_t batch_cluster_smem(bool mixed, int n, int width, int ctas) {
     return (R * (vt * (1 + (size_t)width) + 2 * (size_t)width) + 4 * ns + 15) / 16 * 16;
 }
 
-cudaError_t batch_cluster_launch(cudaStream_t st, bool mixed, bool small, int systems, size_t smem,
-                                 const BatchClusterArgs& a) {
-    typedef void (*Kernel)(BatchClusterArgs);
-    const bool one = a.ctas == 1;
-    Kernel k;
+namespace {
+typedef void (*ClusterKernel)(BatchClusterArgs);
+
+ClusterKernel cluster_kernel(bool mixed, bool small, bool one) {
     if (small)
-        k = mixed ? (one ? (Kernel)batch_cluster_mixed_kernel<kSmall, kSmallRows, false>
-                         : (Kernel)batch_cluster_mixed_kernel<kSmall, kSmallRows, true>)
-                  : (one ? (Kernel)batch_cluster_fp64_kernel<kSmall, kSmallRows, false>
-                         : (Kernel)batch_cluster_fp64_kernel<kSmall, kSmallRows, true>);
-    else
-        k = mixed ? (one ? (Kernel)batch_cluster_mixed_kernel<kWide32, kWideRows32, false>
-                         : (Kernel)batch_cluster_mixed_kernel<kWide32, kWideRows32, true>)
-                  : (one ? (Kernel)batch_cluster_fp64_kernel<kWide64, kWideRows64, false>
-                         : (Kernel)batch_cluster_fp64_kernel<kWide64, kWideRows64, true>);
+        return mixed ? (one ? (ClusterKernel)batch_cluster_mixed_kernel<kSmall, kSmallRows, false>
+                            : (ClusterKernel)batch_cluster_mixed_kernel<kSmall, kSmallRows, true>)
+                     : (one ? (ClusterKernel)batch_cluster_fp64_kernel<kSmall, kSmallRows, false>
+                            : (ClusterKernel)batch_cluster_fp64_kernel<kSmall, kSmallRows, true>);
+    return mixed ? (one ? (ClusterKernel)batch_cluster_mixed_kernel<kWide32, kWideRows32, false>
+                        : (ClusterKernel)batch_cluster_mixed_kernel<kWide32, kWideRows32, true>)
+                 : (one ? (ClusterKernel)batch_cluster_fp64_kernel<kWide64, kWideRows64, false>
+                        : (ClusterKernel)batch_cluster_fp64_kernel<kWide64, kWideRows64, true>);
+}
+
+cudaError_t cluster_config(ClusterKernel k, bool mixed, bool small, int systems, int ctas, size_t smem,
+                           cudaStream_t st, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr) {
     cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmem);
-    if (e == cudaSuccess && a.ctas > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(systems * a.ctas));
-    cfg.blockDim = dim3((unsigned)(small ? kSmall : (mixed ? kWide32 : kWide64)));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    *cfg = {};
+    cfg->gridDim = dim3((unsigned)(systems * ctas));
+    cfg->blockDim = dim3((unsigned)(small ? kSmall : (mixed ? kWide32 : kWide64)));
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)a.ctas;
+    attr[0].val.clusterDim.x = (unsigned)ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = a.ctas > 1 ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, k, a);
+    cfg->attrs = attr;
+    cfg->numAttrs = ctas > 1 ? 1 : 0;
+    return e;
+}
+}  // namespace
+
+// Asked once per device, kernel and size.
+bool batch_cluster_offered(bool mixed, bool small, int ctas) {
+    if (ctas == 1) return true;
+    constexpr int kMaxDev = 64;
+    static int cache[kMaxDev][2][2][kBcMaxCtas + 1] = {};  // 0 not asked, 1 yes, 2 no
+    int dev = 0;
+    if (ctas > kBcMaxCtas || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) {
+        cudaGetLastError();
+        return false;
+    }
+    int* const known = &cache[dev][mixed][small][ctas];
+    int v = __atomic_load_n(known, __ATOMIC_RELAXED);
+    if (v == 0) {
+        cudaLaunchConfig_t cfg;
+        cudaLaunchAttribute attr[1];
+        const ClusterKernel k = cluster_kernel(mixed, small, false);
+        int clusters = 0;
+        v = cluster_config(k, mixed, small, 1, ctas, batch_cluster_room(mixed, small), nullptr, &cfg, attr) ==
+                        cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, k, &cfg) == cudaSuccess && clusters > 0
+                ? 1
+                : 2;
+        cudaGetLastError();
+        __atomic_store_n(known, v, __ATOMIC_RELAXED);
+    }
+    return v == 1;
+}
+
+cudaError_t batch_cluster_launch(cudaStream_t st, bool mixed, bool small, int systems, size_t smem,
+                                 const BatchClusterArgs& a) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    const ClusterKernel k = cluster_kernel(mixed, small, a.ctas == 1);
+    const cudaError_t e = cluster_config(k, mixed, small, systems, a.ctas, smem, st, &cfg, attr);
+    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, k, a) : e;
 }
 
 }  // namespace xjpcg

@@ -1323,30 +1323,48 @@ static BatchArgs batch_args(const BatchLaunch& L, int smemRows) {
 // ms, fp64 / mixed, one CTA per system against teams of the tuner's size (2 to
 // 8): 1,024 systems 52.9 / 27.4 against 46.3 / 23.9; 2,000 74.5 / 34.5 against
 // 65 / 33; 300 50.5 / 24.0 against 20.2 / 15; 4,096 systems need none.
-cudaError_t batch_team_launch(cudaStream_t st, bool mixed, int ctas, int numSms, int smemRows, const BatchLaunch& L,
-                              int nteam, int* gridOut) {
-    if (L.sliceOff == nullptr || ctas < 2 || ctas > kTeamMax) return cudaErrorInvalidValue;
-    BatchArgs a = batch_args(L, smemRows);
-    a.nteam = nteam;
-    a.teamCtas = ctas;
+static cudaError_t team_config(bool mixed, int ctas, int smemRows, cudaStream_t st, cudaLaunchConfig_t* cfg,
+                               cudaLaunchAttribute* attr, void (**kernel)(BatchArgs), int* clusters) {
     typedef void (*Kernel)(BatchArgs);
-    const Kernel k = mixed ? (Kernel)batched_mixed_kernel<512, 1, true, true> : (Kernel)batched_fp64_kernel<512, 1, true, true>;
+    *kernel = mixed ? (Kernel)batched_mixed_kernel<512, 1, true, true> : (Kernel)batched_fp64_kernel<512, 1, true, true>;
     const size_t smem = (size_t)smemRows * (mixed ? sizeof(float) : sizeof(double));
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)ctas);
-    cfg.blockDim = dim3(512);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    *cfg = {};
+    cfg->gridDim = dim3((unsigned)ctas);
+    cfg->blockDim = dim3(512);
+    cfg->dynamicSmemBytes = smem;
+    cfg->stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)ctas;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg->attrs = attr;
+    cfg->numAttrs = 1;
+    *clusters = 0;
+    return e == cudaSuccess ? cudaOccupancyMaxActiveClusters(clusters, *kernel, cfg) : e;
+}
+
+int batch_team_clusters(bool mixed, int ctas, int smemRows) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    void (*k)(BatchArgs);
     int clusters = 0;
-    if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&clusters, k, &cfg);
+    if (team_config(mixed, ctas, smemRows, nullptr, &cfg, attr, &k, &clusters) == cudaSuccess) return clusters;
+    cudaGetLastError();
+    return 0;
+}
+
+cudaError_t batch_team_launch(cudaStream_t st, bool mixed, int ctas, int smemRows, const BatchLaunch& L, int nteam,
+                              int* gridOut) {
+    if (L.sliceOff == nullptr || ctas < 2 || ctas > kTeamMax) return cudaErrorInvalidValue;
+    BatchArgs a = batch_args(L, smemRows);
+    a.nteam = nteam;
+    a.teamCtas = ctas;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[1];
+    void (*k)(BatchArgs);
+    int clusters = 0;
+    const cudaError_t e = team_config(mixed, ctas, smemRows, st, &cfg, attr, &k, &clusters);
     if (e != cudaSuccess) return e;
     if (clusters < 1) return cudaErrorInvalidConfiguration;
     // no more than the work calls for: a team per long system, a CTA per other

@@ -169,6 +169,7 @@ void PcgHandle::init(int device) {
     m_faultAlloc = envIs("XJPCG_FAULT", "alloc");
     m_faultLaunch = envIs("XJPCG_FAULT", "launch");
     m_faultPost = envIs("XJPCG_FAULT", "post");
+    m_faultCluster = envIs("XJPCG_FAULT", "cluster");
     m_initDone = true;
 }
 
@@ -1070,7 +1071,7 @@ int PcgHandle::loopKernel(uint32_t maxIter, int* layout) {
         *layout = isPat(m_spmvCfg) ? 2 : (isSellNarrow(m_spmvCfg) ? 1 : 0);
     else
         *layout = m_psState == 1 ? 2 : (m_sellNarrow ? 1 : 0);
-    return cg_cluster_fits((int)m_n, m_sellTotal) ? 2 : 1;
+    return !m_faultCluster && cg_cluster_fits((int)m_n, m_sellTotal) ? 2 : 1;
 }
 
 // One launch for the vector init, one for the loop.
@@ -1885,11 +1886,15 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
         return rows <= batch_cluster_rows(mixed, c < 5) &&
                batch_cluster_smem(mixed, n, std::max(1, width[s]), ctasOf(c)) <= batch_cluster_room(mixed, c < 5);
     };
+    // XJPCG_FAULT=cluster: as on a device (or a part of one) that holds no cluster
+    bool offered[kBatchClasses];
+    for (int c = 0; c < kBatchClasses; ++c)
+        offered[c] = ctasOf(c) == 1 || (!m_faultCluster && batch_cluster_offered(mixed, c < 5, ctasOf(c)));
     std::vector<uint8_t> cls(nsys);
     double sms = 0.0;
     for (uint32_t s = 0; s < nsys; ++s) {
         int c = 0;
-        while (c < kBatchClasses && !fits(s, c)) ++c;
+        while (c < kBatchClasses && !(offered[c] && fits(s, c))) ++c;
         if (c == kBatchClasses || hSys[s + 1] - hSys[s] > 65536) return false;
         cls[s] = (uint8_t)c;
         sms += smsOf(c);
@@ -1898,7 +1903,7 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
         more = false;
         sms = 0.0;
         for (uint32_t s = 0; s < nsys; ++s) {
-            if (cls[s] % 5 < 4 && hSys[s + 1] - hSys[s] > 128 * ctasOf(cls[s])) {
+            if (cls[s] % 5 < 4 && offered[cls[s] + 1] && hSys[s + 1] - hSys[s] > 128 * ctasOf(cls[s])) {
                 ++cls[s];
                 more = true;
             }
@@ -2149,7 +2154,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         L.order = m_bOrder.as<int>() + (teams ? nsys : 0);
         L.nsys = (int)(teams ? singles : nsys);
         const cudaError_t err =
-            teams ? batch_team_launch(m_stream, mixed, teams, m_numSms, rows, L, (int)(nsys - singles), &grid)
+            teams ? batch_team_launch(m_stream, mixed, teams, rows, L, (int)(nsys - singles), &grid)
                   : batch_launch(cfg, mixed, m_numSms, rows, m_stream, L, &grid);
         check(cudaEventRecord(m_ev1, m_stream), "event");
         check(err, "batched kernel");
@@ -2163,7 +2168,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         // for this call alone: the tuner's plan stands beside it
         plan.cfg = forced % ncfg;
         plan.smemRows = smemRows[forced / ncfg];
-        plan.teams = teamsEnv == 1 && singles < nsys ? 4 : 0;
+        plan.teams = teamsEnv == 1 && singles < nsys && !m_faultCluster && batch_team_clusters(mixed, 4, plan.smemRows) > 0 ? 4 : 0;
     } else if (m_batchKey != key || plan.cfg < 0) {
         // The sliced shapes (the CSR ones where there is no sliced copy: on
         // 1,024 systems they took 1.1 to 1.9 times as long), with and without
@@ -2181,22 +2186,25 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
                 plan.teams = teams;
             }
         };
-        const bool canTeam = singles < nsys && teamsEnv != 0;
+        // 512-thread CTAs, 4,096 rows or 44 KB of p; team sizes that the device holds
+        std::vector<std::pair<int, int>> teamShapes;  // rows, CTAs
+        if (singles < nsys && teamsEnv != 0 && !m_faultCluster)
+            for (int rows : {std::min(maxN, 4096), std::min(maxN, (int)(44 * 1024 / esz))})
+                for (int teams : {2, 4, 8})
+                    if (batch_team_clusters(mixed, teams, rows) > 0) teamShapes.emplace_back(rows, teams);
+        const bool teamsOnly = teamsEnv == 1 && !teamShapes.empty();
         for (size_t si = 0; si < smemRows.size(); ++si)
             for (int c = 0; c < ncfg; ++c) {
-                if (batch_config_sliced(c) != sliced || (canTeam && teamsEnv == 1)) continue;
+                if (batch_config_sliced(c) != sliced || teamsOnly) continue;
                 consider(c, smemRows[si], 0, &m_batchTuneMs[si * ncfg + c]);
             }
-        if (canTeam) {  // 512-thread CTAs, 4,096 rows or 44 KB of p
-            int c512 = 0;
-            for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
-                batch_config_shape(c, &t, &g);
-                if (batch_config_sliced(c) && t == 512) c512 = c;
-            }
-            float unused = -1.f;
-            for (int rows : {std::min(maxN, 4096), std::min(maxN, (int)(44 * 1024 / esz))})
-                for (int teams : {2, 4, 8}) consider(c512, rows, teams, &unused);
+        int c512 = 0;
+        for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
+            batch_config_shape(c, &t, &g);
+            if (batch_config_sliced(c) && t == 512) c512 = c;
         }
+        float unused = -1.f;
+        for (const auto& t : teamShapes) consider(c512, t.first, t.second, &unused);
         m_batchPlan = plan;
         m_batchKey = key;
     }

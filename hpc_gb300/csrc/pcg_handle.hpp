@@ -353,7 +353,7 @@ class PcgHandle {
     bool m_useGraph = true;
     bool m_fusedUpdate = true;  // XJPCG_FUSED_UPDATE
     int m_loopKernelEnv = -1;   // XJPCG_LOOP_KERNEL: 0 never, 1 also with a forced sliced layout
-    bool m_faultAlloc = false, m_faultLaunch = false, m_faultPost = false, m_initDone = false;  // XJPCG_FAULT hooks
+    bool m_faultAlloc = false, m_faultLaunch = false, m_faultPost = false, m_faultCluster = false, m_initDone = false;  // XJPCG_FAULT hooks
     size_t m_guardBytes = 0;                                   // XJPCG_GUARD_BYTES
     std::vector<std::pair<DevBuf*, std::string>> m_guarded;    // buffers allocated with guards
 

@@ -279,6 +279,8 @@ struct BatchClusterArgs {
 int batch_cluster_rows(bool mixed, bool small);     // most rows of a CTA
 size_t batch_cluster_room(bool mixed, bool small);  // most shared memory of a CTA
 size_t batch_cluster_smem(bool mixed, int n, int width, int ctas);
+// whether the current device can hold clusters of that many such CTAs
+bool batch_cluster_offered(bool mixed, bool small, int ctas);
 // a.ctas CTAs per system, small or wide
 cudaError_t batch_cluster_launch(cudaStream_t st, bool mixed, bool small, int systems, size_t smem,
                                  const BatchClusterArgs& a);
@@ -306,8 +308,10 @@ cudaError_t batch_sell_fill(cudaStream_t st, int nsys, int nslices, const int* s
                             const int* rowptr, const int* col, const double* val, const int* sliceOff,
                             const int* patLen, const int* patOff, VT* sval, uint16_t* scol);
 // the nteam systems after the first nsys of L.order on clusters of ctas (2, 4, 8) CTAs, then the others
-cudaError_t batch_team_launch(cudaStream_t st, bool mixed, int ctas, int numSms, int smemRows, const BatchLaunch& L,
-                              int nteam, int* gridOut);
+cudaError_t batch_team_launch(cudaStream_t st, bool mixed, int ctas, int smemRows, const BatchLaunch& L, int nteam,
+                              int* gridOut);
+// clusters of that many CTAs that the current device holds at once, 0: none
+int batch_team_clusters(bool mixed, int ctas, int smemRows);
 cudaError_t batch_launch(int cfg, bool mixed, int numSms, int smemRows, cudaStream_t st, const BatchLaunch& L,
                          int* gridOut);
 

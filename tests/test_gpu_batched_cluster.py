@@ -175,3 +175,21 @@ def test_batched_arrays_wherever_they_lie(gpu_lib, place):
         assert st == X.SUCCESS, h.last_message()
         _, want, _ = h.batch_solve(batch, 2000, 1e-10)
     assert np.array_equal(x.cpu().numpy(), np.concatenate(want))
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_batches_and_solves_without_clusters(gpu_lib, precision, monkeypatch):
+    # a device that cannot hold a cluster (XJPCG_FAULT=cluster: the question is answered
+    # with no): the kernels that need none run instead, in a forced form too
+    monkeypatch.setenv("XJPCG_FAULT", "cluster")
+    batch = BATCHES["clusters"]()
+    with X.JPCG() as h:
+        for teams in ("-1", "1"):
+            monkeypatch.setenv("XJPCG_BATCH_TEAMS", teams)
+            st, xs, res = h.batch_solve(batch, 20000, 1e-10, precision=precision)
+            assert st == X.SUCCESS, h.last_message()
+            assert h.info().batchSmemRows > 0 and h.info().batchGrid <= len(batch)  # one CTA per system
+            _check(batch, xs, res, precision)
+        s = batch[1]
+        r = h.csr_solve(s.n, s.rowptr, s.col, s.val, s.diag, s.b, 20000, 1e-10)
+        assert r.status == X.SUCCESS and oracle.true_relres(s.rowptr, s.col, s.val, s.b, r.x) <= 1.5e-10
