@@ -2170,9 +2170,8 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         plan.smemRows = smemRows[forced / ncfg];
         plan.teams = teamsEnv == 1 && singles < nsys && !m_faultCluster && batch_team_clusters(mixed, 4, plan.smemRows) > 0 ? 4 : 0;
     } else if (m_batchKey != key || plan.cfg < 0) {
-        // The sliced shapes (the CSR ones where there is no sliced copy: on
-        // 1,024 systems they took 1.1 to 1.9 times as long), with and without
-        // teams.
+        // The sliced shapes (the CSR ones where there is no sliced copy), with and
+        // without teams; then the CSR shapes at the best one's rows.
         m_batchTuneMs.assign((size_t)ncfg * smemRows.size(), -1.f);
         float best = 1e30f;
         auto consider = [&](int c, int rows, int teams, float* told) {
@@ -2205,6 +2204,30 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         }
         float unused = -1.f;
         for (const auto& t : teamShapes) consider(c512, t.first, t.second, &unused);
+        // CSR shapes win on uneven rows (two lanes a row) and on systems of one to a
+        // few slices (128 threads): kernel ms, fp64 / mixed, sliced against CSR, 600
+        // systems of 3,000 rows of Zipf length 9.2 / 7.0 against 4.7 / 3.5, 600 of
+        // 1,452 7-point rows with one of 300 entries 4.2 / 5.2 against 2.8 / 1.6, 5,000
+        // of 40 rows 1.3 / 2.0 against 0.9 / 1.1, 3,000 of 100 - 200 1.8 / 2.8 against
+        // 1.4 / 1.5; on larger stencil systems they take 1.1 to 1.9 times as long.
+        // The winner is one of these two or close to it, so the other four are timed
+        // only where one of the two comes within 1.2 of the best.
+        if (sliced && !teamsOnly) {
+            const int rows = plan.smemRows;
+            const size_t si = std::find(smemRows.begin(), smemRows.end(), rows) - smemRows.begin();
+            const float sliceBest = best;
+            float csrBest = 1e30f;
+            for (int pass = 0; pass < 2 && (pass == 0 || csrBest <= 1.2f * sliceBest); ++pass)
+                for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
+                    batch_config_shape(c, &t, &g);
+                    const bool first = (t == 256 && g == 2) || t == 128;
+                    if (batch_config_sliced(c) || first != (pass == 0)) continue;
+                    float ms = -1.f;
+                    consider(c, rows, 0, &ms);
+                    if (si < smemRows.size()) m_batchTuneMs[si * ncfg + c] = ms;
+                    csrBest = std::min(csrBest, ms);
+                }
+        }
         m_batchPlan = plan;
         m_batchKey = key;
     }

@@ -27,3 +27,26 @@ def test_a_forced_shape_does_not_outlive_its_call(gpu_lib, precision, forced, mo
         assert plan == [getattr(h.info(), f) for f in ("batchThreads", "batchLanes", "batchSliced", "batchSmemRows")]
         for a, b in zip(first, again):
             assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_uneven_rows_find_the_csr_shapes(gpu_lib, precision, monkeypatch):
+    # a row of 300 among rows of 7 holds a slice's other lanes up: the CSR shapes take
+    # less than two thirds of the time
+    monkeypatch.setenv("XJPCG_BATCH_CLUSTERS", "0")
+    rng = np.random.default_rng(4)
+    s = W.variable_stencil((11, 11, 12), 1.0, rng)
+    a = np.zeros((s.n, s.n))
+    a[np.repeat(np.arange(s.n), np.diff(s.rowptr)), s.col] = s.val
+    far = rng.choice(np.arange(800, s.n), 300, replace=False)
+    a[700, far] = a[far, 700] = -rng.uniform(0.1, 1.0, 300)
+    np.fill_diagonal(a, np.abs(a).sum(1) - np.abs(np.diag(a)) + np.diag(a))
+    rows, cols = np.nonzero(a)
+    rowptr = np.concatenate([[0], np.cumsum(np.bincount(rows, minlength=s.n))]).astype(np.int32)
+    hub = W.System(s.n, rowptr, cols.astype(np.int32), a[rows, cols], np.diag(a).copy(), s.b)
+    with X.JPCG() as h:
+        st, xs, res = h.batch_solve([hub] * 400, 20000, 1e-10, precision=precision)
+        assert st == X.SUCCESS, h.last_message()
+        assert h.info().batchSliced == 0
+        for x in xs[:2]:
+            assert np.linalg.norm(hub.b - a @ x) <= 1.5e-10 * np.linalg.norm(hub.b)
