@@ -1776,6 +1776,11 @@ namespace {
 __attribute__((unused)) uint64_t mixKey(uint64_t h, uint64_t v) { return (h ^ v) * 0x100000001b3ull; }
 }  // namespace
 
+namespace {
+// CTAs per system of a class of ClusterPlan
+int batchClassCtas(int c) { return 1 << (c % 5); }
+}  // namespace
+
 // One stream per number of CTAs per system, the larger ahead of the smaller.
 void PcgHandle::batchStreams() {
     if (m_batchFork == nullptr) {
@@ -1861,24 +1866,19 @@ void PcgHandle::batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* 
         const double n = in.sys[s + 1] - in.sys[s], reach = std::max(1, in.width[nsys + s]);
         in.work[s] = ((double)(in.entry[s + 1] - in.entry[s]) + 7.0 * n) * std::min(std::sqrt(n), n / reach);
     }
+    in.reach.assign(in.width.begin() + nsys, in.width.end());
     in.width.resize(nsys);
 }
 
-// The batch with every system in shared memory (batched_cluster.cu).  False
-// when that is not the way for it (nothing has run then).
-bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol, bool mixed) {
+// Whether and how the batch can run with every system in shared memory
+// (batched_cluster.cu).  Class of a system: 0 .. 4 small CTAs, 1, 2, 4, 8 or 16
+// of them, 5 .. 9 wide ones.  The first that holds it; while the GPU has room,
+// twice the CTAs.
+PcgHandle::ClusterPlan PcgHandle::clusterPlan(const BatchInput& in, bool mixed) const {
     const uint32_t nsys = (uint32_t)in.width.size();
     const std::vector<int32_t>&hSys = in.sys, &width = in.width;
-    BatchClusterArgs a;
-    a.sysRow = m_bSysRow.as<int>();
-    a.rowptr = in.rowptr;
-    a.col = in.col;
-    a.val = in.val;
-    a.b = in.b;
-    a.diag = in.diag;
-    // Class of a system: 0 .. 4 small CTAs, 1, 2, 4, 8 or 16 of them, 5 .. 9 wide
-    // ones.  The first that holds it; while the GPU has room, twice the CTAs.
-    auto ctasOf = [](int c) { return 1 << (c % 5); };
+    ClusterPlan plan;
+    auto ctasOf = batchClassCtas;
     auto smsOf = [&](int c) { return ctasOf(c) / (c < 5 ? (mixed ? 6.0 : 5.0) : (mixed ? 3.0 : 2.0)); };
     auto fits = [&](uint32_t s, int c) {
         const int n = hSys[s + 1] - hSys[s];
@@ -1890,12 +1890,13 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
     bool offered[kBatchClasses];
     for (int c = 0; c < kBatchClasses; ++c)
         offered[c] = ctasOf(c) == 1 || (!m_faultCluster && batch_cluster_offered(mixed, c < 5, ctasOf(c)));
-    std::vector<uint8_t> cls(nsys);
+    std::vector<uint8_t>& cls = plan.cls;
+    cls.resize(nsys);
     double sms = 0.0;
     for (uint32_t s = 0; s < nsys; ++s) {
         int c = 0;
         while (c < kBatchClasses && !(offered[c] && fits(s, c))) ++c;
-        if (c == kBatchClasses || hSys[s + 1] - hSys[s] > 65536) return false;
+        if (c == kBatchClasses || hSys[s + 1] - hSys[s] > 65536) return plan;
         cls[s] = (uint8_t)c;
         sms += smsOf(c);
     }
@@ -1920,8 +1921,48 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
     //   600 of 1,000 - 2,500                8.4          5.6         3.7
     //   300 of 200 - 20,000                 24.6 / 10    18 / 14     4.1 / 3.5
     //   2,000 of 200 - 20,000               145 / 57     66 / 37     28 / 24
-    if (sms > (mixed ? 4.0 : 2.5) * m_numSms) return false;
-    alloc(m_bOrder, sizeof(int32_t) * nsys, "batch order");
+    if (sms > (mixed ? 4.0 : 2.5) * m_numSms) return plan;
+    plan.offered = true;
+    // Without timing the other kernels, where this one is known to win: stencils
+    // (few entries a row, columns near the diagonal) in a batch that has fewer
+    // systems than the GPU has SMs, or whose longest systems would keep single SMs
+    // busy.  Against the streaming kernels' best, fp64 / mixed: 8 to 100 systems of
+    // 1,452 7-point rows 0.62 - 0.90 / 0.59 - 0.81, of 8,000 0.71 - 1.01 / 0.61 -
+    // 0.76; 5 of 2,162 - 17,550 rows 0.74 / 0.48.  Elsewhere it can lose, and the
+    // tuner times both: 300 and 900 such even systems 1.56 / 1.27 and - / 1.83; rows
+    // beyond 8 entries, random columns or a long row in every system (padding to the
+    // longest row takes CTAs) 0.7 to 12.  A batch of systems within one slice takes
+    // 20 us either way.
+    double mean = 0.0, most = 0.0;
+    int maxN = 0;
+    bool stencils = true;
+    for (uint32_t s = 0; s < nsys; ++s) {
+        const int n = hSys[s + 1] - hSys[s];
+        maxN = std::max(maxN, n);
+        mean += in.work[s] / nsys;
+        most = std::max(most, in.work[s]);
+        stencils = stencils && (n <= 64 || (width[s] <= kBatchPatMax && 2 * in.reach[s] <= n));
+    }
+    plan.sure = stencils && (nsys < 100 || (most >= 3.0 * mean && sms <= 1.5 * m_numSms) ||
+                             (maxN <= 32 && sms <= 0.8 * m_numSms));
+    return plan;
+}
+
+// Solves the batch that way; device time in *ms.
+void PcgHandle::runClusters(const BatchInput& in, const ClusterPlan& plan, uint32_t maxIter, double tol, bool mixed,
+                            float* ms) {
+    const uint32_t nsys = (uint32_t)in.width.size();
+    const std::vector<int32_t>&hSys = in.sys, &width = in.width;
+    const std::vector<uint8_t>& cls = plan.cls;
+    auto ctasOf = batchClassCtas;
+    BatchClusterArgs a;
+    a.sysRow = m_bSysRow.as<int>();
+    a.rowptr = in.rowptr;
+    a.col = in.col;
+    a.val = in.val;
+    a.b = in.b;
+    a.diag = in.diag;
+    alloc(m_bClusterOrder, sizeof(int32_t) * nsys, "batch order");
     std::vector<int32_t> order(nsys);
     for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
     // by class, the longest first in each
@@ -1929,7 +1970,8 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
         if (cls[p] != cls[q]) return cls[p] > cls[q];
         return in.work[p] > in.work[q];
     });
-    check(cudaMemcpyAsync(m_bOrder.p, order.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice, m_stream), "H2D");
+    check(cudaMemcpyAsync(m_bClusterOrder.p, order.data(), sizeof(int32_t) * nsys, cudaMemcpyHostToDevice, m_stream),
+          "H2D");
     a.width = m_bWidth.as<int>();
     a.x = m_bX.as<double>();
     a.res = m_bRes.as<BatchResult>();
@@ -1956,7 +1998,7 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
             const int s = order[end];
             smem = std::max(smem, batch_cluster_smem(mixed, hSys[s + 1] - hSys[s], std::max(1, width[s]), teamOf));
         }
-        a.order = m_bOrder.as<int>() + at;
+        a.order = m_bClusterOrder.as<int>() + at;
         a.ctas = teamOf;
         if (err == cudaSuccess) err = cudaStreamWaitEvent(m_batchStream[c], m_batchFork, 0);
         if (err == cudaSuccess) err = batch_cluster_launch(m_batchStream[c], mixed, c < 5, (int)(end - at), smem, a);
@@ -1969,8 +2011,7 @@ bool PcgHandle::batchClusters(const BatchInput& in, uint32_t maxIter, double tol
     check(cudaEventRecord(m_ev1, m_stream), "event");
     check(cudaEventSynchronize(m_ev1), "event");
     check(err, "batched cluster kernel");
-    check(cudaEventElapsedTime(&m_batchMs, m_ev0, m_ev1), "event");
-    return true;
+    check(cudaEventElapsedTime(ms, m_ev0, m_ev1), "event");
 }
 
 uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
@@ -1993,9 +2034,12 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     // Forced kernel shapes and layouts take the kernels they name.
     const int forced = envInt("XJPCG_BATCH_CFG", -1);
     const bool forcedShape = forced >= 0 || envInt("XJPCG_BATCH_SLICED", 1) == 0 || envInt("XJPCG_BATCH_PATTERNS", 1) == 0;
-    m_batchClusterCtas = 0;
-    if (!forcedShape && envInt("XJPCG_BATCH_CLUSTERS", 1) != 0 && batchClusters(in, maxIter, tol, mixed))
+    ClusterPlan clusters;
+    if (!forcedShape && envInt("XJPCG_BATCH_CLUSTERS", 1) != 0) clusters = clusterPlan(in, mixed);
+    if (clusters.sure) {
+        runClusters(in, clusters, maxIter, tol, mixed, &m_batchMs);
         return batchResults(nsys, total, x, tol, results, onDevice);
+    }
     // Queue order: the longest solves first.
     std::vector<int32_t> order(nsys);
     for (uint32_t s = 0; s < nsys; ++s) order[s] = (int32_t)s;
@@ -2017,6 +2061,24 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     std::vector<int32_t> teamOrder(order);
     std::stable_sort(teamOrder.begin(), teamOrder.end(), [&](int32_t p, int32_t q) { return isLong[p] < isLong[q]; });
     uint32_t singles = (uint32_t)std::count(isLong.begin(), isLong.end(), 0);
+    // Per-system SELL-32 copy for the sliced kernels: offered when every system has
+    // at most 65,536 rows and the copy fits 32-bit offsets.
+    int64_t nslices = 0;
+    for (uint32_t s = 0; s < nsys; ++s) nslices += (hSys[s + 1] - hSys[s] + 31) / 32;
+    const bool sliced = maxN <= 65536 &&
+                        nslices * 32 * (int64_t)std::max(maxRowLen, kBatchPatMax) < 0x7fffff00ll &&
+                        envInt("XJPCG_BATCH_SLICED", 1) != 0;
+    if (!sliced) singles = nsys;  // the team kernels read the sliced copy
+    // 0: no teams, 1: always, -1: where they are faster
+    const int teamsEnv = envInt("XJPCG_BATCH_TEAMS", forcedShape ? 0 : -1);
+    const uint64_t shape = mixKey(mixKey(mixKey(nsys, (uint64_t)total), (uint64_t)nnz), (uint64_t)maxN);
+    const uint64_t key = mixKey(mixKey(shape, nsys - singles),
+                                (uint64_t)precision + 7 + (sliced ? 1000 : 0) + 10000 * (uint64_t)(teamsEnv + 1) +
+                                    (clusters.offered ? 100000 : 0));
+    if (forced < 0 && m_batchKey == key && m_batchPlan.clusters) {
+        runClusters(in, clusters, maxIter, tol, mixed, &m_batchMs);
+        return batchResults(nsys, total, x, tol, results, onDevice);
+    }
     const size_t vb = sizeof(double) * ((size_t)total + 4), fb = sizeof(float) * ((size_t)total + 4);
     alloc(m_bOrder, sizeof(int32_t) * 2 * nsys, "batch order");
     for (DevBuf* v : {&m_bR, &m_bAp, &m_bJ, &m_bP}) alloc(*v, vb, "batch vector");
@@ -2028,14 +2090,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
                           m_stream),
           "H2D");
 
-    // Per-system SELL-32 copy for the sliced kernels: 32-row slices of each
-    // system, values slice-column-major, 16-bit local columns.  Offered when
-    // every system has at most 65,536 rows and the copy fits 32-bit offsets.
-    int64_t nslices = 0;
-    for (uint32_t s = 0; s < nsys; ++s) nslices += (hSys[s + 1] - hSys[s] + 31) / 32;
-    const bool sliced = maxN <= 65536 &&
-                        nslices * 32 * (int64_t)std::max(maxRowLen, kBatchPatMax) < 0x7fffff00ll &&
-                        envInt("XJPCG_BATCH_SLICED", 1) != 0;
+    // 32-row slices of each system, values slice-column-major, 16-bit local columns
     if (sliced) {
         const int nsl = (int)nslices;
         std::vector<int32_t> hBase(nsys + 1, 0);
@@ -2083,7 +2138,6 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         }
     }
 
-    if (!sliced) singles = nsys;  // the team kernels read the sliced copy
     BatchLaunch L;
     L.sysRow = m_bSysRow.as<int>();
     L.rowptr = in.rowptr;
@@ -2135,11 +2189,6 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         rows = std::min(maxN, rows);
         if (std::find(smemRows.begin(), smemRows.end(), rows) == smemRows.end()) smemRows.push_back(rows);
     }
-    // 0: no teams, 1: always, -1: where they are faster
-    const int teamsEnv = envInt("XJPCG_BATCH_TEAMS", forcedShape ? 0 : -1);
-    const uint64_t shape = mixKey(mixKey(mixKey(nsys, (uint64_t)total), (uint64_t)nnz), (uint64_t)maxN);
-    const uint64_t key = mixKey(mixKey(shape, nsys - singles),
-                                (uint64_t)precision + 7 + (sliced ? 1000 : 0) + 10000 * (uint64_t)(teamsEnv + 1));
     // One batch; teams: CTAs per long system, 0 for none.
     auto runOnce = [&](int cfg, int rows, int teams, float* ms) {
         if (mixed && teams == 0 && !batch_config_sliced(cfg) && L.val32 == nullptr) {
@@ -2166,6 +2215,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
     BatchPlan plan = m_batchPlan;
     if (forced >= 0 && forced < ncfg * (int)smemRows.size()) {
         // for this call alone: the tuner's plan stands beside it
+        plan = BatchPlan();
         plan.cfg = forced % ncfg;
         plan.smemRows = smemRows[forced / ncfg];
         plan.teams = teamsEnv == 1 && singles < nsys && !m_faultCluster && batch_team_clusters(mixed, 4, plan.smemRows) > 0 ? 4 : 0;
@@ -2173,6 +2223,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         // The sliced shapes (the CSR ones where there is no sliced copy), with and
         // without teams; then the CSR shapes at the best one's rows.
         m_batchTuneMs.assign((size_t)ncfg * smemRows.size(), -1.f);
+        plan = BatchPlan();
         float best = 1e30f;
         auto consider = [&](int c, int rows, int teams, float* told) {
             float ms = 0;
@@ -2228,13 +2279,23 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
                     csrBest = std::min(csrBest, ms);
                 }
         }
+        if (clusters.offered) {
+            float ms = 0;
+            runClusters(in, clusters, maxIter, tol, mixed, &ms);
+            plan.clusters = ms <= best;
+        }
         m_batchPlan = plan;
         m_batchKey = key;
     }
-    faultPoint("batched launch");
-    runOnce(plan.cfg, plan.smemRows, plan.teams, &m_batchMs);
-    m_batchCfg = plan.cfg;
-    m_batchSmemRows = plan.smemRows;
+    if (plan.clusters) {
+        runClusters(in, clusters, maxIter, tol, mixed, &m_batchMs);
+    } else {
+        faultPoint("batched launch");
+        runOnce(plan.cfg, plan.smemRows, plan.teams, &m_batchMs);
+        m_batchCfg = plan.cfg;
+        m_batchSmemRows = plan.smemRows;
+        m_batchClusterCtas = 0;
+    }
     return batchResults(nsys, total, x, tol, results, onDevice);
 }
 

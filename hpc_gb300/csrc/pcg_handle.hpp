@@ -209,14 +209,22 @@ class PcgHandle {
     int loopKernel(uint32_t maxIter, int* layout);
     // A batch's arrays on the device, and what the host needs of them.
     struct BatchInput {
-        std::vector<int32_t> sys, entry, width;  // first row and entry of each system (and the ends), longest row
-        std::vector<double> work;                // of each system, a guess
+        std::vector<int32_t> sys, entry;    // first row and entry of each system, and the ends
+        std::vector<int32_t> width, reach;  // its longest row, its columns' largest distance from the diagonal
+        std::vector<double> work;           // a guess
         const int *rowptr = nullptr, *col = nullptr;
         const double *val = nullptr, *diag = nullptr, *b = nullptr;
     };
     void batchInput(uint32_t nsys, const int32_t* sysRow, const int32_t* rowPtr, const int32_t* colIdx,
                     const double* values, const double* diag, const double* b, bool onDevice, BatchInput& in);
-    bool batchClusters(const BatchInput& in, uint32_t maxIter, double tol, bool mixed);
+    // The batch from shared memory: whether it can, whether it is known to be the
+    // fastest way, and the class of each system.
+    struct ClusterPlan {
+        bool offered = false, sure = false;
+        std::vector<uint8_t> cls;
+    };
+    ClusterPlan clusterPlan(const BatchInput& in, bool mixed) const;
+    void runClusters(const BatchInput& in, const ClusterPlan& plan, uint32_t maxIter, double tol, bool mixed, float* ms);
     void batchStreams();
     uint32_t batchResults(uint32_t nsys, int total, double* x, double tol, BatchResult* results, bool onDevice);
     void launchLoopKernel(int form, int layout, uint32_t maxIter);
@@ -322,16 +330,17 @@ class PcgHandle {
     bool m_haveX = false, m_haveLambda = false;
 
     // batched solves
-    DevBuf m_bSysRow, m_bOrder, m_bRowptr, m_bCol, m_bVal, m_bVal32, m_bB, m_bDiag, m_bX, m_bR, m_bAp, m_bJ;
+    DevBuf m_bSysRow, m_bOrder, m_bClusterOrder, m_bRowptr, m_bCol, m_bVal, m_bVal32, m_bB, m_bDiag, m_bX, m_bR, m_bAp, m_bJ;
     DevBuf m_bR32, m_bD32, m_bAp32, m_bJ32, m_bP, m_bP32, m_bRes, m_bQueue;
     DevBuf m_bsBase, m_bsLen, m_bsOff, m_bsScan, m_bsVal, m_bsVal32, m_bsCol;  // per-system SELL-32 copy
     DevBuf m_bsPatLen, m_bsPatOff;  // its slices' shared column offsets
     DevBuf m_bsMeta, m_bsSysPat;    // slice records, and each system's offsets
     int m_batchCfg = -1, m_batchSmemRows = 0, m_batchGrid = 0;  // of the last batch of the streaming kernels
     // The tuner's choice for batches of m_batchKey's kind: kernel shape, rows of p
-    // in shared memory, CTAs per long system (0: one each).
+    // in shared memory, CTAs per long system (0: one each); or from shared memory.
     struct BatchPlan {
         int cfg = -1, smemRows = 0, teams = 0;
+        bool clusters = false;
     };
     BatchPlan m_batchPlan;
     uint64_t m_batchKey = 0;
