@@ -683,6 +683,8 @@ constexpr int kSmall = 128, kSmallRows = 4;
 constexpr size_t kWideSmem = 96 * 1024, kSmallSmem = 40 * 1024;
 }  // namespace
 
+int batch_cluster_threads(bool mixed, bool small) { return small ? kSmall : (mixed ? kWide32 : kWide64); }
+
 int batch_cluster_rows(bool mixed, bool small) {
     return small ? kSmall * kSmallRows : (mixed ? kWide32 * kWideRows32 : kWide64 * kWideRows64);
 }
@@ -718,7 +720,7 @@ cudaError_t cluster_config(ClusterKernel k, bool mixed, bool small, int systems,
     if (e == cudaSuccess && ctas > 8) e = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     *cfg = {};
     cfg->gridDim = dim3((unsigned)(systems * ctas));
-    cfg->blockDim = dim3((unsigned)(small ? kSmall : (mixed ? kWide32 : kWide64)));
+    cfg->blockDim = dim3((unsigned)batch_cluster_threads(mixed, small));
     cfg->dynamicSmemBytes = smem;
     cfg->stream = st;
     attr[0].id = cudaLaunchAttributeClusterDimension;

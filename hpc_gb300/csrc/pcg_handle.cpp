@@ -1990,6 +1990,7 @@ void PcgHandle::runClusters(const BatchInput& in, const ClusterPlan& plan, uint3
     check(cudaEventRecord(m_batchFork, m_stream), "event");
     cudaError_t err = cudaSuccess;
     m_batchClusterCtas = 0;
+    m_batchClusterThreads = batch_cluster_threads(mixed, cls[order[0]] < 5);
     for (uint32_t at = 0; at < nsys;) {
         const int c = cls[order[at]], teamOf = ctasOf(c);
         uint32_t end = at;
@@ -2000,6 +2001,7 @@ void PcgHandle::runClusters(const BatchInput& in, const ClusterPlan& plan, uint3
         }
         a.order = m_bClusterOrder.as<int>() + at;
         a.ctas = teamOf;
+        if (batch_cluster_threads(mixed, c < 5) != m_batchClusterThreads) m_batchClusterThreads = 0;
         if (err == cudaSuccess) err = cudaStreamWaitEvent(m_batchStream[c], m_batchFork, 0);
         if (err == cudaSuccess) err = batch_cluster_launch(m_batchStream[c], mixed, c < 5, (int)(end - at), smem, a);
         // joined whatever happened: nothing of the batch outlives the call
@@ -2419,7 +2421,7 @@ void PcgHandle::fillInfo(XJPCG_GbInfo_t* info) const {
     info->loopMode = m_useGraph ? 1u : 0u;
     // 0: the last fp64 solve ran its loop in one kernel; the host loop issues batches of 16
     info->loopUnroll = m_lastOneKernel ? 0u : (m_useGraph ? (uint32_t)kLoopUnroll : 16u);
-    info->kernelsPerIter = m_fusedUpdate ? 2u : 3u;
+    info->kernelsPerIter = (m_fusedUpdate ? 2u : 3u) + (isSorted(m_spmvCfg) && sortedHubs(m_spmvCfg) > 0 ? 1u : 0u);
     if (m_batchCfg >= 0) {
         int t = 0, l = 0;
         batch_config_shape(m_batchCfg, &t, &l);
@@ -2428,7 +2430,7 @@ void PcgHandle::fillInfo(XJPCG_GbInfo_t* info) const {
         info->batchSliced = batch_config_sliced(m_batchCfg) ? 1u : 0u;
     }
     if (m_batchClusterCtas > 0) {
-        info->batchThreads = 256u;
+        info->batchThreads = (uint32_t)m_batchClusterThreads;
         info->batchLanes = 1u;
         info->batchSliced = 1u;
     }

@@ -350,7 +350,8 @@ class PcgHandle {
     static constexpr int kBatchClasses = 10;             // 1, 2, 4, 8, 16 small CTAs per system, then wide ones
     cudaStream_t m_batchStream[kBatchClasses] = {};      // one per class, created on first use
     cudaEvent_t m_batchFork = nullptr, m_batchJoin[kBatchClasses] = {};
-    int m_batchClusterCtas = 0;                          // CTAs of the last cluster batch, 0: the other kernels ran
+    int m_batchClusterCtas = 0;     // CTAs of the last batch from shared memory, 0: the streaming kernels ran
+    int m_batchClusterThreads = 0;  // their size, 0: of both sizes
 
     // graph
     cudaGraphExec_t m_exec = nullptr;

@@ -276,6 +276,7 @@ struct BatchClusterArgs {
     int ctas = 1;  // CTAs per system: 1 .. 16
     uint32_t muteAt = ~0u;  // fault injection: the iteration in which the last CTA does not post to the first
 };
+int batch_cluster_threads(bool mixed, bool small);  // of a CTA
 int batch_cluster_rows(bool mixed, bool small);     // most rows of a CTA
 size_t batch_cluster_room(bool mixed, bool small);  // most shared memory of a CTA
 size_t batch_cluster_smem(bool mixed, int n, int width, int ctas);

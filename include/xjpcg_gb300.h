@@ -36,7 +36,7 @@ typedef struct {
                               3 = sliced with int16 column offsets, 4 = sliced with rows sorted by
                               length (long rows one warp each), 5 = sliced with column offsets
                               shared by the 32 rows of a slice */
-    uint32_t batchThreads; /* batched solves: CTA size chosen by the tuner */
+    uint32_t batchThreads; /* batched solves: CTA size of the last batch; 0: CTAs of two sizes */
     uint32_t batchLanes;   /* batched solves: lanes per row */
     uint32_t batchSmemRows;/* batched solves: rows of p held in shared memory */
     uint32_t batchGrid;    /* batched solves: CTAs of the persistent launch */
@@ -50,8 +50,10 @@ typedef struct {
     double uploadIdxMs;    /* of which the row and column index copies (on the handle's stream) */
     double uploadValMs;    /* of which the value copy (on the side stream, from its start) */
     uint32_t loopUnroll;   /* iterations per pass of a graph loop's body (kernels past the stop return at once);
-                              0 = the last fp64 solve ran as two launches, the init and the whole loop */
-    uint32_t kernelsPerIter; /* kernels per fp64 iteration: 2 (SpMV, fused vector kernel) or 3 (separate) */
+                              0 (test before dividing) = the last fp64 solve ran as two launches, the init and
+                              the whole loop, whatever spmvLayout says, over a sliced copy */
+    uint32_t kernelsPerIter; /* kernels per fp64 iteration of a graph or host loop: 2 (SpMV, fused vector kernel)
+                              or 3 (separate), and one more where the SpMV copies hub columns first */
 } XJPCG_GbInfo_t;
 
 /* Per-system outcome of a batched solve. */
