@@ -95,17 +95,20 @@ void PcgHandle::check(cudaError_t e, const char* what) {
 }
 
 void PcgHandle::alloc(DevBuf& b, size_t bytes, const char* what) {
+    if (!tryAlloc(b, bytes, what)) throw AllocFailed(std::string("device allocation failed for ") + what);
+}
+
+bool PcgHandle::tryAlloc(DevBuf& b, size_t bytes, const char* what) {
     // XJPCG_FAULT=alloc: every allocation after the handle's own set-up fails
     // as a cudaMalloc failure would (host-side fault injection).
-    if (m_faultAlloc && m_initDone && bytes > b.bytes)
-        throw AllocFailed(std::string("device allocation failed for ") + what);
-    if (!b.ensure(bytes, &m_generation, m_guardBytes))
-        throw AllocFailed(std::string("device allocation failed for ") + what);
+    if (m_faultAlloc && m_initDone && bytes > b.bytes) return false;
+    if (!b.ensure(bytes, &m_generation, m_guardBytes)) return false;
     if (m_guardBytes > 0) {
         bool known = false;
         for (const auto& g : m_guarded) known = known || g.first == &b;
         if (!known) m_guarded.emplace_back(&b, what);
     }
+    return true;
 }
 
 // Debug handles (XJPCG_GUARD_BYTES > 0 when the handle is created) allocate
@@ -170,6 +173,7 @@ void PcgHandle::init(int device) {
     m_faultLaunch = envIs("XJPCG_FAULT", "launch");
     m_faultPost = envIs("XJPCG_FAULT", "post");
     m_faultCluster = envIs("XJPCG_FAULT", "cluster");
+    m_faultHubs = envIs("XJPCG_FAULT", "hubs");
     m_initDone = true;
 }
 
@@ -593,44 +597,57 @@ bool PcgHandle::ensureSorted() {
         m_ssState = 2;
         return false;
     }
-    // Hub columns pay where x is larger than an L1 and they take a fifth of the
-    // gathers (39 % at 300,007 rows of the Zipf system: 11 % faster than the unroll of
-    // 4 without; 28 % at 2M rows: 5 % slower to 3 % faster, which the tuner settles; the
-    // copy of their x costs a launch, 2.5 us).
-    m_ssHubs = 0;
-    constexpr int kHubs = 16384;
-    if (n > 2 * kHubs) {
-        int entries = 0;
-        check(sellsort_hub_entries(m_stream, kHubs, m_ssSorted.as<int>(), m_rowptr.as<int>(), m_blockSums.as<int>(),
-                                   &entries),
-              "hub rows");
-        if ((uint64_t)entries * 5 >= m_nnz) {
-            alloc(m_ssHubOf, sizeof(int) * ((size_t)n + 4), "hub columns");
-            alloc(m_ssHubCol, sizeof(int) * ((size_t)m_nnz + 32), "recoded columns");
-            alloc(m_ssHubX, sizeof(double) * kHubs, "hub values");
-            check(sellsort_recode(m_stream, n, (int64_t)m_nnz, kHubs, m_ssSorted.as<int>(), m_col.as<int>(),
-                                  m_ssHubOf.as<int>(), m_ssHubCol.as<int>()),
-                  "hub columns");
-            m_ssHubs = kHubs;
-        }
-    }
     alloc(m_ssCol, sizeof(int) * ((size_t)total + 32), "sorted sliced columns");
     alloc(m_ssVal, sizeof(double) * ((size_t)total + 32), "sorted sliced values");
     check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), m_col.as<int>(), m_val.as<double>(),
                                 m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssCol.as<int>(), m_ssVal.as<double>()),
           "sorted sliced fill");
-    if (m_ssHubs > 0) {
-        alloc(m_ssHubScol, sizeof(int) * ((size_t)total + 32), "recoded sliced columns");
-        check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), m_ssHubCol.as<int>(), m_val.as<double>(),
-                                    m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssHubScol.as<int>(),
-                                    m_ssVal.as<double>()),
-              "sorted sliced fill");
-    }
+    buildHubs(nLong, total);
     m_ssLong = nLong;
     m_ssTotal = total;
     m_ssState = 1;
     m_ss32Valid = false;
     return true;
+}
+
+// Hub columns of the length-sorted copy.  They pay where x is larger than an L1
+// and they take a fifth of the gathers (39 % at 300,007 rows of the Zipf system: 11 %
+// faster than the unroll of 4 without; 28 % at 2M rows: 5 % slower to 3 % faster,
+// which the tuner settles; the copy of their x costs a launch, 2.5 us).  They cost 8
+// bytes per entry, which the rest of the handle does without: they are left out
+// where that is more than a quarter of the free memory, or cannot be had.
+void PcgHandle::buildHubs(int nLong, int64_t total) {
+    constexpr int kHubs = 16384;
+    const int n = (int)m_n;
+    m_ssHubs = 0;
+    if (n <= 2 * kHubs) return;
+    int entries = 0;
+    check(sellsort_hub_entries(m_stream, kHubs, m_ssSorted.as<int>(), m_rowptr.as<int>(), m_blockSums.as<int>(),
+                               &entries),
+          "hub rows");
+    if ((uint64_t)entries * 5 < m_nnz) return;
+    const size_t ofB = sizeof(int) * ((size_t)n + 4), colB = sizeof(int) * ((size_t)m_nnz + 32),
+                 scolB = sizeof(int) * ((size_t)total + 32), xB = sizeof(double) * kHubs;
+    size_t more = 0, free = 0, all = 0;  // beyond what an earlier matrix left
+    for (const auto& b : {std::make_pair(&m_ssHubOf, ofB), std::make_pair(&m_ssHubCol, colB),
+                          std::make_pair(&m_ssHubScol, scolB), std::make_pair(&m_ssHubX, xB)})
+        more += b.first->bytes < b.second ? b.second : 0;
+    if (more > 0) check(cudaMemGetInfo(&free, &all), "cudaMemGetInfo");
+    if (4 * more > free || m_faultHubs || !tryAlloc(m_ssHubOf, ofB, "hub columns") ||
+        !tryAlloc(m_ssHubCol, colB, "recoded columns") || !tryAlloc(m_ssHubScol, scolB, "recoded sliced columns") ||
+        !tryAlloc(m_ssHubX, xB, "hub values")) {
+        for (DevBuf* b : {&m_ssHubOf, &m_ssHubCol, &m_ssHubScol, &m_ssHubX}) b->release();
+        ++m_generation;
+        return;
+    }
+    check(sellsort_recode(m_stream, n, (int64_t)m_nnz, kHubs, m_ssSorted.as<int>(), m_col.as<int>(),
+                          m_ssHubOf.as<int>(), m_ssHubCol.as<int>()),
+          "hub columns");
+    check(sellsort_fill<double>(m_stream, n, nLong, m_rowptr.as<int>(), m_ssHubCol.as<int>(), m_val.as<double>(),
+                                m_ssSorted.as<int>(), m_ssSliceOff.as<int>(), m_ssHubScol.as<int>(),
+                                m_ssVal.as<double>()),
+          "sorted sliced fill");
+    m_ssHubs = kHubs;
 }
 
 void PcgHandle::ensureMergeScratch() {

@@ -178,6 +178,7 @@ class PcgHandle {
     void check(cudaError_t e, const char* what);
     void faultPoint(const char* what);
     void alloc(DevBuf& b, size_t bytes, const char* what);
+    bool tryAlloc(DevBuf& b, size_t bytes, const char* what);
     void finishMatrix();     // after CSR exists: values pad, tuning
     void tuneSpmv();
     int numSpmvCfgs() const;
@@ -275,6 +276,7 @@ class PcgHandle {
     DevBuf m_ssHubOf, m_ssHubCol, m_ssHubScol, m_ssHubX;
     int m_ssHubs = 0;  // columns whose x the unroll of 8 reads from a compact copy
     int sortedHubs(int cfg) const;
+    void buildHubs(int nLong, int64_t total);
     bool m_ss32Valid = false;
     int m_sellState = 0;  // 0 not built, 1 built, 2 rejected (too much padding)
     DevBuf m_mergeRow, m_mergeVal, m_mergePart;  // merge-path carries and partials
@@ -363,7 +365,7 @@ class PcgHandle {
     bool m_useGraph = true;
     bool m_fusedUpdate = true;  // XJPCG_FUSED_UPDATE
     int m_loopKernelEnv = -1;   // XJPCG_LOOP_KERNEL: 0 never, 1 also with a forced sliced layout
-    bool m_faultAlloc = false, m_faultLaunch = false, m_faultPost = false, m_faultCluster = false, m_initDone = false;  // XJPCG_FAULT hooks
+    bool m_faultAlloc = false, m_faultLaunch = false, m_faultPost = false, m_faultCluster = false, m_faultHubs = false, m_initDone = false;  // XJPCG_FAULT hooks
     size_t m_guardBytes = 0;                                   // XJPCG_GUARD_BYTES
     std::vector<std::pair<DevBuf*, std::string>> m_guarded;    // buffers allocated with guards
 

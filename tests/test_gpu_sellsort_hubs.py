@@ -49,3 +49,23 @@ def test_spmv_and_solves_with_hub_columns(gpu_lib, n):
     finally:
         for k in env:
             os.environ.pop(k, None)
+
+
+def test_without_memory_for_hub_columns_the_solve_goes_on(gpu_lib, monkeypatch):
+    # XJPCG_FAULT=hubs: their buffers cannot be had.  The same layout without them
+    # sums every row in the same order.
+    n = 50001
+    s = W.zipf_spd(n, hi=1500, seed=n)
+    x = np.random.default_rng(2).uniform(-1.0, 1.0, n)
+    monkeypatch.setenv("XJPCG_SPMV_LANES", "-4")
+    out = {}
+    for fault in ("", "hubs"):
+        monkeypatch.setenv("XJPCG_FAULT", fault)
+        with X.JPCG() as h:
+            r = h.csr_solve(n, s.rowptr, s.col, s.val, s.diag, s.b, 3000, 1e-10)
+            assert r.status == X.SUCCESS, r.message
+            assert h.info().spmvLayout == 4 and h.info().kernelsPerIter == (2 if fault else 3)
+            m = h.mixed_solve(s.b, s.diag, 3000, 1e-10)
+            assert m.status == X.SUCCESS, m.message
+            out[fault] = h.spmv(x)
+    assert np.array_equal(out[""], out["hubs"])
