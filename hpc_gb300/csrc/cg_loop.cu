@@ -13,8 +13,8 @@
 // Two forms:
 //   cg_cluster_kernel  one cluster of up to 16 CTAs; p is gathered, and the
 //                      sums are exchanged, through distributed shared memory;
-//                      so is the matrix kept on the chip if it fits.  Three
-//                      cluster barriers per iteration.
+//                      the matrix stays on the chip.  Three cluster barriers
+//                      per iteration.
 //   cg_loop_kernel     one CTA per SM, cooperative; sums go through posts and
 //                      counters in global memory, the matrix streams from L2.
 //
@@ -222,7 +222,6 @@ __global__ void __launch_bounds__(kLoopThreads, 1) cg_loop_kernel(LoopArgs a) {
         meta[i] = md;
     }
     if (tid == 0) sRz = a.state->rz;
-    __syncthreads();
     __syncthreads();
     const double tols = a.state->tols;
     const uint32_t maxIterP1 = a.state->maxIterP1;
@@ -503,13 +502,14 @@ __device__ __forceinline__ void to_all(double* place, double v, int P, int lane)
 
 }  // namespace
 
-// One cluster.  R rows per CTA, so a column's owner is column / R.  The matrix
-// part in shared memory holds, per entry, the value and the cluster address of
-// its p, so a gather is one load (about 250 cycles).  Every CTA writes its part
+// One cluster.  R rows per CTA, so a column's owner is column / R.  The matrix,
+// in shared memory, holds per entry the value and the cluster address of its p,
+// so a gather is one load (about 250 cycles; 4.5 cycles more per entry and CTA
+// where the lanes' addresses lie scattered).  NARROW: 16-bit column offsets.  Every CTA writes its part
 // of a sum to every CTA; after the cluster barrier each adds all of them in the
 // same order.  A CTA always runs to the same decision as the others, and no
 // CTA is read or written by another after its last cluster barrier.
-template <int LAY>
+template <bool NARROW>
 __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs a) {
     extern __shared__ __align__(16) unsigned char loopSmem[];
     __shared__ double slots[3][kClusterMax], part[2][kClusterThreads];
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
     double* const sz = sx + R;
     double* const sp = sz + R;
     double* const sj = sp + R;
-    int4* const meta = reinterpret_cast<int4*>(sj + R);
+    int2* const meta = reinterpret_cast<int2*>(sj + R);
     double* const mv = reinterpret_cast<double*>(meta + R / 32);
     for (int i = tid; i < R; i += nt) {
         const int e = row0 + i;
@@ -533,40 +533,25 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
         sj[i] = in ? a.J[e] : 0.0;
         sx[i] = 0.0;
     }
-    for (int i = tid; i < ns; i += nt) {
+    for (int i = tid; i < ns; i += nt) {  // slice records: {first value, columns}
         const int off = a.sliceOff[s0 + i];
-        int4 md = make_int4(off, (a.sliceOff[s0 + i + 1] - off) >> 5, off, 0);
-        if (LAY == 2) {
-            md.w = a.patLen[s0 + i] > 0 ? 1 : 0;
-            md.z = md.w ? a.patOff[a.patIdx[s0 + i]] : a.genOff[s0 + i];
-        }
-        meta[i] = md;
+        meta[i] = make_int2(off, (a.sliceOff[s0 + i + 1] - off) >> 5);
     }
     if (tid == 0) sRz = a.state->rz;
     __syncthreads();
     const int mat0 = ns > 0 ? meta[0].x : 0;
     const int matN = ns > 0 ? meta[ns - 1].x + 32 * meta[ns - 1].y - mat0 : 0;
-    const bool onChip = (int64_t)matN * 12 <= a.matBytes;
     uint32_t* const mc = reinterpret_cast<uint32_t*>(mv + matN);
-    // where entry j of this lane's row finds its p, in the cluster's shared memory
-    auto place = [&](const int4& md, int row, int j) {
-        int c;
-        if (LAY == 0)
-            c = a.col32[md.z + j * 32 + lane];
-        else if (LAY == 1)
-            c = min(row, a.n - 1) + a.col16[md.z + j * 32 + lane];
-        else
-            c = md.w ? row + a.pat[md.z + j] : a.gcol[md.z + j * 32 + lane];
-        return map_rank(sp + c % R, (uint32_t)(c / R));
-    };
-    if (onChip)
-        for (int ls = wid; ls < ns; ls += nw) {
-            const int4 md = meta[ls];
-            for (int j = 0; j < md.y; ++j) {
-                mv[md.x - mat0 + j * 32 + lane] = a.sval[md.x + j * 32 + lane];
-                mc[md.x - mat0 + j * 32 + lane] = place(md, row0 + ls * 32 + lane, j);
-            }
+    // where an entry's row finds its p, in the cluster's shared memory
+    for (int ls = wid; ls < ns; ls += nw) {
+        const int2 md = meta[ls];
+        const int row = min(row0 + ls * 32 + lane, a.n - 1);
+        for (int j = 0; j < md.y; ++j) {
+            const int e = md.x + j * 32 + lane, c = NARROW ? row + a.col16[e] : a.col32[e];
+            mv[e - mat0] = a.sval[e];
+            mc[e - mat0] = map_rank(sp + c % R, (uint32_t)(c / R));
         }
+    }
     const double tols = a.state->tols;
     const uint32_t maxIterP1 = a.state->maxIterP1;
     cluster_sync();
@@ -577,23 +562,18 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
         // ---- Ap = A p ----
         double dacc = 0.0;
         for (int ls = wid; ls < ns; ls += nw) {
-            const int4 md = meta[ls];
+            const int2 md = meta[ls];
             const int r = ls * 32 + lane;
             double acc = 0.0;
-            if (onChip) {
-                const int at = md.x - mat0 + lane;
-                for (int j = 0; j < md.y; j += kCols) {
-                    double xv[kCols];
+            const int at = md.x - mat0 + lane;
+            for (int j = 0; j < md.y; j += kCols) {
+                double xv[kCols];
 #pragma unroll
-                    for (int u = 0; u < kCols; ++u)
-                        if (j + u < md.y) xv[u] = ld_cluster(mc[at + (j + u) * 32]);
+                for (int u = 0; u < kCols; ++u)
+                    if (j + u < md.y) xv[u] = ld_cluster(mc[at + (j + u) * 32]);
 #pragma unroll
-                    for (int u = 0; u < kCols; ++u)
-                        if (j + u < md.y) acc = fma(mv[at + (j + u) * 32], xv[u], acc);
-                }
-            } else {
-                for (int j = 0; j < md.y; ++j)
-                    acc = fma(a.sval[md.x + j * 32 + lane], ld_cluster(place(md, row0 + r, j)), acc);
+                for (int u = 0; u < kCols; ++u)
+                    if (j + u < md.y) acc = fma(mv[at + (j + u) * 32], xv[u], acc);
             }
             if (row0 + r >= a.n) acc = 0.0;
             sz[r] = acc;
@@ -723,17 +703,17 @@ LoopShape cluster_shape(int n) {
     s.P = (nslices + ns - 1) / ns;
     s.rows = 32 * ns;
     s.threads = std::max(64, std::min(kClusterThreads, 32 * ns));
-    s.fixed = sizeof(double) * 5 * (size_t)s.rows + sizeof(int4) * (size_t)ns;
+    s.fixed = sizeof(double) * 5 * (size_t)s.rows + sizeof(int2) * (size_t)(ns + ns % 2);
     return s;
 }
 
-template <int LAY>
+template <bool NARROW>
 cudaError_t cluster_config(const LoopShape& s, size_t smem, cudaStream_t st, cudaLaunchConfig_t* cfg,
                            cudaLaunchAttribute* attr) {
-    cudaError_t e = cudaFuncSetAttribute(cg_cluster_kernel<LAY>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(cg_cluster_kernel<NARROW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)kClusterSmem);
     if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(cg_cluster_kernel<LAY>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+        e = cudaFuncSetAttribute(cg_cluster_kernel<NARROW>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     *cfg = {};
     cfg->gridDim = dim3((unsigned)s.P);
     cfg->blockDim = dim3((unsigned)s.threads);
@@ -765,8 +745,8 @@ bool device_takes_cluster() {
         cudaLaunchConfig_t cfg;
         cudaLaunchAttribute attr[1];
         int clusters = 0;
-        v = cluster_config<2>(s, kClusterSmem, nullptr, &cfg, attr) == cudaSuccess &&
-                    cudaOccupancyMaxActiveClusters(&clusters, cg_cluster_kernel<2>, &cfg) == cudaSuccess && clusters > 0
+        v = cluster_config<true>(s, kClusterSmem, nullptr, &cfg, attr) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&clusters, cg_cluster_kernel<true>, &cfg) == cudaSuccess && clusters > 0
                 ? 1
                 : 2;
         cudaGetLastError();
@@ -775,12 +755,12 @@ bool device_takes_cluster() {
     return v == 1;
 }
 
-template <int LAY>
+template <bool NARROW>
 cudaError_t cluster_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& a) {
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr[1];
-    const cudaError_t e = cluster_config<LAY>(s, a.smem, st, &cfg, attr);
-    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, cg_cluster_kernel<LAY>, a) : e;
+    const cudaError_t e = cluster_config<NARROW>(s, a.smem, st, &cfg, attr);
+    return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, cg_cluster_kernel<NARROW>, a) : e;
 }
 }  // namespace
 
@@ -790,22 +770,121 @@ cudaError_t cluster_launch(cudaStream_t st, const LoopShape& s, const LoopArgs& 
 // 9.0 / 10.7, 20^3 (272,000) 10.6 / 10.6.
 constexpr int64_t kClusterWork = 210000;
 
-bool cg_cluster_fits(int n, int64_t stored) {
+bool cg_cluster_fits(int n, int64_t stored, const LoopBalance& b) {
     if (n <= 0 || stored + 7 * (int64_t)n > kClusterWork) return false;
-    const LoopShape s = cluster_shape(n);
-    if (s.fixed + 16 * (size_t)(stored / s.P) + 1024 > kClusterSmem) return false;
+    if (cluster_shape(n).fixed + 32 * 12 * (size_t)b.clusterCols > kClusterSmem) return false;
     return device_takes_cluster();
 }
 
-cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a) {
+cudaError_t cg_cluster_launch(cudaStream_t st, bool narrow, LoopArgs a) {
     const LoopShape s = cluster_shape(a.n);
     a.nslices = (a.n + 31) / 32;
     a.rows = s.rows;
-    a.matBytes = (int)((kClusterSmem - s.fixed) / 16 * 16);
-    a.smem = s.fixed + (size_t)a.matBytes;
-    if (layout == 0) return cluster_launch<0>(st, s, a);
-    if (layout == 1) return cluster_launch<1>(st, s, a);
-    return cluster_launch<2>(st, s, a);
+    a.smem = kClusterSmem;  // whatever the matrix takes: one CTA per SM
+    return narrow ? cluster_launch<true>(st, s, a) : cluster_launch<false>(st, s, a);
+}
+
+namespace {
+// Stored columns of the CTA and of the warp that have most, in both forms, and the
+// widest slice.  One thread per CTA and warp of the grid form, then of the cluster.
+__global__ void loop_balance_kernel(int nslices, int P, int nw, int clusterSlices, int clusterWarps,
+                                    const int* __restrict__ sliceOff, LoopBalance* out) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, grid = P * nw;
+    const bool cluster = t >= grid;
+    int s0, s1, w, W;
+    if (!cluster) {
+        const int q = t / nw;
+        s0 = (int)((int64_t)nslices * q / P), s1 = (int)((int64_t)nslices * (q + 1) / P);
+        w = t % nw, W = nw;
+    } else {
+        const int q = (t - grid) / clusterWarps;
+        s0 = min(nslices, q * clusterSlices), s1 = min(nslices, s0 + clusterSlices);
+        w = (t - grid) % clusterWarps, W = clusterWarps;
+    }
+    if (s0 >= s1) return;
+    int cols = 0, widest = 0;
+    for (int s = s0 + w; s < s1; s += W) {
+        const int width = (sliceOff[s + 1] - sliceOff[s]) >> 5;
+        cols += width;
+        widest = max(widest, width);
+    }
+    atomicMax(cluster ? &out->clusterWarp : &out->gridWarp, cols);
+    if (!cluster) atomicMax(&out->widest, widest);
+    if (w == 0) {
+        const int all = (sliceOff[s1] - sliceOff[s0]) >> 5;
+        atomicMax(cluster ? &out->clusterCols : &out->gridCols, all);
+    }
+    if (t == 0) out->last = sliceOff[nslices - 1];
+}
+
+// Stored entries whose column does not follow that of the lane before: one warp
+// per slice.  A row past its last entry counts as on the diagonal.
+__global__ void loop_scattered_kernel(int n, int nslices, const int* __restrict__ rowptr, const int* __restrict__ col,
+                                      LoopBalance* out) {
+    const int lane = threadIdx.x & 31;
+    int count = 0;
+    for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < nslices; s += (gridDim.x * blockDim.x) >> 5) {
+        const int row = min(32 * s + lane, n - 1);
+        const int j0 = rowptr[row], j1 = 32 * s + lane < n ? rowptr[row + 1] : j0;
+        const int w = __reduce_max_sync(0xffffffffu, j1 - j0);
+        for (int j = 0; j < w; ++j) {
+            const int c = j0 + j < j1 ? col[j0 + j] : row;
+            const int before = __shfl_up_sync(0xffffffffu, c, 1);
+            count += lane > 0 && c != before + 1 ? 1 : 0;
+        }
+    }
+    count = __reduce_add_sync(0xffffffffu, count);
+    if (lane == 0 && count > 0) atomicAdd(&out->scattered, count);
+}
+}  // namespace
+
+cudaError_t cg_loop_balance(cudaStream_t st, int n, int numSms, int64_t stored, const int* sliceOff, const int* rowptr,
+                            const int* col, LoopBalance* out) {
+    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(LoopBalance), st);
+    if (e != cudaSuccess) return e;
+    const LoopShape g = loop_shape(n, numSms), c = cluster_shape(n);
+    const int nslices = (n + 31) / 32, threads = g.P * (g.threads / 32) + c.P * (c.threads / 32);
+    loop_balance_kernel<<<(threads + 127) / 128, 128, 0, st>>>(nslices, g.P, g.threads / 32, c.rows / 32, c.threads / 32,
+                                                              sliceOff, out);
+    if (stored + 7 * (int64_t)n <= kClusterWork)
+        loop_scattered_kernel<<<std::max(1, std::min(numSms * 4, (nslices + 3) / 4)), 128, 0, st>>>(n, nslices, rowptr,
+                                                                                                  col, out);
+    return cudaGetLastError();
+}
+
+// A lane owns a row, a CTA an equal number of slices: uneven rows make an
+// iteration as long as its longest warp (64 cycles for each column, an FMA of its
+// rows' chains) or its fullest CTA (16 cycles, the FP64 pipe).  The graph loop's
+// SpMV strides the slices over all SMs, or where the rows are uneven enough for
+// every layout to be timed (a padded copy above 1.1 of the entries) gives long rows
+// a warp or more.  The one kernel gains 5 - 10 us per iteration elsewhere, so it is
+// kept where the surplus is below that.  us per iteration, one kernel / graph, and the
+// surplus in 1,000 cycles:
+//   all layouts   20,000 rows of 129 at most 19.7 / 31.9 (2), 16^3 with a row of 120
+//                 11.6 / 17.8 (7), 2,000 of 100 - 160 19.3 / 19.5 (9), 100,000 of 4 -
+//                 60, ascending, 30.6 / 30.5 (5), 20,000 7-point with a row of 300 30.0
+//                 / 27.4 (19), 97,000 with 16 of them 33.9 / 19.0 (17), 50,000 with one of
+//                 600 50.5 / 28.5 (38), 2,000 rows of 400 - 676 51.9 / 21.3 (39)
+//   sliced only   400,000 7-point with a row of 3,000 216 / 627 (0: the graph's kernels
+//                 wait for that row too), 7-point and 27-point halves of 48^3 23.1 /
+//                 30.8 (8), 60^3 36.1 / 38.3 (15), 76^3 60.3 / 58.7 (29), 648,000
+//                 7-point and 64,000 27-point rows 51.9 / 41.4 (42)
+// The cluster or the grid: a scattered entry costs the cluster 4.5 cycles of its
+// CTA, a column of the longest warp the grid about 130; and the cluster's fullest CTA
+// must not lag behind the grid's by more than the 2 us that it gains.  Cluster / grid,
+// random rows: 500 of 100 (47,000 scattered) 12.3 / 18.2, 1,000 of 32 (34,000) 9.6 /
+// 11.5, of 64 (65,000) 14.8 / 14.0, 2,000 of 16 (36,000) 9.6 / 10.0, of 32 (68,000)
+// 14.8 / 11.4, 4,000 of 32 (135,000) 27.5 / 12.0 (graph 17.5); 27-point 16^3 in
+// random order (102,000) 21.4 / 10.7, in grid order (15,000) 7.6 / 10.6.
+int cg_loop_form(int n, int numSms, int64_t stored, bool allLayouts, const LoopBalance& b) {
+    if (!cg_loop_fits(n, numSms)) return 0;
+    const int64_t cols = stored / 32, even = 16 * cols / numSms;
+    const int64_t grid = std::max<int64_t>(16ll * b.gridCols, 64ll * b.gridWarp);
+    const int64_t cluster = std::max<int64_t>(16ll * b.clusterCols, 64ll * b.clusterWarp);
+    const int64_t graph = allLayouts ? even : std::max<int64_t>(even, 64ll * b.widest);
+    if (grid > graph + (allLayouts ? 8000 : 20000)) return 0;
+    if (b.scattered > 27000 + 460 * b.gridWarp || cluster > grid + 16 * cols / kClusterMax + 4000) return 1;
+    return cg_cluster_fits(n, stored, b) ? 2 : 1;
 }
 
 // The vectors have to fit in shared memory, all but J (1,065,216 rows on 152 SMs; J too up to 856,064).

@@ -767,10 +767,20 @@ bool PcgHandle::ensureSell() {
           "sliced layout");
     // Padding of the phantom rows past n in the last slice is a fixed cost
     // and does not count against the layout.
-    int lastOff = 0;
-    check(cudaMemcpyAsync(&lastOff, m_sliceOff.as<int>() + nslices - 1, sizeof(int), cudaMemcpyDeviceToHost, m_stream),
-          "D2H");
+    m_loopBalance = LoopBalance();
+    if (cg_loop_fits((int)m_n, m_numSms)) {
+        alloc(m_balance, sizeof(LoopBalance), "slice balance");
+        check(cg_loop_balance(m_stream, (int)m_n, m_numSms, total, m_sliceOff.as<int>(), m_rowptr.as<int>(),
+                              m_col.as<int>(), m_balance.as<LoopBalance>()),
+              "slice balance");
+        check(cudaMemcpyAsync(&m_loopBalance, m_balance.p, sizeof(LoopBalance), cudaMemcpyDeviceToHost, m_stream), "D2H");
+    } else {
+        check(cudaMemcpyAsync(&m_loopBalance.last, m_sliceOff.as<int>() + nslices - 1, sizeof(int),
+                              cudaMemcpyDeviceToHost, m_stream),
+              "D2H");
+    }
     check(cudaStreamSynchronize(m_stream), "sync");
+    const int lastOff = m_loopBalance.last;
     const int64_t phantom = (int64_t)(nslices * 32 - (int64_t)m_n) * ((total - lastOff) / 32);
     m_sellPadRatio = (double)(total - phantom) / (double)std::max<uint64_t>(m_nnz, 1);
     if ((uint64_t)(total - phantom) > m_nnz + m_nnz / 2 + 64 || total > 0x7fffff00ll) {
@@ -1077,6 +1087,10 @@ int PcgHandle::loopKernel(uint32_t maxIter, int* layout) {
     if (!m_useGraph || !m_fusedUpdate || m_loopKernelEnv == 0 || maxIter > 0xfffffff0u) return 0;
     if (forced && (m_loopKernelEnv != 1 || !(isSell(m_spmvCfg) || isPat(m_spmvCfg)))) return 0;
     if (!cg_loop_fits((int)m_n, m_numSms) || !ensureSell()) return 0;  // too large, or rows too uneven
+    // timeConfigs() times more than the sliced kernels where the copy pads more than 10 %
+    int form = cg_loop_form((int)m_n, m_numSms, m_sellTotal, m_sellPadRatio > 1.1, m_loopBalance);
+    if (form == 0 && !forced) return 0;
+    if (form == 0) form = 1;
     // Gathers that are not coalesced want the graph loop's 48 warps per SM and L1
     // once the vectors take most of the shared memory.  Random columns, us per
     // iteration (this kernel / graph loop): 200,000 rows of 14 25.7 / 34.4, 500,000
@@ -1088,7 +1102,8 @@ int PcgHandle::loopKernel(uint32_t maxIter, int* layout) {
         *layout = isPat(m_spmvCfg) ? 2 : (isSellNarrow(m_spmvCfg) ? 1 : 0);
     else
         *layout = m_psState == 1 ? 2 : (m_sellNarrow ? 1 : 0);
-    return !m_faultCluster && cg_cluster_fits((int)m_n, m_sellTotal) ? 2 : 1;
+    if (form == 2 && m_faultCluster) form = 1;
+    return form;
 }
 
 // One launch for the vector init, one for the loop.
@@ -1119,7 +1134,9 @@ void PcgHandle::launchLoopKernel(int form, int layout, uint32_t maxIter) {
     a.J = m_J.as<double>();
     a.state = st;
     if (form == 2) {
-        check(cg_cluster_launch(m_stream, layout, a), "cluster loop kernel");
+        a.sliceOff = m_sliceOff.as<int>();
+        a.sval = m_sellVal.as<double>();
+        check(cg_cluster_launch(m_stream, m_sellNarrow, a), "cluster loop kernel");
         return;
     }
     a.tag0 = m_loopTag;

@@ -311,6 +311,8 @@ class PcgHandle {
     DevBuf m_b, m_diag, m_x, m_r, m_p, m_J, m_Ap;
     DevBuf m_state, m_partials, m_records;
     uint64_t m_recCap = 0;
+    DevBuf m_balance;             // of the sliced copy, on the device
+    LoopBalance m_loopBalance{};  // and here
     DevBuf m_loopSync;       // counters and posts of the persistent loop kernel
     uint32_t m_loopTag = 0;  // next unused tag; 0: m_loopSync is to be cleared
     DevBuf m_scratchY;

@@ -186,17 +186,30 @@ struct LoopArgs {
     CgState* state = nullptr;
 
     uint32_t tag0 = 0;  // tags tag0 .. tag0 + iterations - 1 are this launch's own
-    // set by cg_loop_launch
-    int nslices = 0, rows = 0, matBytes = 0;
+    // set by cg_loop_launch and cg_cluster_launch
+    int nslices = 0, rows = 0;
     size_t smem = 0;
     uint32_t* counters = nullptr;
     ulonglong2* posts = nullptr;
     int jOnChip = 0;
 };
-bool cg_loop_fits(int n, int numSms);  // the grid form
+// How a sliced copy's columns (slice widths) spread over the kernels' CTAs and warps.
+struct LoopBalance {
+    int last;                      // offset of the last slice
+    int widest;                    // columns of the widest slice
+    int gridCols, gridWarp;        // grid form: most columns of a CTA, of a warp
+    int clusterCols, clusterWarp;  // the same in the cluster form
+    int scattered;                 // entries whose column does not follow the lane before's (small systems only)
+};
+bool cg_loop_fits(int n, int numSms);  // the grid form's vectors fit on the chip
+cudaError_t cg_loop_balance(cudaStream_t st, int n, int numSms, int64_t stored, const int* sliceOff, const int* rowptr,
+                            const int* col, LoopBalance* out);
+// Which form suits the matrix: 0 none, 1 over the grid, 2 in one cluster.
+// allLayouts: the graph loop's SpMV could be one that is not sliced.
+int cg_loop_form(int n, int numSms, int64_t stored, bool allLayouts, const LoopBalance& b);
 // the same in one cluster of up to 16 CTAs, for small systems
-bool cg_cluster_fits(int n, int64_t stored);
-cudaError_t cg_cluster_launch(cudaStream_t st, int layout, LoopArgs a);
+bool cg_cluster_fits(int n, int64_t stored, const LoopBalance& b);
+cudaError_t cg_cluster_launch(cudaStream_t st, bool narrow, LoopArgs a);  // plain sliced copy
 size_t cg_loop_sync_bytes(int numSms);
 // stored: entries of the layout; layout: 0 sliced with int32 columns, 1 int16 offsets, 2 slice-shared
 // offsets; sync: cg_loop_sync_bytes bytes, the first 512 cleared before each launch.
