@@ -490,15 +490,20 @@ void PcgHandle::refreshSellValues() {
 }
 
 // Configuration index space: [0, ncsr) staged CSR shapes, [ncsr, ncsr +
-// nsell) sliced unroll depths, then the sorted-sliced unroll depths, then the
-// merge-path kernel.
-int PcgHandle::numSpmvCfgs() const { return mergeCfg() + 1; }
+// nsell) sliced unroll depths, then the shared-offset ones, the first sorted-sliced
+// ones, the merge-path kernel, and the sorted-sliced ones that came after it.
+static constexpr int kSortedBeforeMerge = 2;
+
+int PcgHandle::numSpmvCfgs() const { return mergeCfg() + 1 + sellsort_num_configs() - kSortedBeforeMerge; }
 
 int PcgHandle::patCfg0() const { return spmv_num_configs() + sell_num_configs(); }
 
 int PcgHandle::sortedCfg0() const { return patCfg0() + sellpat_num_configs(); }
 
-int PcgHandle::mergeCfg() const { return sortedCfg0() + sellsort_num_configs(); }
+int PcgHandle::mergeCfg() const { return sortedCfg0() + kSortedBeforeMerge; }
+
+// The configuration among the sorted-sliced ones.
+int PcgHandle::sortedIndex(int cfg) const { return cfg - sortedCfg0() - (cfg > mergeCfg() ? 1 : 0); }
 
 bool PcgHandle::isSell(int cfg) const {
     return cfg >= spmv_num_configs() && cfg < spmv_num_configs() + sell_num_configs();
@@ -507,10 +512,10 @@ bool PcgHandle::isSell(int cfg) const {
 bool PcgHandle::isSellNarrow(int cfg) const { return isSell(cfg) && sell_config_narrow(cfg - spmv_num_configs()); }
 
 int PcgHandle::sortedHubs(int cfg) const {
-    return sellsort_config_unroll(cfg - sortedCfg0()) == 8 ? m_ssHubs : 0;
+    return sellsort_config_hubs(sortedIndex(cfg)) ? m_ssHubs : 0;
 }
 
-bool PcgHandle::isSorted(int cfg) const { return cfg >= sortedCfg0() && cfg < mergeCfg(); }
+bool PcgHandle::isSorted(int cfg) const { return cfg >= sortedCfg0() && cfg < numSpmvCfgs() && cfg != mergeCfg(); }
 
 bool PcgHandle::isPat(int cfg) const { return cfg >= patCfg0() && cfg < sortedCfg0(); }
 
@@ -667,7 +672,7 @@ int PcgHandle::spmvGrid64(int cfg) {
         return merge_tiles((int)m_n, (int64_t)m_nnz);
     }
     if (isSorted(cfg))
-        return ensureSorted() ? sellsort_grid<double>(cfg - sortedCfg0(), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
+        return ensureSorted() ? sellsort_grid<double>(sortedIndex(cfg), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
     if (isPat(cfg)) return ensurePat() ? sellpat_grid<double>(cfg - patCfg0(), (int)m_n, m_numSms) : 0;
     if (!isSell(cfg)) return spmv_grid<double>(cfg, (int)m_n, m_numSms);
     if (!ensureSell() || (isSellNarrow(cfg) && !m_sellNarrow)) return 0;
@@ -680,7 +685,7 @@ int PcgHandle::spmvGrid32(int cfg) {
         return merge_tiles((int)m_n, (int64_t)m_nnz);
     }
     if (isSorted(cfg))
-        return ensureSorted() ? sellsort_grid<float>(cfg - sortedCfg0(), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
+        return ensureSorted() ? sellsort_grid<float>(sortedIndex(cfg), (int)m_n, m_ssLong, sortedHubs(cfg), m_numSms) : 0;
     if (isPat(cfg)) return ensurePat() ? sellpat_grid<float>(cfg - patCfg0(), (int)m_n, m_numSms) : 0;
     if (!isSell(cfg)) return spmv_grid<float>(cfg, (int)m_n, m_numSms);
     if (!ensureSell() || (isSellNarrow(cfg) && !m_sellNarrow)) return 0;
@@ -710,7 +715,7 @@ cudaError_t PcgHandle::spmv64(int cfg, int grid, const double* x, double* y, con
                                            m_psVal.as<double>(), x, y, b, st, part, mode, done);
     if (isSorted(cfg))
         return spmv_sellsort_launch<double>(
-            cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
+            sortedIndex(cfg), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
             (sortedHubs(cfg) > 0 ? m_ssHubScol : m_ssCol).as<int>(), m_ssVal.as<double>(), m_rowptr.as<int>(),
             (sortedHubs(cfg) > 0 ? m_ssHubCol : m_col).as<int>(), m_val.as<double>(), x, y, b, sortedHubs(cfg),
             m_ssHubX.as<double>(), st, part, mode, done);
@@ -740,7 +745,7 @@ cudaError_t PcgHandle::spmv32(int cfg, int grid, const float* x, float* y, const
                                           m_psVal32.as<float>(), x, y, b, st, part, mode, done);
     if (isSorted(cfg))
         return spmv_sellsort_launch<float>(
-            cfg - sortedCfg0(), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
+            sortedIndex(cfg), grid, m_stream, (int)m_n, m_ssLong, m_ssSorted.as<int>(), m_ssSliceOff.as<int>(),
             (sortedHubs(cfg) > 0 ? m_ssHubScol : m_ssCol).as<int>(), m_ssVal32.as<float>(), m_rowptr.as<int>(),
             (sortedHubs(cfg) > 0 ? m_ssHubCol : m_col).as<int>(), m_val32.as<float>(), x, y, b, sortedHubs(cfg),
             m_ssHubX.as<float>(), st, part, mode, done);
@@ -2421,7 +2426,7 @@ int PcgHandle::tuning(float* ms, int* shape, int cap) const {
             // length-sorted sliced layout: (1, 1, unroll, 32)
             shape[4 * c] = 1;
             shape[4 * c + 1] = 1;
-            shape[4 * c + 2] = sellsort_config_unroll(c - sortedCfg0());
+            shape[4 * c + 2] = sellsort_config_unroll(sortedIndex(c));
             shape[4 * c + 3] = 32;
         } else if (isSell(c)) {
             // sliced layout: one lane per row, no CTA staging; chunk = unroll,

@@ -275,6 +275,7 @@ class PcgHandle {
     int64_t m_ssTotal = 0;
     DevBuf m_ssHubOf, m_ssHubCol, m_ssHubScol, m_ssHubX;
     int m_ssHubs = 0;  // columns whose x the unroll of 8 reads from a compact copy
+    int sortedIndex(int cfg) const;
     int sortedHubs(int cfg) const;
     void buildHubs(int nLong, int64_t total);
     bool m_ss32Valid = false;

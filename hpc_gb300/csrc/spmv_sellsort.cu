@@ -31,8 +31,11 @@
 // leaves too few warps, and L1 eviction hints (hubs last, others not at all) were
 // better below 500,000 rows only (71 at 300,007, 375 at 2M: two loads per gather,
 // 128 registers).
-// Neither loop over a row's steps is unrolled further: left to the compiler, the
-// unroll of 4 took 55, 101, 204 and 342 us.
+// Neither loop over a row's steps is unrolled further, and six CTAs per SM (five with
+// hubs) are asked for.  FREE leaves both to the compiler, which is slower on Zipf rows
+// (unroll of 4: 55, 101, 204 and 342 us; 400,000 rows 92, 78 without) and faster on even
+// random ones (800,000 rows of 4 - 20, unroll of 8 46.8, 49.0 without; 200,000 of 10
+// - 120 in FP32 46.6 and 47.1): two configurations more for the tuner.
 //
 // Work items, in warp-stride order: the long rows (one warp each), then the
 // slices (one lane per row).  kCgDot / kResidual reduce through the same
@@ -185,8 +188,8 @@ __global__ void ss_hub_x_kernel(int nHubs, const int* __restrict__ sorted, const
     if (i < nHubs) hubX[i] = x[sorted[i]];
 }
 
-template <typename VT, int U, bool HUB>
-__global__ void __launch_bounds__(kSortThreads, HUB ? 5 : 6) spmv_sellsort_kernel(
+template <typename VT, int U, bool HUB, bool FREE>
+__global__ void __launch_bounds__(kSortThreads, HUB ? 5 : (FREE ? 0 : 6)) spmv_sellsort_kernel(
     int n, int nLong, int nSlices, const int* __restrict__ sorted, const int* __restrict__ sliceOff,
     const int* __restrict__ scol, const VT* __restrict__ sval, const int* __restrict__ rowptr,
     const int* __restrict__ col, const VT* __restrict__ val, const VT* __restrict__ x, VT* __restrict__ y,
@@ -206,17 +209,31 @@ __global__ void __launch_bounds__(kSortThreads, HUB ? 5 : 6) spmv_sellsort_kerne
             row = sorted[w];
             const int j0 = rowptr[row], j1 = rowptr[row + 1];
             int j = j0 + lane;
-#pragma unroll 1
-            for (; j + 32 * (U - 1) < j1; j += 32 * U) {
-                VT v[U];
-                int c[U];
+            if constexpr (FREE) {
+                for (; j + 32 * (U - 1) < j1; j += 32 * U) {
+                    VT v[U];
+                    int c[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    v[u] = __ldcs(&val[j + 32 * u]);
-                    c[u] = __ldcs(&col[j + 32 * u]);
+                    for (int u = 0; u < U; ++u) {
+                        v[u] = __ldcs(&val[j + 32 * u]);
+                        c[u] = __ldcs(&col[j + 32 * u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
                 }
+            } else {
+#pragma unroll 1
+                for (; j + 32 * (U - 1) < j1; j += 32 * U) {
+                    VT v[U];
+                    int c[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
+                    for (int u = 0; u < U; ++u) {
+                        v[u] = __ldcs(&val[j + 32 * u]);
+                        c[u] = __ldcs(&col[j + 32 * u]);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
+                }
             }
             for (; j < j1; j += 32) acc = fma((AccT)__ldcs(&val[j]), (AccT)gather<VT, HUB>(x, hubX, __ldcs(&col[j])), acc);
             acc = warp_sum(acc);
@@ -231,17 +248,31 @@ __global__ void __launch_bounds__(kSortThreads, HUB ? 5 : 6) spmv_sellsort_kerne
             const VT* vp = sval + off + lane;
             const int* cp = scol + off + lane;
             int j = 0;
-#pragma unroll 1
-            for (; j + U <= len; j += U) {
-                VT v[U];
-                int c[U];
+            if constexpr (FREE) {
+                for (; j + U <= len; j += U) {
+                    VT v[U];
+                    int c[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) {
-                    v[u] = __ldcs(vp + (j + u) * 32);
-                    c[u] = __ldcs(cp + (j + u) * 32);
+                    for (int u = 0; u < U; ++u) {
+                        v[u] = __ldcs(vp + (j + u) * 32);
+                        c[u] = __ldcs(cp + (j + u) * 32);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
                 }
+            } else {
+#pragma unroll 1
+                for (; j + U <= len; j += U) {
+                    VT v[U];
+                    int c[U];
 #pragma unroll
-                for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
+                    for (int u = 0; u < U; ++u) {
+                        v[u] = __ldcs(vp + (j + u) * 32);
+                        c[u] = __ldcs(cp + (j + u) * 32);
+                    }
+#pragma unroll
+                    for (int u = 0; u < U; ++u) acc = fma((AccT)v[u], (AccT)gather<VT, HUB>(x, hubX, c[u]), acc);
+                }
             }
             for (; j < len; ++j) acc = fma((AccT)__ldcs(vp + j * 32), (AccT)gather<VT, HUB>(x, hubX, __ldcs(cp + j * 32)), acc);
             if (row < 0) continue;
@@ -276,8 +307,9 @@ __global__ void __launch_bounds__(kSortThreads, HUB ? 5 : 6) spmv_sellsort_kerne
 }
 
 // ---- host side ----
-int sellsort_num_configs() { return 2; }
-int sellsort_config_unroll(int cfg) { return cfg == 0 ? 4 : 8; }
+int sellsort_num_configs() { return 4; }
+int sellsort_config_unroll(int cfg) { return cfg % 2 == 0 ? 4 : 8; }
+bool sellsort_config_hubs(int cfg) { return cfg == 1; }
 
 int sellsort_tiles(int n) { return (n + kTileRows - 1) / kTileRows; }
 int sellsort_bins() { return kBins; }
@@ -330,10 +362,10 @@ cudaError_t sellsort_fill(cudaStream_t st, int n, int nLong, const int* rowptr, 
 }
 
 namespace {
-template <typename VT, int U, bool HUB>
+template <typename VT, int U, bool HUB, bool FREE>
 int ss_bps() {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmv_sellsort_kernel<VT, U, HUB>, kSortThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, spmv_sellsort_kernel<VT, U, HUB, FREE>, kSortThreads, 0) !=
         cudaSuccess)
         return 0;
     return nb;
@@ -342,8 +374,13 @@ int ss_bps() {
 
 template <typename VT>
 int sellsort_grid(int cfg, int n, int nLong, int nHubs, int numSms) {
-    const int bps = sellsort_config_unroll(cfg) == 4 ? ss_bps<VT, 4, false>()
-                                                     : (nHubs > 0 ? ss_bps<VT, 8, true>() : ss_bps<VT, 8, false>());
+    int bps;
+    if (cfg == 0)
+        bps = ss_bps<VT, 4, false, false>();
+    else if (cfg == 1)
+        bps = nHubs > 0 ? ss_bps<VT, 8, true, false>() : ss_bps<VT, 8, false, false>();
+    else
+        bps = cfg == 2 ? ss_bps<VT, 4, false, true>() : ss_bps<VT, 8, false, true>();
     if (bps <= 0) return 0;
     const int items = nLong + (n - nLong + 31) / 32;
     const int need = (items + kSortThreads / 32 - 1) / (kSortThreads / 32);
@@ -374,18 +411,22 @@ cudaError_t spmv_sellsort_launch(int cfg, int grid, cudaStream_t st, int n, int 
                                  CgState* state, double* partials, int mode, const uint32_t* doneFlag) {
     if (n <= 0) return cudaSuccess;
     const int nSlices = (n - nLong + 31) / 32;
-    if (sellsort_config_unroll(cfg) == 4) nHubs = 0;
+    if (!sellsort_config_hubs(cfg)) nHubs = 0;
     if (nHubs > 0) ss_hub_x_kernel<VT><<<(nHubs + 127) / 128, 128, 0, st>>>(nHubs, sorted, x, hubX, doneFlag);
     auto go = [&](auto kernel) {
         kernel<<<grid, kSortThreads, 0, st>>>(n, nLong, nSlices, sorted, sliceOff, scol, sval, rowptr, col, val, x, y,
                                               b, hubX, state, partials, mode, doneFlag);
     };
-    if (sellsort_config_unroll(cfg) == 4)
-        go(spmv_sellsort_kernel<VT, 4, false>);
-    else if (nHubs > 0)
-        go(spmv_sellsort_kernel<VT, 8, true>);
+    if (cfg == 0)
+        go(spmv_sellsort_kernel<VT, 4, false, false>);
+    else if (cfg == 1 && nHubs > 0)
+        go(spmv_sellsort_kernel<VT, 8, true, false>);
+    else if (cfg == 1)
+        go(spmv_sellsort_kernel<VT, 8, false, false>);
+    else if (cfg == 2)
+        go(spmv_sellsort_kernel<VT, 4, false, true>);
     else
-        go(spmv_sellsort_kernel<VT, 8, false>);
+        go(spmv_sellsort_kernel<VT, 8, false, true>);
     return cudaGetLastError();
 }
 

@@ -110,6 +110,7 @@ cudaError_t fp64_rate_launch(cudaStream_t st, int grid, int iters, double* out);
 // ---- length-sorted sliced SpMV (spmv_sellsort.cu) ----
 int sellsort_num_configs();
 int sellsort_config_unroll(int cfg);
+bool sellsort_config_hubs(int cfg);  // reads x of the hub columns from a copy, where there are any
 int sellsort_tiles(int n);
 int sellsort_bins();
 // hist/start: sellsort_bins() * sellsort_tiles(n) ints each; sorted: n ints.

@@ -69,3 +69,21 @@ def test_without_memory_for_hub_columns_the_solve_goes_on(gpu_lib, monkeypatch):
             assert m.status == X.SUCCESS, m.message
             out[fault] = h.spmv(x)
     assert np.array_equal(out[""], out["hubs"])
+
+
+@pytest.mark.parametrize("n", [3001, 50001])
+def test_loops_left_to_the_compiler_give_the_same_bits(gpu_lib, n):
+    # the last two configurations of the table, after the merge path's
+    s = W.zipf_spd(n, hi=1500, seed=n)
+    x = np.random.default_rng(3).uniform(-1.0, 1.0, n)
+    with X.JPCG() as h:
+        h.csr_solve(n, s.rowptr, s.col, s.val, s.diag, s.b, 1, 1e-10)
+        shapes = [t[:4] for t in h.spmv_tuning()]
+        depths = {u: [c for c, t in enumerate(shapes) if t == (1, 1, u, 32)] for u in (4, 8)}
+        assert [c for u in (4, 8) for c in depths[u]][1::2] == [len(shapes) - 2, len(shapes) - 1]
+        for u in (4, 8):
+            y = []
+            for c in depths[u]:
+                h.set_spmv_config(c)
+                y.append(h.spmv(x))
+            assert np.array_equal(y[0], y[1])
