@@ -239,30 +239,24 @@ struct BatchResult {      // layout of XJPCG_GbBatchResult_t
     double res;           // fp64: sqrt(r.r / b.b) of the recursive residual; mixed: true residual
 };
 struct BatchLaunch {
-    int nsys;
-    const int* sysRow;
-    const int* order;
-    const int* rowptr;
-    const int* col;
-    const double* val;
-    const float* val32;
-    const double* b;
-    const double* diag;
-    double* x;
-    double* r;
-    double* Ap;
-    double* J;
-    float* r32;
-    float* d32;
-    float* Ap32;
-    float* J32;
-    double* pGlobal;
-    float* p32Global;
-    BatchResult* res;
-    uint32_t* queue;
-    uint32_t maxIterP1;
-    double tol;
-    double delta2;  // mixed: reliable-update threshold, squared
+    int nsys = 0;
+    const int* sysRow = nullptr;
+    const int* order = nullptr;
+    const int* rowptr = nullptr;
+    const int* col = nullptr;
+    const double* val = nullptr;
+    const float* val32 = nullptr;  // mixed CSR kernels (null: not built)
+    const double* b = nullptr;
+    const double* diag = nullptr;
+    double *x = nullptr, *r = nullptr, *Ap = nullptr, *J = nullptr;
+    float *r32 = nullptr, *d32 = nullptr, *Ap32 = nullptr, *J32 = nullptr;
+    double* pGlobal = nullptr;
+    float* p32Global = nullptr;
+    BatchResult* res = nullptr;
+    uint32_t* queue = nullptr;
+    uint32_t maxIterP1 = 0;
+    double tol = 0.0;
+    double delta2 = 0.0;  // mixed: reliable-update threshold, squared
     // per-system SELL-32 copy for the sliced kernels (null: not built)
     const int* sliceBase = nullptr;
     const int* sliceOff = nullptr;
