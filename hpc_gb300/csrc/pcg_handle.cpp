@@ -2284,18 +2284,39 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
                 for (int teams : {2, 4, 8})
                     if (batch_team_clusters(mixed, teams, rows) > 0) teamShapes.emplace_back(rows, teams);
         const bool teamsOnly = teamsEnv == 1 && !teamShapes.empty();
-        for (size_t si = 0; si < smemRows.size(); ++si)
+        int c512 = 0, csr2 = 0, c128 = 0;  // 512 threads, sliced; CSR: 256 threads, two lanes a row; 128 threads
+        for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
+            batch_config_shape(c, &t, &g);
+            if (batch_config_sliced(c) && t == 512) c512 = c;
+            if (!batch_config_sliced(c) && t == 256 && g == 2) csr2 = c;
+            if (!batch_config_sliced(c) && t == 128) c128 = c;
+        }
+        // From shared memory first: where the usual choices among the others take 1.3
+        // times as long, the rest is not timed (270 systems of 1,000 - 18,630 rows: 3
+        // solves of 20 - 25 ms instead of 20).
+        float clusterMs = 1e30f;
+        bool all = true;
+        if (clusters.offered) {
+            float ms = 0, unused = -1.f;
+            runClusters(in, clusters, maxIter, tol, mixed, &ms);
+            clusterMs = ms;
+            const size_t last = (smemRows.size() - 1) * ncfg;
+            for (int c : {c512, csr2, c128}) {
+                if ((c == c512 && !sliced) || (c == c128 && maxN > 2048) || teamsOnly) continue;
+                if (best > 1.3f * clusterMs) consider(c, smemRows.back(), 0, &m_batchTuneMs[last + c]);
+            }
+            for (const auto& t : teamShapes)
+                if (best > 1.3f * clusterMs && t.second == 4) consider(c512, t.first, t.second, &unused);
+            all = best <= 1.3f * clusterMs;
+        }
+        for (size_t si = 0; si < smemRows.size() && all; ++si)
             for (int c = 0; c < ncfg; ++c) {
                 if (batch_config_sliced(c) != sliced || teamsOnly) continue;
                 consider(c, smemRows[si], 0, &m_batchTuneMs[si * ncfg + c]);
             }
-        int c512 = 0;
-        for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
-            batch_config_shape(c, &t, &g);
-            if (batch_config_sliced(c) && t == 512) c512 = c;
-        }
         float unused = -1.f;
-        for (const auto& t : teamShapes) consider(c512, t.first, t.second, &unused);
+        for (const auto& t : teamShapes)
+            if (all) consider(c512, t.first, t.second, &unused);
         // CSR shapes win on uneven rows (two lanes a row) and on systems of one to a
         // few slices (128 threads): kernel ms, fp64 / mixed, sliced against CSR, 600
         // systems of 3,000 rows of Zipf length 9.2 / 7.0 against 4.7 / 3.5, 600 of
@@ -2304,7 +2325,7 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
         // 1.4 / 1.5; on larger stencil systems they take 1.1 to 1.9 times as long.
         // The winner is one of these two or close to it, so the other four are timed
         // only where one of the two comes within 1.2 of the best.
-        if (sliced && !teamsOnly) {
+        if (sliced && !teamsOnly && all) {
             const int rows = plan.smemRows;
             const size_t si = std::find(smemRows.begin(), smemRows.end(), rows) - smemRows.begin();
             const float sliceBest = best;
@@ -2312,19 +2333,16 @@ uint32_t PcgHandle::batchSolve(uint32_t nsys, const int32_t* sysRow, const int32
             for (int pass = 0; pass < 2 && (pass == 0 || csrBest <= 1.2f * sliceBest); ++pass)
                 for (int c = 0, t = 0, g = 0; c < ncfg; ++c) {
                     batch_config_shape(c, &t, &g);
-                    const bool first = (t == 256 && g == 2) || t == 128;
+                    const bool first = c == csr2 || c == c128;
                     if (batch_config_sliced(c) || first != (pass == 0)) continue;
+                    if (c == c128 && maxN > 2048) continue;  // too few threads for such a system
                     float ms = -1.f;
                     consider(c, rows, 0, &ms);
                     if (si < smemRows.size()) m_batchTuneMs[si * ncfg + c] = ms;
                     csrBest = std::min(csrBest, ms);
                 }
         }
-        if (clusters.offered) {
-            float ms = 0;
-            runClusters(in, clusters, maxIter, tol, mixed, &ms);
-            plan.clusters = ms <= best;
-        }
+        plan.clusters = clusters.offered && clusterMs <= best;
         m_batchPlan = plan;
         m_batchKey = key;
     }
