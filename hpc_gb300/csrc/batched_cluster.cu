@@ -37,44 +37,23 @@ constexpr int kInfoLocal = 1 << 17;   // every column of the slice lies in this 
 constexpr uint64_t kBcWaitNs = 2000000000ull;  // 2 s
 constexpr uint32_t kBatchLost = 2;             // status of a system whose CTAs lost one another
 
-__device__ __forceinline__ void bc_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
 // All threads that work on the system.
 template <bool MULTI>
 __device__ __forceinline__ void system_sync() {
     if (MULTI)
-        bc_cluster_sync();
+        cluster_sync();
     else
         __syncthreads();
 }
 
-__device__ __forceinline__ uint32_t bc_map(const void* p, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
-    return a;
-}
 __device__ __forceinline__ double bc_load(const double* p, uint32_t rank) {
     double v;
-    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(bc_map(p, rank)));
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(cluster_addr(p, rank)));
     return v;
 }
 __device__ __forceinline__ float bc_load(const float* p, uint32_t rank) {
     float v;
-    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(bc_map(p, rank)));
-    return v;
-}
-
-__device__ __forceinline__ int bc_warp_min(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-__device__ __forceinline__ int bc_warp_max(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(cluster_addr(p, rank)));
     return v;
 }
 
@@ -106,7 +85,7 @@ __device__ void load_rows(const Rows<VT>& s, const int* __restrict__ rowptr, con
         int cur = q < j1 ? col[q] - row : INT_MAX;
         const int most = min(kBatchPatMax, s.w);
         while (ok) {
-            const int m = bc_warp_min(cur);
+            const int m = warp_min(cur);
             if (m == INT_MAX) break;
             if (L == most || first + m < 0 || first + 31 + m >= s.n) {
                 ok = false;
@@ -136,7 +115,7 @@ __device__ void load_rows(const Rows<VT>& s, const int* __restrict__ rowptr, con
             const bool local = first + lo >= s.row0 && first + 31 + hi < s.row0 + s.R;
             if (lane == 0) s.info[ls] = L | kInfoShared | (local ? kInfoLocal : 0);
         } else {
-            const int w = bc_warp_max(j1 - j0);
+            const int w = warp_max(j1 - j0);
             bool local = true;
             for (int k = 0; k < w; ++k) {
                 const bool has = j0 + k < j1;
@@ -213,12 +192,12 @@ struct SumBox {
 template <typename T>
 __device__ __forceinline__ void post(T* slot, uint64_t* bar, uint32_t rank, T v) {
     if constexpr (sizeof(T) == 8)
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(bc_map(slot, rank)),
-                     "l"(__double_as_longlong(v)), "r"(bc_map(bar, rank))
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(cluster_addr(slot, rank)),
+                     "l"(__double_as_longlong(v)), "r"(cluster_addr(bar, rank))
                      : "memory");
     else
-        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(bc_map(slot, rank)),
-                     "r"(__float_as_uint(v)), "r"(bc_map(bar, rank))
+        asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(cluster_addr(slot, rank)),
+                     "r"(__float_as_uint(v)), "r"(cluster_addr(bar, rank))
                      : "memory");
 }
 
@@ -281,7 +260,7 @@ __device__ __forceinline__ T system_sum(const T (&v)[NV], SumBox<NT, T, NV>& box
                 lost.parity = parity;
                 lost.late = &box.bar;
                 if (lane < C)
-                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(bc_map(&lost.mark, (uint32_t)lane)), "r"(next)
+                    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(&lost.mark, (uint32_t)lane)), "r"(next)
                                  : "memory");
             }
             t = warp_sum(lane < C ? box.slots[wid][lane] : T(0));
@@ -338,7 +317,7 @@ __global__ void __launch_bounds__(NT, NT > 256 ? 2 : 5) batch_cluster_fp64_kerne
             mbar_init(&boxB.bar, 1);
             mbar_fence_init();
         }
-        bc_cluster_sync();
+        cluster_sync();
     }
     // r = b, J = 1 / diag, p = J r, x = 0 (cgVector.hpp:101-114)
     double r[K], x[K], J[K], p[K], z[K];
@@ -468,7 +447,7 @@ __global__ void __launch_bounds__(NT, NT > 128 ? 3 : 6) batch_cluster_mixed_kern
             mbar_init(&boxB.bar, 1);
             mbar_fence_init();
         }
-        bc_cluster_sync();
+        cluster_sync();
     }
     double* const xs = a.x + r0;  // the system's x
     double* const x = xs + s.row0;

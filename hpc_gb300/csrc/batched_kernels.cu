@@ -80,7 +80,8 @@ struct BatchArgs {
 };
 
 // The rows of a system that a CTA works on: all of them, or in the team kernels
-// (TEAM) its share of whole slices.
+// (TEAM) its share of whole slices.  Teams take systems above 2,048 rows, so that each
+// of at most 8 CTAs has some.
 struct Share {
     int lo, hi;  // rows
     int q, C;    // rank and size of the team
@@ -102,20 +103,17 @@ __device__ __forceinline__ Share share_of(int n, int C) {
 // memory before it is visible to them after.
 template <bool TEAM>
 __device__ __forceinline__ void team_barrier() {
-    if (TEAM) {
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    } else {
+    if (TEAM)
+        cluster_sync();
+    else
         __syncthreads();
-    }
 }
 
 // v into the same place of every CTA of the team (lanes of one warp).
 template <typename P, typename T>
 __device__ __forceinline__ void team_post(P* place, T v, int C, int lane) {
     if (lane < C) {
-        uint32_t a;
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(place)), "r"(lane));
+        const uint32_t a = cluster_addr(place, (uint32_t)lane);
         if (sizeof(T) == 8)
             asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"((double)v) : "memory");
         else
@@ -441,6 +439,13 @@ __device__ __forceinline__ void block_allreduce(T (&v)[NV]) {
         block_allsum<NT, NV, T>(v);
 }
 
+// Space for the threads' values, one for all sums of NV doubles in a kernel.
+template <int NT, int NV>
+__device__ __forceinline__ double (&parts())[NV][NT] {
+    __shared__ double part[NV][NT];
+    return part;
+}
+
 // block_allreduce of doubles plus one quotient of a total, q = num /
 // total[QI] (OVER = true) or total[QI] / num (OVER = false), formed by warp 0
 // alone, which holds the totals, and returned in every thread with them.
@@ -452,13 +457,6 @@ __device__ __forceinline__ void block_allreduce(T (&v)[NV]) {
 // cost about 10 k FP64 operations per system and iteration, whatever the
 // system's size.  (The mixed kernel keeps per-thread divides: its FP64 pipe is
 // otherwise idle, and the helper's registers made its sliced form spill.)
-// Space for the threads' values, one for all sums of NV doubles in a kernel.
-template <int NT, int NV>
-__device__ __forceinline__ double (&parts())[NV][NT] {
-    __shared__ double part[NV][NT];
-    return part;
-}
-
 template <int NT, int NV, int QI, bool OVER>
 __device__ __forceinline__ double block_allreduce_q(double (&v)[NV], double num) {
     // the narrow form of block_allsum: warp 0 adds every thread's value
@@ -490,8 +488,9 @@ __device__ __forceinline__ double block_allreduce_q(double (&v)[NV], double num)
 }
 
 // The team forms of the CTA sums: the CTAs' totals meet in every CTA's slots
-// and each adds them in the same order.  They end with a barrier of the CTA;
-// two calls of the same instantiation are a team barrier apart.
+// and each adds them in the same order: one warp per value for doubles, which then
+// ends with a barrier of the CTA, every thread for floats, after the team's barrier.
+// Two calls of the same instantiation are a team barrier apart.
 constexpr int kTeamMax = 8;
 template <int NT, int NV, bool QUOT, int QI, bool OVER>
 __device__ __forceinline__ double team_allreduce_q(double (&v)[NV], double num, const Share& sh) {
@@ -811,203 +810,203 @@ template <int NT, int G, bool SL, bool TEAM>
 __device__ __forceinline__ void mixed_system(const BatchArgs& a, int sys, float* pS, int* sPat) {
     const int tid = threadIdx.x;
     const int lane = tid % G;
-            const int r0 = a.sysRow[sys], n = a.sysRow[sys + 1] - r0;
-            const int e0 = a.rowptr[r0];
-            float* P = !TEAM && n <= a.smemRows ? pS : a.p32Global + r0;
-            const Share sh = share_of<TEAM>(n, a.teamCtas);
-            const int lo = sh.lo, hi = sh.hi;
-            // the system's shared column offsets (read after the barrier below)
-            if (SL && kBatchSys32 && threadIdx.x <= kBatchPatMax)
-                sPat[threadIdx.x] = a.sysPat[(size_t)sys * (kBatchPatMax + 1) + threadIdx.x];
-            const int* rp = a.rowptr + r0;
-            const int* cl = a.col + e0;
-            const double* vl = a.val + e0;
-            const float* vl32 = a.val32 + e0;
-            float* r = a.r32 + r0;
-            float* d = a.d32 + r0;
-            float* J = a.J32 + r0;
-            float* Ap = a.Ap32 + r0;
-            double* x = a.x + r0;
-            // x = 0, d = 0, J = 1/diag, r = b, p = J r
-            double bbA = 0;
-            float rzA = 0.f;
+    const int r0 = a.sysRow[sys], n = a.sysRow[sys + 1] - r0;
+    const int e0 = a.rowptr[r0];
+    float* P = !TEAM && n <= a.smemRows ? pS : a.p32Global + r0;
+    const Share sh = share_of<TEAM>(n, a.teamCtas);
+    const int lo = sh.lo, hi = sh.hi;
+    // the system's shared column offsets (read after the barrier below)
+    if (SL && kBatchSys32 && threadIdx.x <= kBatchPatMax)
+        sPat[threadIdx.x] = a.sysPat[(size_t)sys * (kBatchPatMax + 1) + threadIdx.x];
+    const int* rp = a.rowptr + r0;
+    const int* cl = a.col + e0;
+    const double* vl = a.val + e0;
+    const float* vl32 = a.val32 + e0;
+    float* r = a.r32 + r0;
+    float* d = a.d32 + r0;
+    float* J = a.J32 + r0;
+    float* Ap = a.Ap32 + r0;
+    double* x = a.x + r0;
+    // x = 0, d = 0, J = 1/diag, r = b, p = J r
+    double bbA = 0;
+    float rzA = 0.f;
+    for (int i = lo + tid; i < hi; i += NT) {
+        const double bi = a.b[r0 + i];
+        const float ji = (float)(1.0 / a.diag[r0 + i]);
+        const float ri = (float)bi;
+        x[i] = 0.0;
+        d[i] = 0.f;
+        J[i] = ji;
+        r[i] = ri;
+        P[i] = ji * ri;
+        bbA = fma(bi, bi, bbA);
+        rzA = fmaf(ri, ji * ri, rzA);
+    }
+    double v0[2] = {bbA, (double)rzA};
+    sums<NT, 2, TEAM, double>(v0, sh);
+    if (TEAM) team_barrier<TEAM>();  // p is whole, and the sums' slots are read
+    const double bb = v0[0];
+    const double tols = bb * a.tol * a.tol;
+    double rz = v0[1], rrMax = bb, rrTrue = bb;
+    uint32_t k = 0, outer = 0;
+    bool bd = false, stop = false;
+    while (!stop) {
+        // Ap = A p (FP32), p.Ap
+        float pAp = 0.f;
+        if (SL) {
+            const int* so = a.sliceOff + a.sliceBase[sys];
+            const int sysL = kBatchSys32 ? sPat[0] : 0;
+            int j = (lo + tid) >> 5;
+            for (; 32 * (j + NT / 32) < hi; j += 2 * (NT / 32)) {
+                float acc0, acc1;
+                slice_pair<float, float, 0, kBatchPat32, kBatchSys32>(
+                    so, a.patLen + a.sliceBase[sys], a.patOff + (size_t)a.sliceBase[sys] * kBatchPatMax,
+                    a.meta + a.sliceBase[sys], sPat, sysL, j, j + NT / 32, NT, a.sval32, a.scol, P, tid & 31, acc0,
+                    acc1);
+                const int row0 = 32 * j + (tid & 31), row1 = row0 + NT;
+                if (row0 < hi) {
+                    Ap[row0] = acc0;
+                    pAp = fmaf(P[row0], acc0, pAp);
+                }
+                if (row1 < hi) {
+                    Ap[row1] = acc1;
+                    pAp = fmaf(P[row1], acc1, pAp);
+                }
+            }
+            for (; 32 * j < hi; j += NT / 32) {
+                const float acc = slice_dot<float, float>(so, j, a.sval32, a.scol, P, tid & 31);
+                const int row = 32 * j + (tid & 31);
+                if (row < hi) {
+                    Ap[row] = acc;
+                    pAp = fmaf(P[row], acc, pAp);
+                }
+            }
+        } else {
+            for (int rb = (tid >> 5) * (32 / G); rb < n; rb += NT / G) {
+                const int row = rb + (tid & 31) / G;
+                float acc = 0.f;
+                if (row < n) {
+                    const int s0 = rp[row] - e0, s1 = rp[row + 1] - e0;
+                    for (int q = s0 + lane; q < s1; q += G) acc = fmaf(vl32[q], P[cl[q]], acc);
+                }
+                if (G > 1) {
+#pragma unroll
+                    for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
+                }
+                if (lane == 0 && row < n) {
+                    Ap[row] = acc;
+                    pAp = fmaf(P[row], acc, pAp);
+                }
+            }
+        }
+        float v1[1] = {pAp};
+        sums<NT, 1, TEAM, float>(v1, sh);
+        const double alphaD = rz / (double)v1[0];
+        const float alpha = (float)alphaD;
+        float rrP = 0.f, rzP = 0.f;
+        constexpr int UPDM = kBatchUpd;
+        int i = lo + tid;
+        for (; i + (UPDM - 1) * NT < hi; i += UPDM * NT) {
+            float pv[UPDM], dv[UPDM], av[UPDM], qv[UPDM], jv[UPDM];
+#pragma unroll
+            for (int u = 0; u < UPDM; ++u) {
+                pv[u] = P[i + u * NT];
+                dv[u] = d[i + u * NT];
+                av[u] = Ap[i + u * NT];
+                qv[u] = r[i + u * NT];
+                jv[u] = J[i + u * NT];
+            }
+#pragma unroll
+            for (int u = 0; u < UPDM; ++u) {
+                const float ri = fmaf(-alpha, av[u], qv[u]);
+                const float zi = ri * jv[u];
+                d[i + u * NT] = fmaf(alpha, pv[u], dv[u]);
+                r[i + u * NT] = ri;
+                Ap[i + u * NT] = zi;
+                rrP = fmaf(ri, ri, rrP);
+                rzP = fmaf(ri, zi, rzP);
+            }
+        }
+        for (; i < hi; i += NT) {
+            const float ri = fmaf(-alpha, Ap[i], r[i]);
+            const float zi = ri * J[i];
+            d[i] = fmaf(alpha, P[i], d[i]);
+            r[i] = ri;
+            Ap[i] = zi;  // Ap is spent: keep z = J r for the p update
+            rrP = fmaf(ri, ri, rrP);
+            rzP = fmaf(ri, zi, rzP);
+        }
+        float w[2] = {rrP, rzP};
+        sums<NT, 2, TEAM, float>(w, sh);
+        ++k;
+        const double rrN = w[0], rzN = w[1];
+        if (rrN > rrMax) rrMax = rrN;
+        bd = !isfinite(alphaD) || !isfinite(rrN) || !isfinite(rzN);
+        const bool refresh = bd || rrN < a.delta2 * rrMax || rrN < tols || k + 1u >= a.maxIterP1;
+        double beta;
+        if (!refresh) {
+            beta = rzN / rz;
+            rz = rzN;
+        } else {
+            // fold, FP64 true residual, FP32 restart from it
             for (int i = lo + tid; i < hi; i += NT) {
-                const double bi = a.b[r0 + i];
-                const float ji = (float)(1.0 / a.diag[r0 + i]);
-                const float ri = (float)bi;
-                x[i] = 0.0;
+                x[i] += (double)d[i];
                 d[i] = 0.f;
-                J[i] = ji;
-                r[i] = ri;
-                P[i] = ji * ri;
-                bbA = fma(bi, bi, bbA);
-                rzA = fmaf(ri, ji * ri, rzA);
             }
-            double v0[2] = {bbA, (double)rzA};
-            sums<NT, 2, TEAM, double>(v0, sh);
-            if (TEAM) team_barrier<TEAM>();  // p is whole, and the sums' slots are read
-            const double bb = v0[0];
-            const double tols = bb * a.tol * a.tol;
-            double rz = v0[1], rrMax = bb, rrTrue = bb;
-            uint32_t k = 0, outer = 0;
-            bool bd = false, stop = false;
-            while (!stop) {
-                // Ap = A p (FP32), p.Ap
-                float pAp = 0.f;
-                if (SL) {
-                    const int* so = a.sliceOff + a.sliceBase[sys];
-                    const int sysL = kBatchSys32 ? sPat[0] : 0;
-                    int j = (lo + tid) >> 5;
-                    for (; 32 * (j + NT / 32) < hi; j += 2 * (NT / 32)) {
-                        float acc0, acc1;
-                        slice_pair<float, float, 0, kBatchPat32, kBatchSys32>(
-                            so, a.patLen + a.sliceBase[sys], a.patOff + (size_t)a.sliceBase[sys] * kBatchPatMax,
-                            a.meta + a.sliceBase[sys], sPat, sysL, j, j + NT / 32, NT, a.sval32, a.scol, P, tid & 31, acc0,
-                            acc1);
-                        const int row0 = 32 * j + (tid & 31), row1 = row0 + NT;
-                        if (row0 < hi) {
-                            Ap[row0] = acc0;
-                            pAp = fmaf(P[row0], acc0, pAp);
-                        }
-                        if (row1 < hi) {
-                            Ap[row1] = acc1;
-                            pAp = fmaf(P[row1], acc1, pAp);
-                        }
-                    }
-                    for (; 32 * j < hi; j += NT / 32) {
-                        const float acc = slice_dot<float, float>(so, j, a.sval32, a.scol, P, tid & 31);
-                        const int row = 32 * j + (tid & 31);
-                        if (row < hi) {
-                            Ap[row] = acc;
-                            pAp = fmaf(P[row], acc, pAp);
-                        }
-                    }
-                } else {
-                    for (int rb = (tid >> 5) * (32 / G); rb < n; rb += NT / G) {
-                        const int row = rb + (tid & 31) / G;
-                        float acc = 0.f;
-                        if (row < n) {
-                            const int s0 = rp[row] - e0, s1 = rp[row + 1] - e0;
-                            for (int q = s0 + lane; q < s1; q += G) acc = fmaf(vl32[q], P[cl[q]], acc);
-                        }
-                        if (G > 1) {
-    #pragma unroll
-                            for (int o = G / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o, G);
-                        }
-                        if (lane == 0 && row < n) {
-                            Ap[row] = acc;
-                            pAp = fmaf(P[row], acc, pAp);
-                        }
-                    }
-                }
-                float v1[1] = {pAp};
-                sums<NT, 1, TEAM, float>(v1, sh);
-                const double alphaD = rz / (double)v1[0];
-                const float alpha = (float)alphaD;
-                float rrP = 0.f, rzP = 0.f;
-                constexpr int UPDM = kBatchUpd;
-                int i = lo + tid;
-                for (; i + (UPDM - 1) * NT < hi; i += UPDM * NT) {
-                    float pv[UPDM], dv[UPDM], av[UPDM], qv[UPDM], jv[UPDM];
-    #pragma unroll
-                    for (int u = 0; u < UPDM; ++u) {
-                        pv[u] = P[i + u * NT];
-                        dv[u] = d[i + u * NT];
-                        av[u] = Ap[i + u * NT];
-                        qv[u] = r[i + u * NT];
-                        jv[u] = J[i + u * NT];
-                    }
-    #pragma unroll
-                    for (int u = 0; u < UPDM; ++u) {
-                        const float ri = fmaf(-alpha, av[u], qv[u]);
-                        const float zi = ri * jv[u];
-                        d[i + u * NT] = fmaf(alpha, pv[u], dv[u]);
-                        r[i + u * NT] = ri;
-                        Ap[i + u * NT] = zi;
-                        rrP = fmaf(ri, ri, rrP);
-                        rzP = fmaf(ri, zi, rzP);
-                    }
-                }
-                for (; i < hi; i += NT) {
-                    const float ri = fmaf(-alpha, Ap[i], r[i]);
-                    const float zi = ri * J[i];
-                    d[i] = fmaf(alpha, P[i], d[i]);
-                    r[i] = ri;
-                    Ap[i] = zi;  // Ap is spent: keep z = J r for the p update
-                    rrP = fmaf(ri, ri, rrP);
-                    rzP = fmaf(ri, zi, rzP);
-                }
-                float w[2] = {rrP, rzP};
-                sums<NT, 2, TEAM, float>(w, sh);
-                ++k;
-                const double rrN = w[0], rzN = w[1];
-                if (rrN > rrMax) rrMax = rrN;
-                bd = !isfinite(alphaD) || !isfinite(rrN) || !isfinite(rzN);
-                const bool refresh = bd || rrN < a.delta2 * rrMax || rrN < tols || k + 1u >= a.maxIterP1;
-                double beta;
-                if (!refresh) {
-                    beta = rzN / rz;
-                    rz = rzN;
-                } else {
-                    // fold, FP64 true residual, FP32 restart from it
-                    for (int i = lo + tid; i < hi; i += NT) {
-                        x[i] += (double)d[i];
-                        d[i] = 0.f;
-                    }
-                    team_barrier<TEAM>();
-                    double rrA = 0;
-                    for (int row = lo + tid; row < hi; row += NT) {
-                        const int s0 = rp[row] - e0, s1 = rp[row + 1] - e0;
-                        double acc = 0;
-                        for (int q = s0; q < s1; ++q) acc = fma(vl[q], x[cl[q]], acc);
-                        const double ri = a.b[r0 + row] - acc;
-                        r[row] = (float)ri;
-                        rrA = fma(ri, ri, rrA);
-                    }
-                    __syncthreads();
-                    float rzR = 0.f;
-                    for (int i = lo + tid; i < hi; i += NT) {
-                        const float zi = r[i] * J[i];
-                        Ap[i] = zi;
-                        rzR = fmaf(r[i], zi, rzR);
-                    }
-                    double v3[2] = {rrA, (double)rzR};
-                    sums<NT, 2, TEAM, double>(v3, sh);
-                    ++outer;
-                    rrTrue = v3[0];
-                    rrMax = rrTrue;
-                    stop = !(rrTrue > tols) || k + 1u >= a.maxIterP1;
-                    if (bd || !isfinite(rrTrue) || !isfinite(v3[1])) {
-                        bd = true;
-                        stop = true;
-                    }
-                    beta = v3[1] / rz;
-                    rz = v3[1];
-                }
-                if (stop) break;
-                const float betaF = (float)beta;
-                int t = lo + tid;
-                for (; t + (UPDM - 1) * NT < hi; t += UPDM * NT) {  // z + beta p
-                    float pv[UPDM], zv[UPDM];
-    #pragma unroll
-                    for (int u = 0; u < UPDM; ++u) {
-                        pv[u] = P[t + u * NT];
-                        zv[u] = Ap[t + u * NT];
-                    }
-    #pragma unroll
-                    for (int u = 0; u < UPDM; ++u) P[t + u * NT] = fmaf(betaF, pv[u], zv[u]);
-                }
-                for (; t < hi; t += NT) P[t] = fmaf(betaF, P[t], Ap[t]);  // z + beta p
-                team_barrier<TEAM>();
+            team_barrier<TEAM>();
+            double rrA = 0;
+            for (int row = lo + tid; row < hi; row += NT) {
+                const int s0 = rp[row] - e0, s1 = rp[row + 1] - e0;
+                double acc = 0;
+                for (int q = s0; q < s1; ++q) acc = fma(vl[q], x[cl[q]], acc);
+                const double ri = a.b[r0 + row] - acc;
+                r[row] = (float)ri;
+                rrA = fma(ri, ri, rrA);
             }
-            if (tid == 0 && sh.q == 0) {
-                BatchResult& o = a.res[sys];
-                o.itersRun = k;
-                o.iters = k;
-                o.outer = outer;
-                o.res = sqrt(rrTrue / bb);
-                o.status = bd ? 1u : 0u;
+            __syncthreads();
+            float rzR = 0.f;
+            for (int i = lo + tid; i < hi; i += NT) {
+                const float zi = r[i] * J[i];
+                Ap[i] = zi;
+                rzR = fmaf(r[i], zi, rzR);
             }
+            double v3[2] = {rrA, (double)rzR};
+            sums<NT, 2, TEAM, double>(v3, sh);
+            ++outer;
+            rrTrue = v3[0];
+            rrMax = rrTrue;
+            stop = !(rrTrue > tols) || k + 1u >= a.maxIterP1;
+            if (bd || !isfinite(rrTrue) || !isfinite(v3[1])) {
+                bd = true;
+                stop = true;
+            }
+            beta = v3[1] / rz;
+            rz = v3[1];
+        }
+        if (stop) break;
+        const float betaF = (float)beta;
+        int t = lo + tid;
+        for (; t + (UPDM - 1) * NT < hi; t += UPDM * NT) {  // z + beta p
+            float pv[UPDM], zv[UPDM];
+#pragma unroll
+            for (int u = 0; u < UPDM; ++u) {
+                pv[u] = P[t + u * NT];
+                zv[u] = Ap[t + u * NT];
+            }
+#pragma unroll
+            for (int u = 0; u < UPDM; ++u) P[t + u * NT] = fmaf(betaF, pv[u], zv[u]);
+        }
+        for (; t < hi; t += NT) P[t] = fmaf(betaF, P[t], Ap[t]);  // z + beta p
+        team_barrier<TEAM>();
+    }
+    if (tid == 0 && sh.q == 0) {
+        BatchResult& o = a.res[sys];
+        o.itersRun = k;
+        o.iters = k;
+        o.outer = outer;
+        o.res = sqrt(rrTrue / bb);
+        o.status = bd ? 1u : 0u;
+    }
     team_barrier<TEAM>();
 }
 
@@ -1091,18 +1090,6 @@ bool batch_config_sliced(int cfg) { return kBatchCfgs[cfg].sliced; }
 
 // ---- per-system SELL-32 copy ----
 namespace {
-__device__ __forceinline__ int warp_max_i(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-__device__ __forceinline__ int warp_min_i(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 // System of global slice g: the largest s with sliceBase[s] <= g.
 __device__ __forceinline__ int system_of_slice(const int* __restrict__ sliceBase, int nsys, int g) {
     int lo = 0, hi = nsys - 1;
@@ -1144,12 +1131,12 @@ __global__ void bsell_width_kernel(int nsys, int nslices, const int* __restrict_
         const int lr = first + lane;
         const bool in = lr < n;
         const int j0 = in ? rowptr[r0 + lr] : 0, j1 = in ? rowptr[r0 + lr + 1] : 0;
-        const int w = warp_max_i(j1 - j0);
+        const int w = warp_max(j1 - j0);
         bool ok = patterns && __all_sync(0xffffffffu, in);
         int L = 0, q = j0, myOff = 0;
         int cur = q < j1 ? col[q] - lr : INT_MAX;
         while (ok) {
-            const int m = warp_min_i(cur);
+            const int m = warp_min(cur);
             if (m == INT_MAX) break;
             if (L == kBatchPatMax || first + m < 0 || first + 31 + m >= n) {
                 ok = false;
@@ -1328,7 +1315,8 @@ static cudaError_t team_config(bool mixed, int ctas, int smemRows, cudaStream_t 
     typedef void (*Kernel)(BatchArgs);
     *kernel = mixed ? (Kernel)batched_mixed_kernel<512, 1, true, true> : (Kernel)batched_fp64_kernel<512, 1, true, true>;
     const size_t smem = (size_t)smemRows * (mixed ? sizeof(float) : sizeof(double));
-    cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // the most that any call asks for, so that threads may set it side by side
+    cudaError_t e = cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
     *cfg = {};
     cfg->gridDim = dim3((unsigned)ctas);
     cfg->blockDim = dim3(512);

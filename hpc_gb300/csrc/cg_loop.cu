@@ -475,19 +475,6 @@ constexpr int kClusterThreads = 512;
 constexpr int kClusterMax = 16;
 constexpr size_t kClusterSmem = 212 * 1024;  // beside 14 KB of static shared memory
 
-// Every thread of the cluster; distributed shared memory written before is
-// visible after.
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ uint32_t map_rank(const void* p, uint32_t rank) {
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_addr(p)), "r"(rank));
-    return a;
-}
-
 __device__ __forceinline__ double ld_cluster(uint32_t a) {
     double v;
     asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a));
@@ -497,7 +484,7 @@ __device__ __forceinline__ double ld_cluster(uint32_t a) {
 // v, in every lane, into the same place of every CTA of the cluster.
 __device__ __forceinline__ void to_all(double* place, double v, int P, int lane) {
     if (lane < P)
-        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(map_rank(place, (uint32_t)lane)), "d"(v) : "memory");
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(place, (uint32_t)lane)), "d"(v) : "memory");
 }
 
 }  // namespace
@@ -549,7 +536,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1) cg_cluster_kernel(LoopArgs
         for (int j = 0; j < md.y; ++j) {
             const int e = md.x + j * 32 + lane, c = NARROW ? row + a.col16[e] : a.col32[e];
             mv[e - mat0] = a.sval[e];
-            mc[e - mat0] = map_rank(sp + c % R, (uint32_t)(c / R));
+            mc[e - mat0] = cluster_addr(sp + c % R, (uint32_t)(c / R));
         }
     }
     const double tols = a.state->tols;
