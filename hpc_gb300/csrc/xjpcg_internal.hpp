@@ -130,7 +130,7 @@ cudaError_t sellsort_hub_entries(cudaStream_t st, int nHubs, const int* sorted, 
 // out (nnz ints): col with those rows' columns as ~place; hubOf: n ints.
 cudaError_t sellsort_recode(cudaStream_t st, int n, int64_t nnz, int nHubs, const int* sorted, const int* col, int* hubOf,
                             int* out);
-// nHubs > 0 (unroll 8 only): scol and col are recoded columns, hubX has room for
+// nHubs > 0 (sellsort_config_hubs only): scol and col are recoded columns, hubX has room for
 // nHubs values.
 template <typename VT>
 cudaError_t spmv_sellsort_launch(int cfg, int grid, cudaStream_t st, int n, int nLong, const int* sorted,
